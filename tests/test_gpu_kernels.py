@@ -92,6 +92,40 @@ def test_linear(K, dtype, M, N, K_):
         assert torch.equal(alone[0], got32[M - 1])
 
 
+@pytest.mark.parametrize("inner", [4, 36, 256, 260, 516, 1028, 4868])
+@pytest.mark.parametrize("outputs", [1, 31, 67, 130])
+def test_linear_float32_one_order_over_all_its_kernels(K, outputs, inner):
+    """Around the borders of the kernels (16 rows, tiles of 64 rows and 64 or 128 outputs, chunks and slices of the inner size): against
+    float64, with a bias and added into a tensor, and a row has the same bits alone, among others and from an address that only the
+    general kernel takes. Bound: the chains are at most inner / 2 roundings of the magnitude of sum |x w|, whose random
+    walk stays within a few roundings; 2e-6 of the result's scale is what the other tests of this product allow."""
+    g = torch.Generator().manual_seed(inner)
+    x = torch.randn(150, inner, generator=g).cuda()
+    w = torch.randn(outputs, inner, generator=g).cuda()
+    b = torch.randn(outputs, generator=g).cuda()
+    want = x.double() @ w.double().T + b.double()
+    shifted = torch.empty(x.numel() + 1, device="cuda")[1:].view_as(x)
+    shifted.copy_(x)
+    assert shifted.data_ptr() % 16 != 0
+    general = K.linear(shifted, w, bias=b)
+    close(general.cpu(), want.cpu(), 2e-6)
+    for M in (1, 2, 3, 4, 5, 13, 16, 17, 64, 65, 150):
+        assert torch.equal(K.linear(x[:M], w, bias=b), general[:M]), f"{M} rows"
+        into = x.new_full((M, outputs), 2.0)
+        K.linear(x[:M], w, add_to=into, bias=b)
+        assert torch.equal(into, general[:M] + 2.0), f"{M} rows, added"
+
+
+@pytest.mark.parametrize("rows", [100, 300])
+def test_linear_float32_wide_tiles(K, rows):
+    """Enough outputs for tiles of 128: the bits of the narrow ones."""
+    g = torch.Generator().manual_seed(3)
+    x, w = torch.randn(rows, 896, generator=g).cuda(), torch.randn(9731, 896, generator=g).cuda()
+    got = K.linear(x, w)
+    for lo in (0, 9600):
+        assert torch.equal(got[:, lo:lo + 131], K.linear(x, w[lo:lo + 131].contiguous()))
+
+
 def test_linear_float32_is_true_32bit(K):
     """Inputs that a reduced-precision matrix mode (TF32, bfloat16) would round: 1 + 2^-12 squared."""
     x = torch.full((4, 64), 1 + 2.0 ** -12)
