@@ -15,11 +15,13 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "scan_sums.cuh"
 
 namespace {
 
 constexpr int ML_THREADS = 128;
-constexpr int ML_TILE = 8;   // tokens per stage; the gates of a tile are scanned by the first ML_TILE lanes of the first warp
+constexpr int ML_TILE = 16;   // tokens per stage, a token's gates per lane of the gates' warp
+static inline __host__ __device__ constexpr int ml_parts(int dmax) { return dmax >= 32 ? dmax / 8 : 4; }
 
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 // ln sigmoid(x) = min(x, 0) - ln(1 + exp(-|x|))
@@ -38,10 +40,12 @@ template <typename T>
 __global__ void __launch_bounds__(128) mlstm_prepare_kernel(const T* __restrict__ z, int z_stride, int q_col, int k_col, const float* __restrict__ gates,
                                                             int g_stride, const float* __restrict__ bias_i, const float* __restrict__ bias_f, float cap,
                                                             float q_scale, float* __restrict__ qf, float* __restrict__ kf, float* __restrict__ ig,
-                                                            float* __restrict__ fg, int H, int D) {
+                                                            float* __restrict__ fg, int H, int D, int* __restrict__ readers, int num_readers) {
     pdl_trigger();
     pdl_wait();
     const int n = blockIdx.x;
+    if (n == 0)   // the scan's counts of readers start from zero
+        for (int i = threadIdx.x; i < num_readers; i += blockDim.x) readers[i] = 0;
     const T* row = z + (size_t)n * z_stride;
     const int HD = H * D;
     for (int i = threadIdx.x; i < HD; i += blockDim.x) {
@@ -57,87 +61,57 @@ __global__ void __launch_bounds__(128) mlstm_prepare_kernel(const T* __restrict_
     }
 }
 
-template <int PARTS> __device__ __forceinline__ float parts_sum(float v) {
-#pragma unroll
-    for (int o = 1; o < PARTS; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// Block (x, h, r): COLS columns of head h of request r, PARTS lanes to a group of CPL columns, each lane holding DPL entries of each
-// of them in registers (16-byte pieces, PARTS pieces apart). Rows of q and k come in tiles of ML_TILE tokens through a two-stage ring
-// (cp.async); a tile's gates are loaded into registers a tile ahead by the first warp, which walks the chain of maxima over the tile
-// and turns the gates into (a, b, m) per token, a token per lane, so the exponentials are taken once per token and block, not once
-// per thread.
-template <typename T, int DMAX, int PARTS, int CPL>
-__global__ void __launch_bounds__(ML_THREADS) mlstm_scan_kernel(const T* __restrict__ v, int v_stride, int v_col, const float* __restrict__ qf,
-                                                                const float* __restrict__ kf, const float* __restrict__ ig, const float* __restrict__ fg,
-                                                                float* __restrict__ state, float* __restrict__ mstate, const int* __restrict__ seq_starts,
-                                                                const int* __restrict__ seq_slots, float* __restrict__ num, float* __restrict__ m_out,
-                                                                int H, int D, int DV) {
-    constexpr int DPL = DMAX / PARTS, COLS = (ML_THREADS / PARTS) * CPL, Q = DMAX / 4;   // COLS: the block's columns, CPL to a group of lanes
-    __shared__ __align__(16) float k_s[2][ML_TILE][DMAX];
-    __shared__ __align__(16) float q_s[2][ML_TILE][DMAX];
-    __shared__ float a_s[2][ML_TILE], b_s[2][ML_TILE], m_s[2][ML_TILE];
-    __shared__ float v_s[2][ML_TILE][COLS];
+// Block (x, h, r): COLS columns of head h of request r, PARTS lanes (D / 8) to CPL columns side by side, each lane holding DPL entries of
+// each in registers (16-byte pieces, PARTS pieces apart), in pairs for the packed multiply-add. Rows of q and k
+// come in tiles of ML_TILE tokens through a two-stage ring (cp.async). A fifth warp does nothing but the gates: while the other four
+// work on a tile it walks the chain of maxima over the next one and turns the gates into (a, b, m) per token, a token per lane, so the
+// chain and the exponentials are nobody's wait. Nothing is reduced token by token: the lanes of a column add up PARTS sums together,
+// each ending with one (parts_scatter). A full tile has no branch between its tokens, and a token's rows are loaded while the one
+// before is worked on.
+//
+// The walk is bound by a token's instructions on one warp (its latency hides behind the next token's, nothing feeds back): with four
+// columns to a group of 16 lanes on 80 blocks, a branch per token and the gates between two tiles on the first of the four warps, a
+// prompt of 1,301 tokens (8 heads of 128 x 128, beside one of 700) took 659 us; this form 162 us.
+//
+// The request's m is read by every block of its (h, r) and written by one: the block that is the LAST to have read it, as `readers`
+// (zeroed by the prepare kernel) tells, so that no block that starts late reads what an early one left.
+template <typename T, int DMAX, int CPL>
+__global__ void __launch_bounds__(ML_THREADS + 32) mlstm_scan_kernel(const T* __restrict__ v, int v_stride, int v_col, const float* __restrict__ qf,
+                                                                     const float* __restrict__ kf, const float* __restrict__ ig, const float* __restrict__ fg,
+                                                                     float* __restrict__ state, float* mstate, const int* __restrict__ seq_starts,
+                                                                     const int* __restrict__ seq_slots, float* __restrict__ num, float* __restrict__ m_out,
+                                                                     int* __restrict__ readers, int H, int D, int DV) {
+    constexpr int PARTS = ml_parts(DMAX), DPL = DMAX / PARTS, COLS = ML_THREADS / PARTS * CPL, Q = DMAX / 4, P2 = DPL / 2, BATCH = PARTS / CPL;
+    extern __shared__ __align__(16) float ml_smem[];
+    float* k_s = ml_smem;                          // [2][ML_TILE][DMAX]
+    float* q_s = k_s + 2 * ML_TILE * DMAX;
+    float* v_s = q_s + 2 * ML_TILE * DMAX;         // [2][ML_TILE][COLS]
+    float* a_s = v_s + 2 * ML_TILE * COLS;         // [2][ML_TILE]
+    float* b_s = a_s + 2 * ML_TILE;
     pdl_wait();
-    const int part = threadIdx.x % PARTS, my_col = (threadIdx.x / PARTS) * CPL;   // the first of the lane group's CPL columns, within the block
-    const int col = blockIdx.x * COLS + my_col;
     const int h = blockIdx.y, r = blockIdx.z;
     const int C = DV + 1;                 // the last column is the normaliser
-    const bool vec = (D & 3) == 0;
     const int s0 = seq_starts[r], s1 = seq_starts[r + 1];
     const int slot = seq_slots[r];
-    float* st = state + ((size_t)slot * H + h) * C * D;
-    float S[CPL][DPL];
-#pragma unroll
-    for (int u = 0; u < CPL; ++u)
-#pragma unroll
-        for (int i = 0; i < DPL / 4; ++i) {
-            const int d = 4 * PARTS * i + 4 * part;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) S[u][4 * i + c] = (col + u < C && d + c < D) ? st[(size_t)(col + u) * D + d + c] : 0.f;
+    if (threadIdx.x >= ML_THREADS) {      // the warp of the gates
+        const int lane = threadIdx.x - ML_THREADS;
+        float m_carry = *(volatile float*)(mstate + (size_t)slot * H + h);
+        __syncwarp();
+        bool writes = false;
+        if (lane == 0 && s0 < s1) {
+            __threadfence();              // (the read above comes before the count)
+            writes = atomicAdd(readers + (size_t)r * H + h, 1) == (int)gridDim.x - 1;
         }
-    float m_carry = mstate[(size_t)slot * H + h];   // (every lane of the first warp keeps it)
-
-    auto fetch = [&](int base, int buf) {
-        const int count = min(ML_TILE, s1 - base);
-        for (int i = threadIdx.x; i < count * Q; i += ML_THREADS) {
-            const int t = i / Q, d = (i % Q) * 4;
-            const size_t off = ((size_t)(base + t) * H + h) * D + d;
-            if (vec && d < D) {
-                cp_async16(&k_s[buf][t][d], kf + off);
-                cp_async16(&q_s[buf][t][d], qf + off);
-            } else {
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    k_s[buf][t][d + c] = d + c < D ? kf[off + c] : 0.f;
-                    q_s[buf][t][d + c] = d + c < D ? qf[off + c] : 0.f;
-                }
+        float pre_i, pre_f;
+        auto load = [&](int base) {
+            pre_i = -INFINITY;            // a token past the end changes nothing: m -> max(0 + m, -inf)
+            pre_f = 0.f;
+            if (lane < ML_TILE && base + lane < s1) {
+                pre_i = ig[(size_t)(base + lane) * H + h];
+                pre_f = fg[(size_t)(base + lane) * H + h];
             }
-        }
-    };
-    // a tile's gates (lane t < ML_TILE of the first warp: token t) and the block's columns of v, into registers a tile ahead
-    constexpr int VPT = (ML_TILE * COLS + ML_THREADS - 1) / ML_THREADS;
-    float pre_i = -INFINITY, pre_f = 0.f, pre_v[VPT];
-    auto load_small = [&](int base) {
-        const int count = min(ML_TILE, s1 - base);
-        pre_i = -INFINITY;   // a token past the end changes nothing: m -> max(0 + m, -inf)
-        pre_f = 0.f;
-        if (threadIdx.x < count) {
-            pre_i = ig[(size_t)(base + threadIdx.x) * H + h];
-            pre_f = fg[(size_t)(base + threadIdx.x) * H + h];
-        }
-#pragma unroll
-        for (int n = 0; n < VPT; ++n) {
-            const int j = ML_THREADS - 1 - threadIdx.x + n * ML_THREADS;
-            const int t = j / COLS, c = blockIdx.x * COLS + j % COLS;
-            float x = 0.f;
-            if (j < count * COLS) x = c < DV ? to_f32(v[(size_t)(base + t) * v_stride + v_col + h * DV + c]) : (c == DV ? 1.f : 0.f);
-            pre_v[n] = x;
-        }
-    };
-    auto store_small = [&](int buf) {
-        if (threadIdx.x < 32) {
+        };
+        auto gates = [&](int base, int buf) {
             // the chain m -> max(f + m, i) over the tile's tokens, walked by every lane of the warp in the tokens' order (each step
             // exactly as a token-by-token walk would take it, so the bits do not depend on where a tile begins); lane t keeps token t's
             float m_run = m_carry, m_prev = m_carry, m_t = m_carry;
@@ -145,86 +119,164 @@ __global__ void __launch_bounds__(ML_THREADS) mlstm_scan_kernel(const T* __restr
             for (int t = 0; t < ML_TILE; ++t) {
                 const float ft = __shfl_sync(0xffffffffu, pre_f, t), it = __shfl_sync(0xffffffffu, pre_i, t);
                 const float m_new = fmaxf(ft + m_run, it);
-                if ((int)threadIdx.x == t) { m_prev = m_run; m_t = m_new; }
+                if (lane == t) { m_prev = m_run; m_t = m_new; }
                 m_run = m_new;
             }
-            if (threadIdx.x >= ML_TILE) m_t = m_run;
-            if (threadIdx.x < ML_TILE) {
-                a_s[buf][threadIdx.x] = expf(pre_f + m_prev - m_t);
-                b_s[buf][threadIdx.x] = expf(pre_i - m_t);
-                m_s[buf][threadIdx.x] = m_t;
+            if (lane < ML_TILE) {
+                a_s[buf * ML_TILE + lane] = expf(pre_f + m_prev - m_t);
+                b_s[buf * ML_TILE + lane] = expf(pre_i - m_t);
+                if (blockIdx.x == 0 && base + lane < s1) m_out[(size_t)(base + lane) * H + h] = m_t;
             }
             m_carry = m_run;
+        };
+        if (s0 < s1) {
+            load(s0);
+            gates(s0, 0);
+            load(s0 + ML_TILE);
         }
+        int buf = 0;
+        for (int base = s0; base < s1; base += ML_TILE, buf ^= 1) {
+            __syncthreads();
+            if (base + ML_TILE < s1) {
+                gates(base + ML_TILE, buf ^ 1);
+                load(base + 2 * ML_TILE);
+            }
+        }
+        pdl_trigger();
+        if (writes) mstate[(size_t)slot * H + h] = m_carry;
+        return;
+    }
+    const int part = threadIdx.x % PARTS, my_col = threadIdx.x / PARTS * CPL;   // the first of the lane's CPL columns, within the block
+    const int col = blockIdx.x * COLS + my_col;
+    const bool vec = (D & 3) == 0;
+    float* st = state + ((size_t)slot * H + h) * C * D;
+    float2 S[CPL][P2];
+#pragma unroll
+    for (int u = 0; u < CPL; ++u)
+#pragma unroll
+        for (int i = 0; i < DPL / 4; ++i) {
+            const int d = 4 * PARTS * i + 4 * part;
+            float x[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x[c] = (col + u < C && d + c < D) ? st[(size_t)(col + u) * D + d + c] : 0.f;
+            S[u][2 * i] = make_float2(x[0], x[1]);
+            S[u][2 * i + 1] = make_float2(x[2], x[3]);
+        }
+    auto fetch = [&](int base, int buf) {
+        const int count = min(ML_TILE, s1 - base);
+        for (int i = threadIdx.x; i < count * Q; i += ML_THREADS) {
+            const int t = i / Q, d = (i % Q) * 4;
+            const size_t off = ((size_t)(base + t) * H + h) * D + d;
+            float *kd = k_s + (buf * ML_TILE + t) * DMAX + d, *qd = q_s + (buf * ML_TILE + t) * DMAX + d;
+            if (vec && d < D) {
+                cp_async16(kd, kf + off);
+                cp_async16(qd, qf + off);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    kd[c] = d + c < D ? kf[off + c] : 0.f;
+                    qd[c] = d + c < D ? qf[off + c] : 0.f;
+                }
+            }
+        }
+    };
+    // the block's columns of v, into registers a tile ahead
+    constexpr int VPT = (ML_TILE * COLS + ML_THREADS - 1) / ML_THREADS;
+    float pre_v[VPT];
+    auto load_v = [&](int base) {
+        const int count = min(ML_TILE, s1 - base);
 #pragma unroll
         for (int n = 0; n < VPT; ++n) {
-            const int j = ML_THREADS - 1 - threadIdx.x + n * ML_THREADS;
-            if (j < ML_TILE * COLS) v_s[buf][j / COLS][j % COLS] = pre_v[n];
+            const int j = threadIdx.x + n * ML_THREADS;
+            const int t = j / COLS, c = blockIdx.x * COLS + j % COLS;
+            float x = 0.f;
+            if (j < count * COLS) x = c < DV ? to_f32(v[(size_t)(base + t) * v_stride + v_col + h * DV + c]) : (c == DV ? 1.f : 0.f);
+            pre_v[n] = x;
+        }
+    };
+    auto store_v = [&](int buf) {
+#pragma unroll
+        for (int n = 0; n < VPT; ++n) {
+            const int j = threadIdx.x + n * ML_THREADS;
+            if (j < ML_TILE * COLS) v_s[buf * ML_TILE * COLS + j] = pre_v[n];
         }
     };
     if (s0 < s1) {
         fetch(s0, 0);
-        load_small(s0);
-        store_small(0);
+        load_v(s0);
     }
     cp_commit();
     int buf = 0;
     for (int base = s0; base < s1; base += ML_TILE, buf ^= 1) {
         const int count = min(ML_TILE, s1 - base);
-        const bool more = base + ML_TILE < s1;
-        if (more) {
+        store_v(buf);                          // (this stage's last readers passed the barrier of the tile between)
+        cp_wait<0>();
+        __syncthreads();                       // this tile is in shared memory, and everyone is done with the other stage
+        if (base + ML_TILE < s1) {
             fetch(base + ML_TILE, buf ^ 1);
-            load_small(base + ML_TILE);
+            load_v(base + ML_TILE);
         }
         cp_commit();
-        cp_wait<1>();
-        __syncthreads();                       // this tile is in shared memory
-        // the tile's tokens in order; every token's partial sums stay in registers and the lanes of a column add them up for all
-        // tokens of the tile together (the shuffles of eight sums overlap instead of waiting for one another)
-        float rq[ML_TILE][CPL];
+        const float* kb = k_s + buf * ML_TILE * DMAX + 4 * part;
+        const float* qb = q_s + buf * ML_TILE * DMAX + 4 * part;
+        struct Row { float2 k[P2], q[P2]; };
+        auto load_row = [&](int t, Row& w) {
 #pragma unroll
-        for (int t = 0; t < ML_TILE; ++t) {
+            for (int i = 0; i < DPL / 4; ++i) {
+                const float4 k4 = *reinterpret_cast<const float4*>(kb + t * DMAX + 4 * PARTS * i);
+                const float4 q4 = *reinterpret_cast<const float4*>(qb + t * DMAX + 4 * PARTS * i);
+                w.k[2 * i] = make_float2(k4.x, k4.y); w.k[2 * i + 1] = make_float2(k4.z, k4.w);
+                w.q[2 * i] = make_float2(q4.x, q4.y); w.q[2 * i + 1] = make_float2(q4.z, q4.w);
+            }
+        };
+        auto token = [&](int t, const Row& w, float* y) {   // y[u]: this lane's share of S^T q of its columns
+            const float a = a_s[buf * ML_TILE + t], b = b_s[buf * ML_TILE + t];
+            const float2 a2 = make_float2(a, a);
 #pragma unroll
-            for (int u = 0; u < CPL; ++u) rq[t][u] = 0.f;
-            if (t < count) {
-                const float a = a_s[buf][t], b = b_s[buf][t];
-                float bv[CPL], r0[CPL], r1[CPL];
+            for (int u = 0; u < CPL; ++u) {
+                const float bv = b * v_s[(buf * ML_TILE + t) * COLS + my_col + u];
+                const float2 bv2 = make_float2(bv, bv);
+                float2 sum[2];
+                sum[0] = sum[1] = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int u = 0; u < CPL; ++u) { bv[u] = b * v_s[buf][t][my_col + u]; r0[u] = 0.f; r1[u] = 0.f; }
-#pragma unroll
-                for (int i = 0; i < DPL / 4; ++i) {   // a piece of k and of q serves all of the lane's columns
-                    const float4 k4 = *reinterpret_cast<const float4*>(&k_s[buf][t][4 * PARTS * i + 4 * part]);
-                    const float4 q4 = *reinterpret_cast<const float4*>(&q_s[buf][t][4 * PARTS * i + 4 * part]);
-#pragma unroll
-                    for (int u = 0; u < CPL; ++u) {
-                        float* s = S[u] + 4 * i;
-                        s[0] = fmaf(bv[u], k4.x, a * s[0]); s[1] = fmaf(bv[u], k4.y, a * s[1]);
-                        s[2] = fmaf(bv[u], k4.z, a * s[2]); s[3] = fmaf(bv[u], k4.w, a * s[3]);
-                        r0[u] = fmaf(s[0], q4.x, r0[u]); r1[u] = fmaf(s[1], q4.y, r1[u]); r0[u] = fmaf(s[2], q4.z, r0[u]); r1[u] = fmaf(s[3], q4.w, r1[u]);
-                    }
+                for (int i = 0; i < P2; ++i) {
+                    S[u][i] = fma2(bv2, w.k[i], mul2(a2, S[u][i]));
+                    sum[i & 1] = fma2(S[u][i], w.q[i], sum[i & 1]);
                 }
+                y[u] = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+            }
+        };
+        float* o = num + ((size_t)base * H + h) * C + col;
+        if (count == ML_TILE) {
+            const int my_t = part / CPL, my_u = part % CPL;   // the sum of a batch that this lane ends with
+            Row now;
+            load_row(0, now);
 #pragma unroll
-                for (int u = 0; u < CPL; ++u) rq[t][u] = r0[u] + r1[u];
+            for (int t0 = 0; t0 < ML_TILE; t0 += BATCH) {
+                float y[PARTS];
+#pragma unroll
+                for (int t = 0; t < BATCH; ++t) {
+                    Row next;
+                    if (t0 + t + 1 < ML_TILE) load_row(t0 + t + 1, next);
+                    token(t0 + t, now, y + t * CPL);
+                    now = next;
+                }
+                const float mine = parts_scatter<PARTS>(y, part);
+                if (col + my_u < C) o[(size_t)(t0 + my_t) * H * C + my_u] = mine;
+            }
+        } else {
+            for (int t = 0; t < count; ++t) {
+                Row now;
+                load_row(t, now);
+                float y[CPL];
+                token(t, now, y);
+#pragma unroll
+                for (int u = 0; u < CPL; ++u) {
+                    const float sum = parts_sum<PARTS>(y[u]);
+                    if (col + u < C && part == 0) o[(size_t)t * H * C + u] = sum;
+                }
             }
         }
-#pragma unroll
-        for (int o = 1; o < PARTS; o <<= 1) {
-#pragma unroll
-            for (int t = 0; t < ML_TILE; ++t)
-#pragma unroll
-                for (int u = 0; u < CPL; ++u) rq[t][u] += __shfl_xor_sync(0xffffffffu, rq[t][u], o);
-        }
-        // every lane of the group holds all sums: lane t of the group stores token t's
-#pragma unroll
-        for (int t = 0; t < ML_TILE; ++t)
-            if (t < count && part == (t % PARTS)) {
-#pragma unroll
-                for (int u = 0; u < CPL; ++u)
-                    if (col + u < C) num[((size_t)(base + t) * H + h) * C + col + u] = rq[t][u];
-            }
-        if (blockIdx.x == 0 && threadIdx.x < count) m_out[(size_t)(base + threadIdx.x) * H + h] = m_s[buf][threadIdx.x];
-        if (more) store_small(buf ^ 1);
-        __syncthreads();                       // everyone is done with this stage before it is filled again
     }
     cp_wait<0>();
     pdl_trigger();
@@ -233,11 +285,11 @@ __global__ void __launch_bounds__(ML_THREADS) mlstm_scan_kernel(const T* __restr
 #pragma unroll
         for (int i = 0; i < DPL / 4; ++i) {
             const int d = 4 * PARTS * i + 4 * part;
+            const float x[4] = {S[u][2 * i].x, S[u][2 * i].y, S[u][2 * i + 1].x, S[u][2 * i + 1].y};
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-                if (col + u < C && d + c < D) st[(size_t)(col + u) * D + d + c] = S[u][4 * i + c];
+                if (col + u < C && d + c < D) st[(size_t)(col + u) * D + d + c] = x[c];
         }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && s0 < s1) mstate[(size_t)slot * H + h] = m_carry;
 }
 
 // One block per (token, head): o = num / (max(|n . q|, exp(-m)) + 1e-6); o / sqrt(mean(o^2) + eps) * w[h * DV + j] * sigmoid(gate).
@@ -260,55 +312,63 @@ __global__ void __launch_bounds__(128) mlstm_finish_kernel(const float* __restri
     }
 }
 
-template <typename T, int DM, int PARTS, int CPL>
+template <typename T, int DM, int CPL>
 int launch_scan_as(const T* v, int v_stride, int v_col, const float* qf, const float* kf, const float* ig, const float* fg, float* state, float* mstate,
-                   const int* seq_starts, const int* seq_slots, float* num, float* m_out, int H, int D, int DV, int R, cudaStream_t s) {
-    constexpr int COLS = (ML_THREADS / PARTS) * CPL;
+                   const int* seq_starts, const int* seq_slots, float* num, float* m_out, int* readers, int H, int D, int DV, int R, bool alone,
+                   cudaStream_t s) {
+    constexpr int COLS = ML_THREADS / ml_parts(DM) * CPL;
+    constexpr int smem = 4 * 2 * ML_TILE * (2 * DM + COLS + 2);
+    if (smem > 48 * 1024) {
+        static const int set = (int)cudaFuncSetAttribute(mlstm_scan_kernel<T, DM, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (set) return set;
+    }
     const dim3 grid((DV + 1 + COLS - 1) / COLS, H, R);
-    return launch_kernel(mlstm_scan_kernel<T, DM, PARTS, CPL>, grid, dim3(ML_THREADS), 0, s, v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts,
-                         seq_slots, num, m_out, H, D, DV);
+    return launch_kernel_on(alone, mlstm_scan_kernel<T, DM, CPL>, grid, dim3(ML_THREADS + 32), (size_t)smem, s, v, v_stride, v_col, qf, kf, ig, fg, state,
+                            mstate, seq_starts, seq_slots, num, m_out, readers, H, D, DV);
 }
 
-// The lanes that share a column depend on the padded key size alone (a lane holds one 16-byte piece of a short column, two from 64
-// entries on: fewer lanes to add up over), and a group of lanes owns up to four columns side by side, so that a piece of k and of q,
-// once fetched from shared memory, serves four columns: with one column to a group the kernel was bound by the instructions around the
-// multiply-adds (31 % of the issue slots busy, a quarter of the instructions multiply-adds; 1.54 ms at 128 entries and 2,048 tokens).
+// The lanes that share a column depend on the padded key size alone, never on the batch: the order of every sum, and with it every bit. How
+// many columns a lane has changes no sum: four where the step's columns are more than fill the device two at a time.
 template <typename T>
 int launch_scan(const T* v, int v_stride, int v_col, const float* qf, const float* kf, const float* ig, const float* fg, float* state, float* mstate,
-                const int* seq_starts, const int* seq_slots, float* num, float* m_out, int H, int D, int DV, int R, cudaStream_t s) {
-#define ML_ARGS v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, H, D, DV, R, s
-    if (D <= 16) return launch_scan_as<T, 16, 4, 1>(ML_ARGS);
-    if (D <= 32) return launch_scan_as<T, 32, 8, 2>(ML_ARGS);
-    if (D <= 64) return launch_scan_as<T, 64, 8, 4>(ML_ARGS);
-    if (D <= 128) return launch_scan_as<T, 128, 16, 4>(ML_ARGS);
-    return launch_scan_as<T, 256, 32, 4>(ML_ARGS);
+                const int* seq_starts, const int* seq_slots, float* num, float* m_out, int* readers, int H, int D, int DV, int R, bool alone,
+                cudaStream_t s) {
+#define ML_ARGS v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, readers, H, D, DV, R, alone, s
+#define ML_AS(DM) return (long long)R * H * (DV + 1) * ml_parts(DM) > 148LL * ML_THREADS * 2 ? launch_scan_as<T, DM, 4>(ML_ARGS) : launch_scan_as<T, DM, 2>(ML_ARGS)
+    if (D <= 16) ML_AS(16);
+    if (D <= 32) ML_AS(32);
+    if (D <= 64) ML_AS(64);
+    if (D <= 128) ML_AS(128);
+    ML_AS(256);
+#undef ML_AS
 #undef ML_ARGS
 }
 
 }  // namespace
 
 // z [N, z_stride] holds q (H * D from q_col) and k (from k_col); gates [N, g_stride] float = [W_i h | W_f h]; outputs qf, kf [N, H, D],
-// ig, fg [N, H], all float.
+// ig, fg [N, H], all float; readers [num_readers] is set to zero.
 LLMIE_API int llmie_mlstm_prepare(const void* z, int z_stride, int q_col, int k_col, const float* gates, int g_stride, const float* bias_i,
-                                  const float* bias_f, float cap, float q_scale, float* qf, float* kf, float* ig, float* fg, int N, int H, int D,
-                                  int dtype, cudaStream_t s) {
+                                  const float* bias_f, float cap, float q_scale, float* qf, float* kf, float* ig, float* fg, int* readers, int num_readers,
+                                  int N, int H, int D, int dtype, cudaStream_t s) {
     if (N <= 0) return 0;
-    if (H <= 0 || D <= 0 || g_stride < 2 * H || q_col < 0 || k_col < 0 || !bias_i || !bias_f) return LLMIE_ERR_BAD_ARGUMENT;
+    if (H <= 0 || D <= 0 || g_stride < 2 * H || q_col < 0 || k_col < 0 || !bias_i || !bias_f || !readers) return LLMIE_ERR_BAD_ARGUMENT;
     if (dtype == DT_F32)
         return launch_kernel(mlstm_prepare_kernel<float>, dim3(N), dim3(128), 0, s, (const float*)z, z_stride, q_col, k_col, gates, g_stride, bias_i, bias_f,
-                             cap, q_scale, qf, kf, ig, fg, H, D);
+                             cap, q_scale, qf, kf, ig, fg, H, D, readers, num_readers);
     return launch_kernel(mlstm_prepare_kernel<bf16>, dim3(N), dim3(128), 0, s, (const bf16*)z, z_stride, q_col, k_col, gates, g_stride, bias_i, bias_f, cap,
-                         q_scale, qf, kf, ig, fg, H, D);
+                         q_scale, qf, kf, ig, fg, H, D, readers, num_readers);
 }
 
-// v: DV columns per head from v_col of rows of v_stride; state [slots, H, DV + 1, D], mstate [slots, H]; num [N, H, DV + 1], m_out [N, H].
+// v: DV columns per head from v_col of rows of v_stride; state [slots, H, DV + 1, D], mstate [slots, H]; num [N, H, DV + 1], m_out [N, H]; readers [R, H]: zeros.
 LLMIE_API int llmie_mlstm_scan(const void* v, int v_stride, int v_col, const float* qf, const float* kf, const float* ig, const float* fg, float* state,
-                               float* mstate, const int* seq_starts, const int* seq_slots, float* num, float* m_out, int H, int D, int DV, int R,
-                               int dtype, cudaStream_t s) {
+                               float* mstate, const int* seq_starts, const int* seq_slots, float* num, float* m_out, int* readers, int H, int D, int DV, int R,
+                               int max_rows, int dtype, cudaStream_t s) {
     if (R <= 0) return 0;
     if (H <= 0 || H > 65535 || R > 65535 || D <= 0 || D > 256 || DV <= 0) return LLMIE_ERR_BAD_ARGUMENT;
-    if (dtype == DT_F32) return launch_scan<float>((const float*)v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, H, D, DV, R, s);
-    return launch_scan<bf16>((const bf16*)v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, H, D, DV, R, s);
+    const bool alone = max_rows >= 64;   // a long walk: see launch_kernel_on
+    if (dtype == DT_F32) return launch_scan<float>((const float*)v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, readers, H, D, DV, R, alone, s);
+    return launch_scan<bf16>((const bf16*)v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, readers, H, D, DV, R, alone, s);
 }
 
 // gate: H * DV columns of rows of gate_stride (storage type); w [H * DV]; out [N, H * DV] of the storage type.

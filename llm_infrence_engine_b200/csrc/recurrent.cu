@@ -9,6 +9,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "scan_sums.cuh"
 
 namespace {
 
@@ -135,29 +136,29 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const T* __restrict_
 }
 
 // ------------------------------------------------------------------------------------------------
-// How both recurrences are laid out. Per head the state S is [D, DV] (D: key channels or state size). Its columns are
-// independent of one another, and within a column a token's work is a sum over D, which sets the length of the chain from one
-// token to the next: so PARTS lanes share a column (up to a whole warp for D of 128 and more), lane part j holding the entries
-// d = 4 PARTS i + 4 j + c (c < 4) in registers; a warp owns 32 / PARTS columns, a block of eight warps 8 times that; a token
-// costs D / PARTS steps per lane plus log2(PARTS) shuffles per sum. In memory a state is kept column by column ([DV][D]), so
-// that a lane's entries are 16-byte pieces and a column's lanes read one contiguous run. Tokens arrive in tiles of SCAN_TILE
-// through a two-stage ring in shared memory (the next tile lands while this one is worked on; rows padded with zeros to DMAX;
-// the parts of a step read contiguous 16-byte pieces: no bank conflict), and with them the block's columns of the token's
-// own input. The order of every sum is fixed by D alone, so a result does not depend on how many rows a step brings.
-constexpr int SCAN_TILE = 8;    // (16 measured 6 % faster on a prompt of 2,048 rows and 15 to 60 % slower on decoded tokens)
-constexpr int SCAN_THREADS = 256;
+// How the recurrences are laid out. Per head the state S is [D, DV] (D: key channels or state size). Its columns are
+// independent of one another, and within a column a token's work is a sum over D: PARTS lanes share a column, lane part j holding
+// the entries d = 4 PARTS i + 4 j + c (c < 4) of CPL columns side by side in registers, in pairs for the packed
+// multiply-add; a block is four warps. In memory a state is kept column by column ([DV][D]), so that a lane's entries are 16-byte
+// pieces and a column's lanes read one contiguous run. Tokens arrive in tiles of SCAN_TILE through a two-stage ring in shared
+// memory (the next tile lands while this one is worked on; rows padded with zeros to DMAX), and with them the block's
+// columns of the token's own input. PARTS depends on D alone and with it the order of every sum, so a result does not depend on
+// how many rows a step brings; CPL changes no sum, so it follows the number of columns of the step.
+//
+// A long walk is bound by what a token costs one warp: bytes from shared memory into registers (128 a cycle for the whole
+// multiprocessor, however many lanes read the same address), multiply-adds, and for the delta rule, whose update needs the token's own
+// sum, the chain multiply-adds -> shuffles -> update. So: few lanes to a column, several columns to a lane, the rows of the next
+// token loaded while this one is worked on, no branch between the tokens of a full tile, and sums that only a token's output
+// needs are not reduced token by token but PARTS of them at a time, each lane ending with one (parts_scatter). Measured (one
+// request of 2,048 tokens, bfloat16), with 32 and 16 lanes to one column before: delta rule, 16 heads of 128 x 128, 744 -> 487 us;
+// state space, 64 heads of 64 values and 128 states, 682 -> 509 us.
+constexpr int SCAN_TILE = 16;
+constexpr int SCAN_THREADS = 128;
 constexpr int SCAN_ALONE_ROWS = 64;   // steps whose longest request brings this many rows launch the scans alone
 
-// The most lanes that may share a column for a padded size DMAX (a lane holds at least one 16-byte piece), and the lanes that do:
-// as many as it takes to fill the device with one request's columns (heads x values), fewer where there are many columns, since every
-// halving of the lanes halves the shuffles and the warps. The choice depends on the model's sizes alone, never on the batch or on the
-// rows of a step: the order of a sum, and with it every bit of a result, is the same however a request is cut.
-static inline int scan_parts(int dmax, int columns) {
-    const int most = dmax >= 128 ? 32 : dmax / 4;
-    int parts = most;
-    while (parts > 8 && (long long)columns * parts > 65536) parts >>= 1;
-    return parts;
-}
+// lanes per column: the delta rule (16 entries a lane and column: its chain is shortest with few shuffles) and the others (8 entries)
+static inline __host__ __device__ constexpr int delta_parts(int dmax) { return dmax >= 256 ? 16 : (dmax >= 128 ? 8 : 4); }
+static inline __host__ __device__ constexpr int scan_parts(int dmax) { return dmax >= 32 ? dmax / 8 : 4; }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -165,11 +166,6 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-template <int PARTS> __device__ __forceinline__ float parts_sum(float v) {
-#pragma unroll
-    for (int o = 1; o < PARTS; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 // rows of `count` tokens, each D floats at src + (first + t) * stride, into dst[t][DMAX] (zeros beyond D)
 template <int DMAX>
@@ -217,39 +213,54 @@ __device__ __forceinline__ void store_column(const float* S, float* st, int part
         }
     }
 }
+template <int DPL, int PARTS>
+__device__ __forceinline__ void load_column(float2* S, const float* st, int part, int D, bool live, bool vec) {
+    float v[DPL];
+    load_column<DPL, PARTS>(v, st, part, D, live, vec);
+#pragma unroll
+    for (int i = 0; i < DPL / 2; ++i) S[i] = make_float2(v[2 * i], v[2 * i + 1]);
+}
+template <int DPL, int PARTS>
+__device__ __forceinline__ void store_column(const float2* S, float* st, int part, int D, bool vec) {
+    float v[DPL];
+#pragma unroll
+    for (int i = 0; i < DPL / 2; ++i) { v[2 * i] = S[i].x; v[2 * i + 1] = S[i].y; }
+    store_column<DPL, PARTS>(v, st, part, D, vec);
+}
 
 // The gated delta rule. For every token, in order:
 //   S <- decay (.) S (row d by decay[d]);  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q
-// With S' = decay (.) S both products of a token are taken from S' in one pass over the registers: r = S'^T k and S'^T q, and
-// then o = S'^T q + u (k . q), the last factor coming with the token. SCALAR: the decay is one number per token and head
-// (decay [N, H]) and comes with the token's other numbers instead of as a row of D.
-template <typename T, int DMAX, int PARTS, bool SCALAR>
+// With S' = decay (.) S both products of a token are taken from S': r = S'^T k and S'^T q, and then o = S'^T q + u (k . q), the last
+// factor coming with the token. SCALAR: the decay is one number per token and head (decay [N, H]) and comes with the token's other
+// numbers instead of as a row of D.
+template <typename T, int DMAX, int CPL, bool SCALAR>
 __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(const T* __restrict__ v, int v_stride, int v_col, const float* __restrict__ qn,
                                                                   const float* __restrict__ kn, const float* __restrict__ kq,
                                                                   const float* __restrict__ decay, const float* __restrict__ beta,
                                                                   float* __restrict__ state, const int* __restrict__ seq_starts,
                                                                   const int* __restrict__ seq_slots, float* __restrict__ out, int H, int G,
                                                                   int D, int DV) {
-    constexpr int DPL = DMAX / PARTS, COLS = SCAN_THREADS / PARTS;
+    constexpr int PARTS = delta_parts(DMAX), DPL = DMAX / PARTS, COLS = SCAN_THREADS / PARTS * CPL, P2 = DPL / 2, BATCH = PARTS / CPL;
     extern __shared__ __align__(16) float scan_smem[];
     float* k_s = scan_smem;                              // [2][SCAN_TILE][DMAX]
     float* q_s = k_s + 2 * SCAN_TILE * DMAX;
     float* g_s = q_s + 2 * SCAN_TILE * DMAX;
-    float* beta_s = g_s + 2 * SCAN_TILE * DMAX;          // [2][SCAN_TILE]
+    float* beta_s = g_s + (SCALAR ? 0 : 2 * SCAN_TILE * DMAX);   // [2][SCAN_TILE]
     float* kq_s = beta_s + 2 * SCAN_TILE;
     float* g1_s = kq_s + 2 * SCAN_TILE;                  // [2][SCAN_TILE]: the decay where it is one number per token
     float* v_s = g1_s + 2 * SCAN_TILE;                   // [2][SCAN_TILE][COLS]
     pdl_wait();
     const int part = threadIdx.x % PARTS;
-    const int col = blockIdx.x * COLS + threadIdx.x / PARTS;
+    const int my_col = threadIdx.x / PARTS * CPL;        // the first of the lane's CPL columns, within the block
+    const int col = blockIdx.x * COLS + my_col;
     const int h = blockIdx.y, r = blockIdx.z;
     const int g = h / (H / G);
-    const bool live = col < DV;
     const bool vec = (D & 3) == 0;
     const int s0 = seq_starts[r], s1 = seq_starts[r + 1];
-    float* st = state + (((size_t)seq_slots[r] * H + h) * DV + (live ? col : 0)) * D;
-    float S[DPL];
-    load_column<DPL, PARTS>(S, st, part, D, live, vec);
+    float* st = state + ((size_t)seq_slots[r] * H + h) * DV * D;
+    float2 S[CPL][P2];
+#pragma unroll
+    for (int u = 0; u < CPL; ++u) load_column<DPL, PARTS>(S[u], st + (size_t)min(col + u, DV - 1) * D, part, D, col + u < DV, vec);
     auto fetch = [&](int base, int buf) {   // the rows of a tile: asynchronous copies
         const int count = min(SCAN_TILE, s1 - base);
         fetch_rows<DMAX>(k_s + buf * SCAN_TILE * DMAX, kn + ((size_t)base * G + g) * D, (size_t)G * D, count, D, vec);
@@ -257,8 +268,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(const T* __res
         if constexpr (!SCALAR) fetch_rows<DMAX>(g_s + buf * SCAN_TILE * DMAX, decay + ((size_t)base * H + h) * D, (size_t)H * D, count, D, vec);
     };
     // A tile's numbers per token (beta, k . q) and the block's columns of v: loaded into registers a tile ahead, put into shared
-    // memory after the tile's work, so that nobody waits for them. Thread i < SCAN_TILE holds token i's two numbers; the
-    // threads from the end backwards hold v, VPT values each.
+    // memory before the tile's work. Thread i < SCAN_TILE holds token i's numbers; the threads from the end backwards hold v,
+    // VPT values each.
     constexpr int VPT = (SCAN_TILE * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
     float pre_beta = 0.f, pre_kq = 0.f, pre_g = 1.f, pre_v[VPT];
     auto load_small = [&](int base) {
@@ -287,80 +298,138 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(const T* __res
             if (j < SCAN_TILE * COLS) v_s[buf * SCAN_TILE * COLS + j] = pre_v[n];
         }
     };
-    const int my_col = threadIdx.x / PARTS;
     if (s0 < s1) {
         fetch(s0, 0);
         load_small(s0);
-        store_small(0);
     }
     cp_commit();
     int buf = 0;
     for (int base = s0; base < s1; base += SCAN_TILE, buf ^= 1) {
         const int count = min(SCAN_TILE, s1 - base);
-        const bool more = base + SCAN_TILE < s1;
-        if (more) {
+        store_small(buf);                      // (this stage's last readers passed the barrier of the tile between)
+        cp_wait<0>();
+        __syncthreads();                       // this tile is in shared memory, and everyone is done with the other stage
+        if (base + SCAN_TILE < s1) {
             fetch(base + SCAN_TILE, buf ^ 1);
             load_small(base + SCAN_TILE);
         }
         cp_commit();
-        cp_wait<1>();
-        __syncthreads();                       // this tile is in shared memory
         const float* kb = k_s + buf * SCAN_TILE * DMAX + 4 * part;
         const float* qb = q_s + buf * SCAN_TILE * DMAX + 4 * part;
         const float* gb = g_s + buf * SCAN_TILE * DMAX + 4 * part;
+        struct Row { float2 k[P2], q[P2], g[SCALAR ? 1 : P2]; };
+        auto load_row = [&](int t, Row& w) {
 #pragma unroll
-        for (int t = 0; t < SCAN_TILE; ++t) {
-            if (t < count) {
-                float rk0 = 0.f, rk1 = 0.f, rq0 = 0.f, rq1 = 0.f;
-                float g1 = 1.f;
-                if constexpr (SCALAR) g1 = g1_s[buf * SCAN_TILE + t];
-#pragma unroll
-                for (int i = 0; i < DPL / 4; ++i) {
-                    const float4 k4 = *reinterpret_cast<const float4*>(kb + t * DMAX + 4 * PARTS * i);
-                    const float4 q4 = *reinterpret_cast<const float4*>(qb + t * DMAX + 4 * PARTS * i);
-                    const float4 g4 = SCALAR ? make_float4(g1, g1, g1, g1) : *reinterpret_cast<const float4*>(gb + t * DMAX + 4 * PARTS * i);
-                    float* s = S + 4 * i;
-                    s[0] *= g4.x; s[1] *= g4.y; s[2] *= g4.z; s[3] *= g4.w;
-                    rk0 = fmaf(s[0], k4.x, rk0); rk1 = fmaf(s[1], k4.y, rk1); rk0 = fmaf(s[2], k4.z, rk0); rk1 = fmaf(s[3], k4.w, rk1);
-                    rq0 = fmaf(s[0], q4.x, rq0); rq1 = fmaf(s[1], q4.y, rq1); rq0 = fmaf(s[2], q4.z, rq0); rq1 = fmaf(s[3], q4.w, rq1);
+            for (int i = 0; i < DPL / 4; ++i) {
+                const float4 k4 = *reinterpret_cast<const float4*>(kb + t * DMAX + 4 * PARTS * i);
+                const float4 q4 = *reinterpret_cast<const float4*>(qb + t * DMAX + 4 * PARTS * i);
+                w.k[2 * i] = make_float2(k4.x, k4.y); w.k[2 * i + 1] = make_float2(k4.z, k4.w);
+                w.q[2 * i] = make_float2(q4.x, q4.y); w.q[2 * i + 1] = make_float2(q4.z, q4.w);
+                if constexpr (!SCALAR) {
+                    const float4 g4 = *reinterpret_cast<const float4*>(gb + t * DMAX + 4 * PARTS * i);
+                    w.g[2 * i] = make_float2(g4.x, g4.y); w.g[2 * i + 1] = make_float2(g4.z, g4.w);
                 }
-                const float rk = parts_sum<PARTS>(rk0 + rk1), rq = parts_sum<PARTS>(rq0 + rq1);
-                const float u = beta_s[buf * SCAN_TILE + t] * (v_s[(buf * SCAN_TILE + t) * COLS + my_col] - rk);
+            }
+            if constexpr (SCALAR) {
+                const float g1 = g1_s[buf * SCAN_TILE + t];
+                w.g[0] = make_float2(g1, g1);
+            }
+        };
+        // one token: rq[u] is this lane's share of S'^T q, u_out[u] the update, of its columns
+        auto token = [&](int t, const Row& w, float* rq, float* u_out) {
+            const float bt = beta_s[buf * SCAN_TILE + t];
+            float sk[CPL];
 #pragma unroll
-                for (int i = 0; i < DPL / 4; ++i) {
-                    const float4 k4 = *reinterpret_cast<const float4*>(kb + t * DMAX + 4 * PARTS * i);
-                    float* s = S + 4 * i;
-                    s[0] = fmaf(k4.x, u, s[0]); s[1] = fmaf(k4.y, u, s[1]); s[2] = fmaf(k4.z, u, s[2]); s[3] = fmaf(k4.w, u, s[3]);
+            for (int u = 0; u < CPL; ++u) {
+                float2 a[2];
+                a[0] = a[1] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < P2; ++i) {
+                    S[u][i] = mul2(S[u][i], w.g[SCALAR ? 0 : i]);
+                    a[i & 1] = fma2(S[u][i], w.k[i], a[i & 1]);
                 }
-                if (live && part == 0) out[(size_t)(base + t) * H * DV + h * DV + col] = fmaf(u, kq_s[buf * SCAN_TILE + t], rq);
+                sk[u] = (a[0].x + a[0].y) + (a[1].x + a[1].y);
+            }
+#pragma unroll
+            for (int u = 0; u < CPL; ++u) sk[u] = parts_sum<PARTS>(sk[u]);
+#pragma unroll
+            for (int u = 0; u < CPL; ++u) {   // (needs nothing of the sums above: runs while they travel)
+                float2 a[2];
+                a[0] = a[1] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < P2; ++i) a[i & 1] = fma2(S[u][i], w.q[i], a[i & 1]);
+                rq[u] = (a[0].x + a[0].y) + (a[1].x + a[1].y);
+            }
+#pragma unroll
+            for (int u = 0; u < CPL; ++u) {
+                const float x = bt * (v_s[(buf * SCAN_TILE + t) * COLS + my_col + u] - sk[u]);
+#pragma unroll
+                for (int i = 0; i < P2; ++i) S[u][i] = fma2(w.k[i], make_float2(x, x), S[u][i]);
+                u_out[u] = x;
+            }
+        };
+        float* o = out + (size_t)base * H * DV + h * DV + col;
+        if (count == SCAN_TILE) {
+            const int my_t = part / CPL, my_u = part % CPL;   // the sum of a batch that this lane ends with
+            Row now;
+            load_row(0, now);
+#pragma unroll
+            for (int t0 = 0; t0 < SCAN_TILE; t0 += BATCH) {
+                float rq[PARTS], u_mine = 0.f;
+#pragma unroll
+                for (int t = 0; t < BATCH; ++t) {
+                    Row next;
+                    if (t0 + t + 1 < SCAN_TILE) load_row(t0 + t + 1, next);
+                    float u[CPL];
+                    token(t0 + t, now, rq + t * CPL, u);
+#pragma unroll
+                    for (int c = 0; c < CPL; ++c)
+                        if (part == t * CPL + c) u_mine = u[c];
+                    now = next;
+                }
+                const float mine = parts_scatter<PARTS>(rq, part);
+                if (col + my_u < DV) o[(size_t)(t0 + my_t) * H * DV + my_u] = fmaf(u_mine, kq_s[buf * SCAN_TILE + t0 + my_t], mine);
+            }
+        } else {
+            for (int t = 0; t < count; ++t) {
+                Row now;
+                load_row(t, now);
+                float rq[CPL], u[CPL];
+                token(t, now, rq, u);
+#pragma unroll
+                for (int c = 0; c < CPL; ++c) {
+                    const float sum = parts_sum<PARTS>(rq[c]);
+                    if (col + c < DV && part == 0) o[(size_t)t * H * DV + c] = fmaf(u[c], kq_s[buf * SCAN_TILE + t], sum);
+                }
             }
         }
-        if (more) store_small(buf ^ 1);
-        __syncthreads();                       // everyone is done with this stage before it is filled again
     }
     cp_wait<0>();
     // Only now may the next kernel's blocks move in: they would wait for this kernel's end, and a multiprocessor full of
     // waiting warps slowed this kernel's own long walk by a third (measured).
     pdl_trigger();
-    if (live) store_column<DPL, PARTS>(S, st, part, D, vec);
+#pragma unroll
+    for (int u = 0; u < CPL; ++u)
+        if (col + u < DV) store_column<DPL, PARTS>(S[u], st + (size_t)(col + u) * D, part, D, vec);
 }
 
 // ------------------------------------------------------------------------------------------------
 // The state-space recurrence with one decay per head. Per head, S is [NS, DV]; for every token, in order:
 //   dt = softplus(dt_raw + dt_bias[h]);  S <- exp(-exp(A_log[h]) dt) S + dt B x^T;  y = S^T C + D[h] x
 // B and C belong to the head's group and come straight from the convolution's result (type T), so their tiles are filled with
-// plain loads a tile ahead; step size and decay are computed while a tile is loaded.
+// plain loads a tile ahead (four entries at a time where the rows allow it); step size and decay are computed as a tile is put into
+// shared memory.
 // FIXED: linear attention with a fixed decay per head, S <- decay[h] S + k v^T; y = S^T q. q, k and v stand in the places of C, B
 // and x (a head of their own each: G = H), pass silu as they are loaded, and there are neither step sizes nor a skip; A_log holds
 // the decays themselves.
-template <typename T, int NMAX, int PARTS, bool FIXED>
+template <typename T, int NMAX, int CPL, bool FIXED>
 __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restrict__ xbc, int x_stride, int x_col, int b_col, int c_col,
                                                                 const T* __restrict__ dt_raw, int dt_stride, const float* __restrict__ A_log,
                                                                 const float* __restrict__ dt_bias, const float* __restrict__ Dskip,
                                                                 float* __restrict__ state, const int* __restrict__ seq_starts,
                                                                 const int* __restrict__ seq_slots, float* __restrict__ out, int H, int G,
                                                                 int NS, int DV) {
-    constexpr int DPL = NMAX / PARTS, COLS = SCAN_THREADS / PARTS;
+    constexpr int PARTS = scan_parts(NMAX), DPL = NMAX / PARTS, COLS = SCAN_THREADS / PARTS * CPL, P2 = DPL / 2, BATCH = PARTS / CPL;
     extern __shared__ __align__(16) float scan_smem[];
     float* b_s = scan_smem;                              // [2][SCAN_TILE][NMAX]
     float* c_s = b_s + 2 * SCAN_TILE * NMAX;
@@ -368,32 +437,43 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
     float* dt_s = a_s + 2 * SCAN_TILE;
     float* x_s = dt_s + 2 * SCAN_TILE;                   // [2][SCAN_TILE][COLS]
     const int part = threadIdx.x % PARTS;
-    const int col = blockIdx.x * COLS + threadIdx.x / PARTS;
+    const int my_col = threadIdx.x / PARTS * CPL;        // the first of the lane's CPL columns, within the block
+    const int col = blockIdx.x * COLS + my_col;
     const int h = blockIdx.y, r = blockIdx.z;
     const int g = h / (H / G);
-    const bool live = col < DV;
     const bool vec = (NS & 3) == 0;
     const float rate = FIXED ? A_log[h] : expf(A_log[h]), bias = FIXED ? 0.f : dt_bias[h], skip = FIXED ? 0.f : Dskip[h];
     pdl_wait();
     const int s0 = seq_starts[r], s1 = seq_starts[r + 1];
-    float* st = state + (((size_t)seq_slots[r] * H + h) * DV + (live ? col : 0)) * NS;
-    float S[DPL];
-    load_column<DPL, PARTS>(S, st, part, NS, live, vec);
+    float* st = state + ((size_t)seq_slots[r] * H + h) * DV * NS;
+    float2 S[CPL][P2];
+#pragma unroll
+    for (int u = 0; u < CPL; ++u) load_column<DPL, PARTS>(S[u], st + (size_t)min(col + u, DV - 1) * NS, part, NS, col + u < DV, vec);
     // A tile (B and C of its tokens, step size and decay, the block's columns of x) is loaded into registers a tile ahead and
-    // put into shared memory after the tile's work, so that nobody waits for it.
-    constexpr int BPT = (SCAN_TILE * NMAX + SCAN_THREADS - 1) / SCAN_THREADS;
+    // put into shared memory before the tile's work.
+    constexpr int QPT = (SCAN_TILE * NMAX / 4 + SCAN_THREADS - 1) / SCAN_THREADS;
     constexpr int XPT = (SCAN_TILE * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
-    float pre_b[BPT], pre_c[BPT], pre_x[XPT], pre_dt = 0.f;
+    const bool vec_in = vec && (x_stride & 3) == 0 && (b_col & 3) == 0 && (c_col & 3) == 0 && ((uintptr_t)xbc & (4 * sizeof(T) - 1)) == 0;
+    float pre_b[QPT][4], pre_c[QPT][4], pre_x[XPT], pre_dt = 0.f;
     auto load_tile = [&](int base) {
         const int count = min(SCAN_TILE, s1 - base);
 #pragma unroll
-        for (int n = 0; n < BPT; ++n) {
+        for (int n = 0; n < QPT; ++n) {
             const int i = threadIdx.x + n * SCAN_THREADS;
-            const int t = i / NMAX, d = i % NMAX;
-            const bool in = t < count && d < NS;
-            const size_t row = (size_t)(base + t) * x_stride;
-            pre_b[n] = in ? to_f32(xbc[row + b_col + g * NS + d]) : 0.f;
-            pre_c[n] = in ? to_f32(xbc[row + c_col + g * NS + d]) : 0.f;
+            const int t = i / (NMAX / 4), d = i % (NMAX / 4) * 4;
+            const T* row = xbc + (size_t)(base + t) * x_stride + g * NS + d;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) pre_b[n][c] = pre_c[n][c] = 0.f;
+            if (t < count && d < NS) {
+                if (vec_in) {
+                    load4(row + b_col, pre_b[n]);
+                    load4(row + c_col, pre_c[n]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (d + c < NS) { pre_b[n][c] = to_f32(row[b_col + c]); pre_c[n][c] = to_f32(row[c_col + c]); }
+                }
+            }
         }
         if (!FIXED && threadIdx.x < count) pre_dt = to_f32(dt_raw[(size_t)(base + threadIdx.x) * dt_stride + h]);
 #pragma unroll
@@ -405,11 +485,15 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
     };
     auto store_tile = [&](int buf) {
 #pragma unroll
-        for (int n = 0; n < BPT; ++n) {
+        for (int n = 0; n < QPT; ++n) {
             const int i = threadIdx.x + n * SCAN_THREADS;
-            if (i < SCAN_TILE * NMAX) {
-                b_s[buf * SCAN_TILE * NMAX + i] = FIXED ? silu_f(pre_b[n]) : pre_b[n];   // (silu(0) = 0: the padding stays)
-                c_s[buf * SCAN_TILE * NMAX + i] = FIXED ? silu_f(pre_c[n]) : pre_c[n];
+            if (i < SCAN_TILE * NMAX / 4) {
+                if constexpr (FIXED) {   // (silu(0) = 0: the padding stays)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) { pre_b[n][c] = silu_f(pre_b[n][c]); pre_c[n][c] = silu_f(pre_c[n][c]); }
+                }
+                store4(b_s + buf * SCAN_TILE * NMAX + 4 * i, pre_b[n]);
+                store4(c_s + buf * SCAN_TILE * NMAX + 4 * i, pre_c[n]);
             }
         }
         if (!FIXED && threadIdx.x < SCAN_TILE) {
@@ -423,41 +507,82 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
             if (j < SCAN_TILE * COLS) x_s[buf * SCAN_TILE * COLS + j] = FIXED ? silu_f(pre_x[n]) : pre_x[n];
         }
     };
-    const int my_col = threadIdx.x / PARTS;
-    if (s0 < s1) {
-        load_tile(s0);
-        store_tile(0);
-    }
+    if (s0 < s1) load_tile(s0);
     int buf = 0;
     for (int base = s0; base < s1; base += SCAN_TILE, buf ^= 1) {
         const int count = min(SCAN_TILE, s1 - base);
-        const bool more = base + SCAN_TILE < s1;
-        __syncthreads();                       // this tile is in shared memory; everyone is done with the other stage
-        if (more) load_tile(base + SCAN_TILE);
+        store_tile(buf);                       // (this stage's last readers passed the barrier of the tile between)
+        __syncthreads();                       // this tile is in shared memory
+        if (base + SCAN_TILE < s1) load_tile(base + SCAN_TILE);
         const float* bb = b_s + buf * SCAN_TILE * NMAX + 4 * part;
         const float* cb = c_s + buf * SCAN_TILE * NMAX + 4 * part;
+        struct Row { float2 b[P2], c[P2]; };
+        auto load_row = [&](int t, Row& w) {
 #pragma unroll
-        for (int t = 0; t < SCAN_TILE; ++t) {
-            if (t < count) {
-                const float xv = x_s[(buf * SCAN_TILE + t) * COLS + my_col];
-                const float a = FIXED ? rate : a_s[buf * SCAN_TILE + t], u = FIXED ? xv : dt_s[buf * SCAN_TILE + t] * xv;
-                float y0 = 0.f, y1 = 0.f;
+            for (int i = 0; i < DPL / 4; ++i) {
+                const float4 b4 = *reinterpret_cast<const float4*>(bb + t * NMAX + 4 * PARTS * i);
+                const float4 c4 = *reinterpret_cast<const float4*>(cb + t * NMAX + 4 * PARTS * i);
+                w.b[2 * i] = make_float2(b4.x, b4.y); w.b[2 * i + 1] = make_float2(b4.z, b4.w);
+                w.c[2 * i] = make_float2(c4.x, c4.y); w.c[2 * i + 1] = make_float2(c4.z, c4.w);
+            }
+        };
+        auto token = [&](int t, const Row& w, float* y) {   // y[u]: this lane's share of S^T C of its columns
+            const float a = FIXED ? rate : a_s[buf * SCAN_TILE + t], dt = FIXED ? 1.f : dt_s[buf * SCAN_TILE + t];
+            const float2 a2 = make_float2(a, a);
 #pragma unroll
-                for (int i = 0; i < DPL / 4; ++i) {
-                    const float4 b4 = *reinterpret_cast<const float4*>(bb + t * NMAX + 4 * PARTS * i);
-                    const float4 c4 = *reinterpret_cast<const float4*>(cb + t * NMAX + 4 * PARTS * i);
-                    float* s = S + 4 * i;
-                    s[0] = fmaf(a, s[0], b4.x * u); s[1] = fmaf(a, s[1], b4.y * u); s[2] = fmaf(a, s[2], b4.z * u); s[3] = fmaf(a, s[3], b4.w * u);
-                    y0 = fmaf(s[0], c4.x, y0); y1 = fmaf(s[1], c4.y, y1); y0 = fmaf(s[2], c4.z, y0); y1 = fmaf(s[3], c4.w, y1);
+            for (int u = 0; u < CPL; ++u) {
+                const float xv = x_s[(buf * SCAN_TILE + t) * COLS + my_col + u];
+                const float in = FIXED ? xv : dt * xv;
+                const float2 in2 = make_float2(in, in);
+                float2 sum[2];
+                sum[0] = sum[1] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < P2; ++i) {
+                    S[u][i] = fma2(a2, S[u][i], mul2(w.b[i], in2));
+                    sum[i & 1] = fma2(S[u][i], w.c[i], sum[i & 1]);
                 }
-                const float y = parts_sum<PARTS>(y0 + y1);
-                if (live && part == 0) out[(size_t)(base + t) * H * DV + h * DV + col] = FIXED ? y : fmaf(skip, xv, y);
+                y[u] = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+            }
+        };
+        float* o = out + (size_t)base * H * DV + h * DV + col;
+        auto put = [&](int t, int u, float y) {
+            o[(size_t)t * H * DV + u] = FIXED ? y : fmaf(skip, x_s[(buf * SCAN_TILE + t) * COLS + my_col + u], y);
+        };
+        if (count == SCAN_TILE) {
+            const int my_t = part / CPL, my_u = part % CPL;   // the sum of a batch that this lane ends with
+            Row now;
+            load_row(0, now);
+#pragma unroll
+            for (int t0 = 0; t0 < SCAN_TILE; t0 += BATCH) {
+                float y[PARTS];
+#pragma unroll
+                for (int t = 0; t < BATCH; ++t) {
+                    Row next;
+                    if (t0 + t + 1 < SCAN_TILE) load_row(t0 + t + 1, next);
+                    token(t0 + t, now, y + t * CPL);
+                    now = next;
+                }
+                const float mine = parts_scatter<PARTS>(y, part);
+                if (col + my_u < DV) put(t0 + my_t, my_u, mine);
+            }
+        } else {
+            for (int t = 0; t < count; ++t) {
+                Row now;
+                load_row(t, now);
+                float y[CPL];
+                token(t, now, y);
+#pragma unroll
+                for (int u = 0; u < CPL; ++u) {
+                    const float sum = parts_sum<PARTS>(y[u]);
+                    if (col + u < DV && part == 0) put(t, u, sum);
+                }
             }
         }
-        if (more) store_tile(buf ^ 1);         // (the other stage: nobody reads it before the next barrier)
     }
     pdl_trigger();                             // (not before: see the delta rule's kernel)
-    if (live) store_column<DPL, PARTS>(S, st, part, NS, vec);
+#pragma unroll
+    for (int u = 0; u < CPL; ++u)
+        if (col + u < DV) store_column<DPL, PARTS>(S[u], st + (size_t)(col + u) * NS, part, NS, vec);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -467,14 +592,15 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
 // with A = -exp(A_log) [C, NS], B and C shared by all channels of a token. The result leaves as y * silu(z) in the storage type.
 // The layout is the one above with a channel in the place of a column: PARTS lanes share a channel, each with its entries of S and
 // of A in registers; a block owns SCAN_THREADS / PARTS channels; tiles of SCAN_TILE tokens are loaded into registers a tile ahead.
-template <typename T, int NMAX, int PARTS>
+// 2,048 channels, 16 states, eight prompts of 64 to 511 tokens (bfloat16), with step sizes waited for as they were loaded and a reduction per token before: 214 -> 105 us.
+template <typename T, int NMAX>
 __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* __restrict__ x, int x_stride, const T* __restrict__ dt_raw, int dt_stride,
                                                                       const T* __restrict__ bc, int bc_stride, int b_col, int c_col,
                                                                       const T* __restrict__ z, int z_stride, const float* __restrict__ A_log,
                                                                       const float* __restrict__ dt_bias, const float* __restrict__ Dskip,
                                                                       float* __restrict__ state, const int* __restrict__ seq_starts,
                                                                       const int* __restrict__ seq_slots, T* __restrict__ out, int C, int NS) {
-    constexpr int DPL = NMAX / PARTS, COLS = SCAN_THREADS / PARTS;
+    constexpr int PARTS = delta_parts(NMAX), DPL = NMAX / PARTS, COLS = SCAN_THREADS / PARTS;
     extern __shared__ __align__(16) float scan_smem[];
     float* b_s = scan_smem;                              // [2][SCAN_TILE][NMAX]
     float* c_s = b_s + 2 * SCAN_TILE * NMAX;
@@ -493,14 +619,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
 #pragma unroll
     for (int i = 0; i < DPL; ++i) A[i] = -expf(A[i]);
     const float skip = live ? Dskip[col] : 0.f;
+    constexpr int BPT = (SCAN_TILE * NMAX + SCAN_THREADS - 1) / SCAN_THREADS;
+    constexpr int XPT = (SCAN_TILE * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
+    float pre_b[BPT], pre_c[BPT], pre_x[XPT], pre_dt[XPT], pre_z[XPT];
+    // (a thread stages the same channel of the block in all its pieces: COLS divides the block)
+    const int stage_c = blockIdx.x * COLS + threadIdx.x % COLS;
+    const float bias = stage_c < C ? dt_bias[stage_c] : 0.f;
     pdl_wait();
     const int s0 = seq_starts[r], s1 = seq_starts[r + 1];
     float* st = state + ((size_t)seq_slots[r] * C + (live ? col : 0)) * NS;
     float S[DPL];
     load_column<DPL, PARTS>(S, st, part, NS, live, vec);
-    constexpr int BPT = (SCAN_TILE * NMAX + SCAN_THREADS - 1) / SCAN_THREADS;
-    constexpr int XPT = (SCAN_TILE * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
-    float pre_b[BPT], pre_c[BPT], pre_x[XPT], pre_dt[XPT], pre_z[XPT];
     auto load_tile = [&](int base) {
         const int count = min(SCAN_TILE, s1 - base);
 #pragma unroll
@@ -519,10 +648,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
             const bool in = j < count * COLS && c < C;
             pre_x[n] = in ? to_f32(x[(size_t)(base + t) * x_stride + c]) : 0.f;
             pre_z[n] = in ? to_f32(z[(size_t)(base + t) * z_stride + c]) : 0.f;
-            pre_dt[n] = in ? softplus_f(to_f32(dt_raw[(size_t)(base + t) * dt_stride + c]) + dt_bias[c]) : 0.f;
+            pre_dt[n] = in ? to_f32(dt_raw[(size_t)(base + t) * dt_stride + c]) : 0.f;
         }
     };
-    auto store_tile = [&](int buf) {
+    auto store_tile = [&](int buf) {   // step sizes and gates are taken here, a tile behind their loads, which nobody waits for
 #pragma unroll
         for (int n = 0; n < BPT; ++n) {
             const int i = threadIdx.x + n * SCAN_THREADS;
@@ -536,48 +665,56 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
             const int j = threadIdx.x + n * SCAN_THREADS;
             if (j < SCAN_TILE * COLS) {
                 x_s[buf * SCAN_TILE * COLS + j] = pre_x[n];
-                dt_s[buf * SCAN_TILE * COLS + j] = pre_dt[n];
-                z_s[buf * SCAN_TILE * COLS + j] = pre_z[n];
+                dt_s[buf * SCAN_TILE * COLS + j] = softplus_f(pre_dt[n] + bias);
+                z_s[buf * SCAN_TILE * COLS + j] = silu_f(pre_z[n]);
             }
         }
     };
-    if (s0 < s1) {
-        load_tile(s0);
-        store_tile(0);
-    }
+    if (s0 < s1) load_tile(s0);
     int buf = 0;
     for (int base = s0; base < s1; base += SCAN_TILE, buf ^= 1) {
         const int count = min(SCAN_TILE, s1 - base);
-        const bool more = base + SCAN_TILE < s1;
-        __syncthreads();                       // this tile is in shared memory; everyone is done with the other stage
-        if (more) load_tile(base + SCAN_TILE);
+        store_tile(buf);                       // (this stage's last readers passed the barrier of the tile between)
+        __syncthreads();                       // this tile is in shared memory
+        if (base + SCAN_TILE < s1) load_tile(base + SCAN_TILE);
         const float* bb = b_s + buf * SCAN_TILE * NMAX + 4 * part;
         const float* cb = c_s + buf * SCAN_TILE * NMAX + 4 * part;
+        auto token = [&](int t) {   // returns this lane's share of the channel's sum
+            const float xv = x_s[(buf * SCAN_TILE + t) * COLS + my_col];
+            const float dt = dt_s[(buf * SCAN_TILE + t) * COLS + my_col];
+            const float u = dt * xv;
+            float y0 = 0.f, y1 = 0.f;
 #pragma unroll
-        for (int t = 0; t < SCAN_TILE; ++t) {
-            if (t < count) {
-                const float xv = x_s[(buf * SCAN_TILE + t) * COLS + my_col];
-                const float dt = dt_s[(buf * SCAN_TILE + t) * COLS + my_col];
-                const float u = dt * xv;
-                float y0 = 0.f, y1 = 0.f;
+            for (int i = 0; i < DPL / 4; ++i) {
+                const float4 b4 = *reinterpret_cast<const float4*>(bb + t * NMAX + 4 * PARTS * i);
+                const float4 c4 = *reinterpret_cast<const float4*>(cb + t * NMAX + 4 * PARTS * i);
+                float* sp = S + 4 * i;
+                const float* ap = A + 4 * i;
+                sp[0] = fmaf(expf(dt * ap[0]), sp[0], b4.x * u); sp[1] = fmaf(expf(dt * ap[1]), sp[1], b4.y * u);
+                sp[2] = fmaf(expf(dt * ap[2]), sp[2], b4.z * u); sp[3] = fmaf(expf(dt * ap[3]), sp[3], b4.w * u);
+                y0 = fmaf(sp[0], c4.x, y0); y1 = fmaf(sp[1], c4.y, y1); y0 = fmaf(sp[2], c4.z, y0); y1 = fmaf(sp[3], c4.w, y1);
+            }
+            return y0 + y1;
+        };
+        auto put = [&](int t, float y) {
+            const int at = (buf * SCAN_TILE + t) * COLS + my_col;
+            out[(size_t)(base + t) * C + col] = from_f32<T>(fmaf(skip, x_s[at], y) * z_s[at]);
+        };
+        if (count == SCAN_TILE) {
 #pragma unroll
-                for (int i = 0; i < DPL / 4; ++i) {
-                    const float4 b4 = *reinterpret_cast<const float4*>(bb + t * NMAX + 4 * PARTS * i);
-                    const float4 c4 = *reinterpret_cast<const float4*>(cb + t * NMAX + 4 * PARTS * i);
-                    float* sp = S + 4 * i;
-                    const float* ap = A + 4 * i;
-                    sp[0] = fmaf(expf(dt * ap[0]), sp[0], b4.x * u); sp[1] = fmaf(expf(dt * ap[1]), sp[1], b4.y * u);
-                    sp[2] = fmaf(expf(dt * ap[2]), sp[2], b4.z * u); sp[3] = fmaf(expf(dt * ap[3]), sp[3], b4.w * u);
-                    y0 = fmaf(sp[0], c4.x, y0); y1 = fmaf(sp[1], c4.y, y1); y0 = fmaf(sp[2], c4.z, y0); y1 = fmaf(sp[3], c4.w, y1);
-                }
-                const float y = parts_sum<PARTS>(y0 + y1);
-                if (live && part == 0) {
-                    const float zv = z_s[(buf * SCAN_TILE + t) * COLS + my_col];
-                    out[(size_t)(base + t) * C + col] = from_f32<T>(fmaf(skip, xv, y) * silu_f(zv));
-                }
+            for (int t0 = 0; t0 < SCAN_TILE; t0 += PARTS) {
+                float y[PARTS];
+#pragma unroll
+                for (int t = 0; t < PARTS; ++t) y[t] = token(t0 + t);
+                const float mine = parts_scatter<PARTS>(y, part);
+                if (live) put(t0 + part, mine);
+            }
+        } else {
+            for (int t = 0; t < count; ++t) {
+                const float y = parts_sum<PARTS>(token(t));
+                if (live && part == 0) put(t, y);
             }
         }
-        if (more) store_tile(buf ^ 1);         // (the other stage: nobody reads it before the next barrier)
     }
     pdl_trigger();                             // (not before: see the delta rule's kernel)
     if (live) store_column<DPL, PARTS>(S, st, part, NS, vec);
@@ -591,61 +728,65 @@ int launch_conv(const T* z, int z_stride, int C, const float* w, const float* bi
                          out_stride, taps, act);
 }
 
-template <typename T, int DM, int PARTS, bool SCALAR>
+// Several columns to a lane as soon as one each would be more warps than the device has schedulers: the step's columns decide (a lane
+// with more of them makes each token longer, but reads the token's rows once for all).
+static inline bool many_columns(long long columns, int parts) { return columns * parts > 148LL * SCAN_THREADS * 2; }
+
+template <typename T, int DM, int CPL, bool SCALAR>
 int launch_delta_scan_one(const T* v, int v_stride, int v_col, const float* qn, const float* kn, const float* kq, const float* decay,
                           const float* beta, float* state, const int* seq_starts, const int* seq_slots, float* out, int H, int G, int D, int DV,
                           int R, bool alone, cudaStream_t s) {
-    constexpr int cols = SCAN_THREADS / PARTS;
+    constexpr int cols = SCAN_THREADS / delta_parts(DM) * CPL;
     const dim3 grid((DV + cols - 1) / cols, H, R);
-    const size_t smem = sizeof(float) * (2 * SCAN_TILE * (3 * DM + 3 + cols));
-    if (smem > 48 * 1024) cudaFuncSetAttribute(delta_scan_kernel<T, DM, PARTS, SCALAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_kernel_on(alone, delta_scan_kernel<T, DM, PARTS, SCALAR>, grid, dim3(SCAN_THREADS), smem, s, v, v_stride, v_col, qn, kn, kq, decay,
+    const size_t smem = sizeof(float) * (2 * SCAN_TILE * ((SCALAR ? 2 : 3) * DM + 3 + cols));
+    if (smem > 48 * 1024) cudaFuncSetAttribute(delta_scan_kernel<T, DM, CPL, SCALAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return launch_kernel_on(alone, delta_scan_kernel<T, DM, CPL, SCALAR>, grid, dim3(SCAN_THREADS), smem, s, v, v_stride, v_col, qn, kn, kq, decay,
                             beta, state, seq_starts, seq_slots, out, H, G, D, DV);
 }
 
-template <typename T, int DM, int PARTS>
+template <typename T, int DM>
 int launch_delta_scan_as(const T* v, int v_stride, int v_col, const float* qn, const float* kn, const float* kq, const float* decay,
                          const float* beta, float* state, const int* seq_starts, const int* seq_slots, float* out, int H, int G, int D, int DV,
                          int R, bool alone, bool scalar, cudaStream_t s) {
-    if (scalar)
-        return launch_delta_scan_one<T, DM, PARTS, true>(v, v_stride, v_col, qn, kn, kq, decay, beta, state, seq_starts, seq_slots, out, H, G, D, DV, R, alone, s);
-    return launch_delta_scan_one<T, DM, PARTS, false>(v, v_stride, v_col, qn, kn, kq, decay, beta, state, seq_starts, seq_slots, out, H, G, D, DV, R, alone, s);
+#define LLMIE_DELTA_ARGS v, v_stride, v_col, qn, kn, kq, decay, beta, state, seq_starts, seq_slots, out, H, G, D, DV, R, alone, s
+    if (many_columns((long long)R * H * DV, delta_parts(DM)))
+        return scalar ? launch_delta_scan_one<T, DM, 2, true>(LLMIE_DELTA_ARGS) : launch_delta_scan_one<T, DM, 2, false>(LLMIE_DELTA_ARGS);
+    return scalar ? launch_delta_scan_one<T, DM, 1, true>(LLMIE_DELTA_ARGS) : launch_delta_scan_one<T, DM, 1, false>(LLMIE_DELTA_ARGS);
+#undef LLMIE_DELTA_ARGS
 }
 
-template <typename T, int NM, int PARTS, bool FIXED>
+template <typename T, int NM, int CPL, bool FIXED>
 int launch_ssm_scan_one(const T* xbc, int x_stride, int x_col, int b_col, int c_col, const T* dt_raw, int dt_stride, const float* A_log,
                        const float* dt_bias, const float* Dskip, float* state, const int* seq_starts, const int* seq_slots, float* out, int H,
                        int G, int NS, int DV, int R, bool alone, cudaStream_t s) {
-    constexpr int cols = SCAN_THREADS / PARTS;
+    constexpr int cols = SCAN_THREADS / scan_parts(NM) * CPL;
     const dim3 grid((DV + cols - 1) / cols, H, R);
     const size_t smem = sizeof(float) * (2 * SCAN_TILE * (2 * NM + 2 + cols));
-    if (smem > 48 * 1024) cudaFuncSetAttribute(ssm_scan_kernel<T, NM, PARTS, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_kernel_on(alone, ssm_scan_kernel<T, NM, PARTS, FIXED>, grid, dim3(SCAN_THREADS), smem, s, xbc, x_stride, x_col, b_col, c_col, dt_raw,
+    if (smem > 48 * 1024) cudaFuncSetAttribute(ssm_scan_kernel<T, NM, CPL, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return launch_kernel_on(alone, ssm_scan_kernel<T, NM, CPL, FIXED>, grid, dim3(SCAN_THREADS), smem, s, xbc, x_stride, x_col, b_col, c_col, dt_raw,
                             dt_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, out, H, G, NS, DV);
 }
 
-template <typename T, int NM, int PARTS>
+template <typename T, int NM>
 int launch_ssm_scan_as(const T* xbc, int x_stride, int x_col, int b_col, int c_col, const T* dt_raw, int dt_stride, const float* A_log,
                        const float* dt_bias, const float* Dskip, float* state, const int* seq_starts, const int* seq_slots, float* out, int H,
                        int G, int NS, int DV, int R, bool alone, cudaStream_t s) {
+#define LLMIE_SSM_ARGS xbc, x_stride, x_col, b_col, c_col, dt_raw, dt_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, out, H, G, NS, DV, R, alone, s
+    const bool many = many_columns((long long)R * H * DV, scan_parts(NM));
     if (!dt_raw)   // no step sizes: the fixed decays of linear attention
-        return launch_ssm_scan_one<T, NM, PARTS, true>(xbc, x_stride, x_col, b_col, c_col, dt_raw, dt_stride, A_log, dt_bias, Dskip, state, seq_starts,
-                                                       seq_slots, out, H, G, NS, DV, R, alone, s);
-    return launch_ssm_scan_one<T, NM, PARTS, false>(xbc, x_stride, x_col, b_col, c_col, dt_raw, dt_stride, A_log, dt_bias, Dskip, state, seq_starts,
-                                                    seq_slots, out, H, G, NS, DV, R, alone, s);
+        return many ? launch_ssm_scan_one<T, NM, 4, true>(LLMIE_SSM_ARGS) : launch_ssm_scan_one<T, NM, 2, true>(LLMIE_SSM_ARGS);
+    return many ? launch_ssm_scan_one<T, NM, 4, false>(LLMIE_SSM_ARGS) : launch_ssm_scan_one<T, NM, 2, false>(LLMIE_SSM_ARGS);
+#undef LLMIE_SSM_ARGS
 }
 
-// the padded size (16, 32, 64, 128 or 256) and the lanes per column (scan_parts) pick the instantiation
-#define LLMIE_SCAN_DISPATCH(FN, SIZE, ...)                                                    \
-    {                                                                                         \
-        const int dm = SIZE <= 16 ? 16 : SIZE <= 32 ? 32 : SIZE <= 64 ? 64 : SIZE <= 128 ? 128 : 256; \
-        const int parts = scan_parts(dm, H * DV);                                             \
-        if (dm == 16) return FN<T, 16, 4>(__VA_ARGS__);                                       \
-        if (dm == 32) return FN<T, 32, 8>(__VA_ARGS__);                                       \
-        if (dm == 64) return parts == 16 ? FN<T, 64, 16>(__VA_ARGS__) : FN<T, 64, 8>(__VA_ARGS__); \
-        if (dm == 128)                                                                        \
-            return parts == 32 ? FN<T, 128, 32>(__VA_ARGS__) : parts == 16 ? FN<T, 128, 16>(__VA_ARGS__) : FN<T, 128, 8>(__VA_ARGS__); \
-        return parts == 32 ? FN<T, 256, 32>(__VA_ARGS__) : parts == 16 ? FN<T, 256, 16>(__VA_ARGS__) : FN<T, 256, 8>(__VA_ARGS__); \
+// the padded size (16, 32, 64, 128 or 256) picks the instantiation
+#define LLMIE_SCAN_DISPATCH(FN, SIZE, ...)              \
+    {                                                   \
+        if (SIZE <= 16) return FN<T, 16>(__VA_ARGS__);   \
+        if (SIZE <= 32) return FN<T, 32>(__VA_ARGS__);   \
+        if (SIZE <= 64) return FN<T, 64>(__VA_ARGS__);   \
+        if (SIZE <= 128) return FN<T, 128>(__VA_ARGS__); \
+        return FN<T, 256>(__VA_ARGS__);                  \
     }
 
 template <typename T>
@@ -663,15 +804,15 @@ int launch_ssm_scan(const T* xbc, int x_stride, int x_col, int b_col, int c_col,
                         seq_slots, out, H, G, NS, DV, R, alone, s)
 }
 
-template <typename T, int NM, int PARTS>
+template <typename T, int NM>
 int launch_selective_scan_as(const T* x, int x_stride, const T* dt_raw, int dt_stride, const T* bc, int bc_stride, int b_col, int c_col, const T* z,
                              int z_stride, const float* A_log, const float* dt_bias, const float* Dskip, float* state, const int* seq_starts,
                              const int* seq_slots, T* out, int C, int NS, int R, bool alone, cudaStream_t s) {
-    constexpr int cols = SCAN_THREADS / PARTS;
+    constexpr int cols = SCAN_THREADS / delta_parts(NM);
     const dim3 grid((C + cols - 1) / cols, 1, R);
     const size_t smem = sizeof(float) * (2 * SCAN_TILE * (2 * NM + 3 * cols));
-    if (smem > 48 * 1024) cudaFuncSetAttribute(selective_scan_kernel<T, NM, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_kernel_on(alone, selective_scan_kernel<T, NM, PARTS>, grid, dim3(SCAN_THREADS), smem, s, x, x_stride, dt_raw, dt_stride, bc, bc_stride,
+    if (smem > 48 * 1024) cudaFuncSetAttribute(selective_scan_kernel<T, NM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return launch_kernel_on(alone, selective_scan_kernel<T, NM>, grid, dim3(SCAN_THREADS), smem, s, x, x_stride, dt_raw, dt_stride, bc, bc_stride,
                             b_col, c_col, z, z_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, out, C, NS);
 }
 
@@ -679,7 +820,6 @@ template <typename T>
 int launch_selective_scan(const T* x, int x_stride, const T* dt_raw, int dt_stride, const T* bc, int bc_stride, int b_col, int c_col, const T* z,
                           int z_stride, const float* A_log, const float* dt_bias, const float* Dskip, float* state, const int* seq_starts,
                           const int* seq_slots, T* out, int C, int NS, int R, bool alone, cudaStream_t s) {
-    const int H = C, DV = 1;   // (the channels are the columns that fill the device)
     LLMIE_SCAN_DISPATCH(launch_selective_scan_as, NS, x, x_stride, dt_raw, dt_stride, bc, bc_stride, b_col, c_col, z, z_stride, A_log, dt_bias, Dskip,
                         state, seq_starts, seq_slots, out, C, NS, R, alone, s)
 }

@@ -131,6 +131,29 @@ def test_matrix_memory_against_the_cell_written_out_and_whatever_the_cut(K):
         assert torch.equal(run(cuts_of(N, sizes)), whole), f"portions of {sizes} give other bits"
 
 
+@pytest.mark.parametrize("D", [16, 40, 64, 128, 132, 256])
+@pytest.mark.parametrize("R", [1, 150])
+def test_matrix_memory_whatever_the_columns_per_lane(K, D, R):
+    """Each padded key size, with few columns in the step (two to a group of lanes) and with many (four): a request has the same bits alone
+    and among 150, whole and cut inside a tile of 16 tokens."""
+    H, DV, N = 2, 33, 37
+    z, (qc, kc, vc, gc), gates, bi, bf, nw = memory_inputs(N, H, D, DV, "float32", seed=D)
+
+    def run(cuts, many):
+        S, M = torch.zeros(many + 1, H, DV + 1, D).cuda(), torch.zeros(many + 1, H).cuda()
+        outs = []
+        for lo, hi in cuts:
+            _, dev = ragged([hi - lo] * many, list(range(many)))
+            num, m = K.mlstm(z[lo:hi].repeat(many, 1).cuda(), qc, kc, vc, gates[lo:hi].repeat(many, 1).cuda(), bi.cuda(), bf.cuda(), 5.0, H, D, DV, S, M, dev)
+            outs.append(torch.cat([num.flatten(1), m], dim=1).view(many, hi - lo, -1))
+        return torch.cat(outs, dim=1), S[:many], M[:many]
+
+    one = run([(0, N)], 1)
+    for got in (run([(0, N)], R), run([(0, 16), (16, 19), (19, 37)], R)):
+        for a, b in zip(got, one):
+            assert torch.equal(a, b.expand_as(a))
+
+
 def test_matrix_memory_reads_back_a_far_write(K):
     """Token 0 is written with an open input gate; 400 tokens follow whose input gates are shut and whose forget gates are open; the
     last token asks with token 0's key: it gets token 0's value back, through a state that was carried over 40 steps of a slot

@@ -218,6 +218,37 @@ def test_state_space_scan_over_ragged_steps(K, dtype, H, G, NS, DV):
         close(dstate, state, "float32", f"ssm_scan state after step {step}", f32=1e-5)
 
 
+@pytest.mark.parametrize("D", [16, 40, 128, 132, 256])
+@pytest.mark.parametrize("kind", ["delta", "delta, one decay per head", "state space"])
+def test_scans_whatever_the_columns_per_lane(K, kind, D):
+    """Each padded size, with few columns in the step (one or two to a group of lanes) and with many (two or four): a request has the same
+    bits alone and among 100, whole and cut inside a tile of 16 tokens."""
+    H, DV, N, many = 4, 33, 37, 100
+    qkv, dt = rnd(N, 2 * H * D + H * DV, seed=1), rnd(N, H, seed=2)
+    per_head = "one" in kind
+    a, b = rnd(N, H if per_head else H * D, seed=3), rnd(N, H, seed=4)
+    A_log, bias, skip = rnd(H, seed=5).cuda() * 0.3, rnd(H if per_head or kind == "state space" else H * D, seed=6).cuda(), rnd(H, seed=7).cuda()
+
+    def run(cuts, R):
+        state = torch.zeros(R + 1, H, DV, D).cuda()
+        outs = []
+        for lo, hi in cuts:
+            _, dev = ragged([hi - lo] * R, list(range(R)))
+            rows = [t[lo:hi].repeat(R, 1).cuda() for t in (qkv, a, b, dt)]
+            if kind == "state space":
+                x = rows[0][:, :H * DV + 2 * D].contiguous()
+                y = K.ssm_scan(x, H, 1, D, DV, rows[3], 0, A_log, bias, skip, state, dev)
+            else:
+                y = K.delta_rule(rows[0], H, H, D, DV, rows[1], rows[2], 0, A_log, bias, state, dev, decay_per_head=per_head)
+            outs.append(y.view(R, hi - lo, -1))
+        return torch.cat(outs, dim=1), state[:R]
+
+    one = run([(0, N)], 1)
+    for got in (run([(0, N)], many), run([(0, 16), (16, 19), (19, 37)], many), run([(0, 5), (5, N)], 1)):
+        for x, y in zip(got, one):
+            assert torch.equal(x, y.expand_as(x))
+
+
 def paged(N_ctx, page, nkv, dk, dv, dtype, seed=0):
     """A pool with one request of ``N_ctx`` tokens on shuffled pages; returns pools, block table and the keys/values in order."""
     pages = -(-N_ctx // page)
