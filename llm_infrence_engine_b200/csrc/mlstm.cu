@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(128) mlstm_prepare_kernel(const T* __restrict_
 //
 // The walk is bound by a token's instructions on one warp (its latency hides behind the next token's, nothing feeds back): with four
 // columns to a group of 16 lanes on 80 blocks, a branch per token and the gates between two tiles on the first of the four warps, a
-// prompt of 1,301 tokens (8 heads of 128 x 128, beside one of 700) took 659 us; this form 162 us.
+// prompt of 1,301 tokens (8 heads of 128 x 128, beside one of 700) took 659 us; this form 140 us.
 //
 // The request's m is read by every block of its (h, r) and written by one: the block that is the LAST to have read it, as `readers`
 // (zeroed by the prepare kernel) tells, so that no block that starts late reads what an early one left.
@@ -182,23 +182,22 @@ __global__ void __launch_bounds__(ML_THREADS + 32) mlstm_scan_kernel(const T* __
     };
     // the block's columns of v, into registers a tile ahead
     constexpr int VPT = (ML_TILE * COLS + ML_THREADS - 1) / ML_THREADS;
-    float pre_v[VPT];
+    T pre_v[VPT];   // (as they are stored: converted here, they would be waited for here)
     auto load_v = [&](int base) {
         const int count = min(ML_TILE, s1 - base);
 #pragma unroll
         for (int n = 0; n < VPT; ++n) {
             const int j = threadIdx.x + n * ML_THREADS;
             const int t = j / COLS, c = blockIdx.x * COLS + j % COLS;
-            float x = 0.f;
-            if (j < count * COLS) x = c < DV ? to_f32(v[(size_t)(base + t) * v_stride + v_col + h * DV + c]) : (c == DV ? 1.f : 0.f);
-            pre_v[n] = x;
+            pre_v[n] = from_f32<T>(c == DV ? 1.f : 0.f);
+            if (j < count * COLS && c < DV) pre_v[n] = v[(size_t)(base + t) * v_stride + v_col + h * DV + c];
         }
     };
     auto store_v = [&](int buf) {
 #pragma unroll
         for (int n = 0; n < VPT; ++n) {
             const int j = threadIdx.x + n * ML_THREADS;
-            if (j < ML_TILE * COLS) v_s[buf * ML_TILE * COLS + j] = pre_v[n];
+            if (j < ML_TILE * COLS) v_s[buf * ML_TILE * COLS + j] = to_f32(pre_v[n]);
         }
     };
     if (s0 < s1) {

@@ -150,8 +150,8 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const T* __restrict_
 // sum, the chain multiply-adds -> shuffles -> update. So: few lanes to a column, several columns to a lane, the rows of the next
 // token loaded while this one is worked on, no branch between the tokens of a full tile, and sums that only a token's output
 // needs are not reduced token by token but PARTS of them at a time, each lane ending with one (parts_scatter). Measured (one
-// request of 2,048 tokens, bfloat16), with 32 and 16 lanes to one column before: delta rule, 16 heads of 128 x 128, 744 -> 487 us;
-// state space, 64 heads of 64 values and 128 states, 682 -> 509 us.
+// request of 2,048 tokens, bfloat16), with 32 and 16 lanes to one column before: delta rule, 16 heads of 128 x 128, 744 -> 432 us;
+// state space, 64 heads of 64 values and 128 states, 682 -> 320 us.
 constexpr int SCAN_TILE = 16;
 constexpr int SCAN_THREADS = 128;
 constexpr int SCAN_ALONE_ROWS = 64;   // steps whose longest request brings this many rows launch the scans alone
@@ -228,6 +228,29 @@ __device__ __forceinline__ void store_column(const float2* S, float* st, int par
     store_column<DPL, PARTS>(v, st, part, D, vec);
 }
 
+// four neighbouring elements as they are stored (taking them apart is left to their use, like converting them)
+template <typename T> struct Four;
+template <> struct Four<float> {
+    float4 w;
+    __device__ __forceinline__ void clear() { w = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ void load(const float* p) { w = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void set(int c, float x) { if (c == 0) w.x = x; else if (c == 1) w.y = x; else if (c == 2) w.z = x; else w.w = x; }
+    __device__ __forceinline__ float get(int c) const { return c == 0 ? w.x : (c == 1 ? w.y : (c == 2 ? w.z : w.w)); }
+};
+template <> struct Four<bf16> {
+    uint2 w;
+    __device__ __forceinline__ void clear() { w = make_uint2(0u, 0u); }
+    __device__ __forceinline__ void load(const bf16* p) { w = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void set(int c, bf16 x) {
+        const uint32_t bits = (uint32_t)__bfloat16_as_ushort(x) << (16 * (c & 1));
+        if (c < 2) w.x |= bits; else w.y |= bits;   // (after clear())
+    }
+    __device__ __forceinline__ float get(int c) const {
+        const uint32_t t = c < 2 ? w.x : w.y;
+        return __uint_as_float((c & 1) ? t & 0xffff0000u : t << 16);
+    }
+};
+
 // The gated delta rule. For every token, in order:
 //   S <- decay (.) S (row d by decay[d]);  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q
 // With S' = decay (.) S both products of a token are taken from S': r = S'^T k and S'^T q, and then o = S'^T q + u (k . q), the last
@@ -271,7 +294,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(const T* __res
     // memory before the tile's work. Thread i < SCAN_TILE holds token i's numbers; the threads from the end backwards hold v,
     // VPT values each.
     constexpr int VPT = (SCAN_TILE * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
-    float pre_beta = 0.f, pre_kq = 0.f, pre_g = 1.f, pre_v[VPT];
+    float pre_beta = 0.f, pre_kq = 0.f, pre_g = 1.f;
+    T pre_v[VPT];   // (as they are stored: converted here, they would be waited for here)
     auto load_small = [&](int base) {
         const int count = min(SCAN_TILE, s1 - base);
         if (threadIdx.x < count) {
@@ -283,7 +307,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(const T* __res
         for (int n = 0; n < VPT; ++n) {
             const int j = SCAN_THREADS - 1 - threadIdx.x + n * SCAN_THREADS;
             const int t = j / COLS, c = blockIdx.x * COLS + j % COLS;
-            pre_v[n] = (j < count * COLS && c < DV) ? to_f32(v[(size_t)(base + t) * v_stride + v_col + h * DV + c]) : 0.f;
+            pre_v[n] = (j < count * COLS && c < DV) ? v[(size_t)(base + t) * v_stride + v_col + h * DV + c] : from_f32<T>(0.f);
         }
     };
     auto store_small = [&](int buf) {
@@ -295,7 +319,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(const T* __res
 #pragma unroll
         for (int n = 0; n < VPT; ++n) {
             const int j = SCAN_THREADS - 1 - threadIdx.x + n * SCAN_THREADS;
-            if (j < SCAN_TILE * COLS) v_s[buf * SCAN_TILE * COLS + j] = pre_v[n];
+            if (j < SCAN_TILE * COLS) v_s[buf * SCAN_TILE * COLS + j] = to_f32(pre_v[n]);
         }
     };
     if (s0 < s1) {
@@ -449,12 +473,13 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
     float2 S[CPL][P2];
 #pragma unroll
     for (int u = 0; u < CPL; ++u) load_column<DPL, PARTS>(S[u], st + (size_t)min(col + u, DV - 1) * NS, part, NS, col + u < DV, vec);
-    // A tile (B and C of its tokens, step size and decay, the block's columns of x) is loaded into registers a tile ahead and
-    // put into shared memory before the tile's work.
+    // A tile (B and C of its tokens, step size and decay, the block's columns of x) is loaded into registers a tile ahead, as it is
+    // stored (converted at once it would be waited for at once: half of the walk), and put into shared memory before the tile's work.
     constexpr int QPT = (SCAN_TILE * NMAX / 4 + SCAN_THREADS - 1) / SCAN_THREADS;
     constexpr int XPT = (SCAN_TILE * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
     const bool vec_in = vec && (x_stride & 3) == 0 && (b_col & 3) == 0 && (c_col & 3) == 0 && ((uintptr_t)xbc & (4 * sizeof(T) - 1)) == 0;
-    float pre_b[QPT][4], pre_c[QPT][4], pre_x[XPT], pre_dt = 0.f;
+    Four<T> pre_b[QPT], pre_c[QPT];
+    T pre_x[XPT], pre_dt = from_f32<T>(0.f);
     auto load_tile = [&](int base) {
         const int count = min(SCAN_TILE, s1 - base);
 #pragma unroll
@@ -462,25 +487,25 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
             const int i = threadIdx.x + n * SCAN_THREADS;
             const int t = i / (NMAX / 4), d = i % (NMAX / 4) * 4;
             const T* row = xbc + (size_t)(base + t) * x_stride + g * NS + d;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) pre_b[n][c] = pre_c[n][c] = 0.f;
+            pre_b[n].clear();
+            pre_c[n].clear();
             if (t < count && d < NS) {
                 if (vec_in) {
-                    load4(row + b_col, pre_b[n]);
-                    load4(row + c_col, pre_c[n]);
+                    pre_b[n].load(row + b_col);
+                    pre_c[n].load(row + c_col);
                 } else {
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
-                        if (d + c < NS) { pre_b[n][c] = to_f32(row[b_col + c]); pre_c[n][c] = to_f32(row[c_col + c]); }
+                        if (d + c < NS) { pre_b[n].set(c, row[b_col + c]); pre_c[n].set(c, row[c_col + c]); }
                 }
             }
         }
-        if (!FIXED && threadIdx.x < count) pre_dt = to_f32(dt_raw[(size_t)(base + threadIdx.x) * dt_stride + h]);
+        if (!FIXED && threadIdx.x < count) pre_dt = dt_raw[(size_t)(base + threadIdx.x) * dt_stride + h];
 #pragma unroll
         for (int n = 0; n < XPT; ++n) {
             const int j = SCAN_THREADS - 1 - threadIdx.x + n * SCAN_THREADS;
             const int t = j / COLS, c = blockIdx.x * COLS + j % COLS;
-            pre_x[n] = (j < count * COLS && c < DV) ? to_f32(xbc[(size_t)(base + t) * x_stride + x_col + h * DV + c]) : 0.f;
+            pre_x[n] = (j < count * COLS && c < DV) ? xbc[(size_t)(base + t) * x_stride + x_col + h * DV + c] : from_f32<T>(0.f);
         }
     };
     auto store_tile = [&](int buf) {
@@ -488,23 +513,26 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
         for (int n = 0; n < QPT; ++n) {
             const int i = threadIdx.x + n * SCAN_THREADS;
             if (i < SCAN_TILE * NMAX / 4) {
-                if constexpr (FIXED) {   // (silu(0) = 0: the padding stays)
+                float b4[4], c4[4];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) { pre_b[n][c] = silu_f(pre_b[n][c]); pre_c[n][c] = silu_f(pre_c[n][c]); }
+                for (int c = 0; c < 4; ++c) {   // (silu(0) = 0: the padding stays)
+                    b4[c] = pre_b[n].get(c);
+                    c4[c] = pre_c[n].get(c);
+                    if constexpr (FIXED) { b4[c] = silu_f(b4[c]); c4[c] = silu_f(c4[c]); }
                 }
-                store4(b_s + buf * SCAN_TILE * NMAX + 4 * i, pre_b[n]);
-                store4(c_s + buf * SCAN_TILE * NMAX + 4 * i, pre_c[n]);
+                store4(b_s + buf * SCAN_TILE * NMAX + 4 * i, b4);
+                store4(c_s + buf * SCAN_TILE * NMAX + 4 * i, c4);
             }
         }
         if (!FIXED && threadIdx.x < SCAN_TILE) {
-            const float dt = softplus_f(pre_dt + bias);
+            const float dt = softplus_f(to_f32(pre_dt) + bias);
             dt_s[buf * SCAN_TILE + threadIdx.x] = dt;
             a_s[buf * SCAN_TILE + threadIdx.x] = expf(-rate * dt);
         }
 #pragma unroll
         for (int n = 0; n < XPT; ++n) {
             const int j = SCAN_THREADS - 1 - threadIdx.x + n * SCAN_THREADS;
-            if (j < SCAN_TILE * COLS) x_s[buf * SCAN_TILE * COLS + j] = FIXED ? silu_f(pre_x[n]) : pre_x[n];
+            if (j < SCAN_TILE * COLS) x_s[buf * SCAN_TILE * COLS + j] = FIXED ? silu_f(to_f32(pre_x[n])) : to_f32(pre_x[n]);
         }
     };
     if (s0 < s1) load_tile(s0);
@@ -621,7 +649,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
     const float skip = live ? Dskip[col] : 0.f;
     constexpr int BPT = (SCAN_TILE * NMAX + SCAN_THREADS - 1) / SCAN_THREADS;
     constexpr int XPT = (SCAN_TILE * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
-    float pre_b[BPT], pre_c[BPT], pre_x[XPT], pre_dt[XPT], pre_z[XPT];
+    T pre_b[BPT], pre_c[BPT], pre_x[XPT], pre_dt[XPT], pre_z[XPT];   // (as they are stored: see above)
     // (a thread stages the same channel of the block in all its pieces: COLS divides the block)
     const int stage_c = blockIdx.x * COLS + threadIdx.x % COLS;
     const float bias = stage_c < C ? dt_bias[stage_c] : 0.f;
@@ -638,17 +666,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
             const int t = i / NMAX, d = i % NMAX;
             const bool in = t < count && d < NS;
             const size_t row = (size_t)(base + t) * bc_stride;
-            pre_b[n] = in ? to_f32(bc[row + b_col + d]) : 0.f;
-            pre_c[n] = in ? to_f32(bc[row + c_col + d]) : 0.f;
+            pre_b[n] = in ? bc[row + b_col + d] : from_f32<T>(0.f);
+            pre_c[n] = in ? bc[row + c_col + d] : from_f32<T>(0.f);
         }
 #pragma unroll
         for (int n = 0; n < XPT; ++n) {
             const int j = threadIdx.x + n * SCAN_THREADS;
             const int t = j / COLS, c = blockIdx.x * COLS + j % COLS;
             const bool in = j < count * COLS && c < C;
-            pre_x[n] = in ? to_f32(x[(size_t)(base + t) * x_stride + c]) : 0.f;
-            pre_z[n] = in ? to_f32(z[(size_t)(base + t) * z_stride + c]) : 0.f;
-            pre_dt[n] = in ? to_f32(dt_raw[(size_t)(base + t) * dt_stride + c]) : 0.f;
+            pre_x[n] = in ? x[(size_t)(base + t) * x_stride + c] : from_f32<T>(0.f);
+            pre_z[n] = in ? z[(size_t)(base + t) * z_stride + c] : from_f32<T>(0.f);
+            pre_dt[n] = in ? dt_raw[(size_t)(base + t) * dt_stride + c] : from_f32<T>(0.f);
         }
     };
     auto store_tile = [&](int buf) {   // step sizes and gates are taken here, a tile behind their loads, which nobody waits for
@@ -656,17 +684,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
         for (int n = 0; n < BPT; ++n) {
             const int i = threadIdx.x + n * SCAN_THREADS;
             if (i < SCAN_TILE * NMAX) {
-                b_s[buf * SCAN_TILE * NMAX + i] = pre_b[n];
-                c_s[buf * SCAN_TILE * NMAX + i] = pre_c[n];
+                b_s[buf * SCAN_TILE * NMAX + i] = to_f32(pre_b[n]);
+                c_s[buf * SCAN_TILE * NMAX + i] = to_f32(pre_c[n]);
             }
         }
 #pragma unroll
         for (int n = 0; n < XPT; ++n) {
             const int j = threadIdx.x + n * SCAN_THREADS;
             if (j < SCAN_TILE * COLS) {
-                x_s[buf * SCAN_TILE * COLS + j] = pre_x[n];
-                dt_s[buf * SCAN_TILE * COLS + j] = softplus_f(pre_dt[n] + bias);
-                z_s[buf * SCAN_TILE * COLS + j] = silu_f(pre_z[n]);
+                x_s[buf * SCAN_TILE * COLS + j] = to_f32(pre_x[n]);
+                dt_s[buf * SCAN_TILE * COLS + j] = softplus_f(to_f32(pre_dt[n]) + bias);
+                z_s[buf * SCAN_TILE * COLS + j] = silu_f(to_f32(pre_z[n]));
             }
         }
     };
