@@ -58,14 +58,31 @@ enum { MODE_PLAIN = 0, MODE_ABSORB = 1, MODE_EXPAND = 2, MODE_ABSORB_TAIL = 3, M
 // A block: up to TOK tokens, one head, 32 result columns (lane = column). Its four warps take a quarter of the inner dimension
 // each, in order, and their partial sums are added in the order of the warps: every result is one fixed sequence of 32-bit
 // multiply-adds, whatever the batch holds.
-template <typename T>
+// STAGED: the block's 32 columns of the matrix are copied to shared memory first, all of them on their way before the kernel ahead
+// has finished (the matrix is a weight): read from global memory 8 rows at a time, a trip to memory per 8 was most of what the
+// kernel took for a few decoded tokens (14 heads, 64 x 256 and 256 x 64: 9.7 -> 4.9 us). Needs columns in whole 16-byte pieces.
+template <typename T, bool STAGED>
 __global__ void __launch_bounds__(128) head_matmul_kernel(const T* __restrict__ x, int x_stride, int x_head, const T* __restrict__ M,
                                                          T* __restrict__ out, int out_stride, int out_head, int N, int K, int J, int mode,
                                                          int R, int rot_dims, const float* __restrict__ cos_t,
                                                          const float* __restrict__ sin_t, const T* __restrict__ gate, int gate_stride) {
-    extern __shared__ __align__(16) float xs[];   // [TOK][K], then [4][TOK][32] partial sums
-    float* part = xs + TOK * K;
+    extern __shared__ __align__(16) float xs[];   // [TOK][KP], then [4][TOK][32] partial sums, then (STAGED) [K][32] of the matrix
+    const int KP = (K + 3) & ~3;
+    float* part = xs + TOK * KP;
+    T* ms = reinterpret_cast<T*>(part + 4 * TOK * 32);
     pdl_trigger();
+    if constexpr (STAGED) {   // (launched so for modes with a product only)
+        constexpr int PIECE = 16 / sizeof(T), PER_ROW = 32 / PIECE;
+        const T* from = M + (size_t)blockIdx.y * K * J + blockIdx.z * 32;
+        for (int i = threadIdx.x; i < K * PER_ROW; i += blockDim.x) {
+            const int k = i / PER_ROW, c = i % PER_ROW * PIECE;
+            if ((int)blockIdx.z * 32 + c < J) {
+                const uint32_t d = (uint32_t)__cvta_generic_to_shared(ms + k * 32 + c);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(from + (size_t)k * J + c) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
     pdl_wait();
     const int n0 = blockIdx.x * TOK, h = blockIdx.y, j0 = blockIdx.z * 32;
     const int nt = min(TOK, N - n0);
@@ -80,10 +97,20 @@ __global__ void __launch_bounds__(128) head_matmul_kernel(const T* __restrict__ 
         return;
     }
     if (mode != MODE_ABSORB_TAIL) {
-        for (int i = threadIdx.x; i < TOK * K; i += blockDim.x) {
-            const int t = i / K, k = i % K;
-            xs[i] = t < nt ? to_f32(x[(size_t)(n0 + t) * x_stride + (size_t)h * x_head + k]) : 0.f;
+        if ((K & 3) == 0 && (x_stride & 3) == 0 && (x_head & 3) == 0 && ((uintptr_t)x & (4 * sizeof(T) - 1)) == 0) {
+            for (int i = threadIdx.x; i < TOK * (K >> 2); i += blockDim.x) {
+                const int t = i / (K >> 2), k = i % (K >> 2) * 4;
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
+                if (t < nt) load4(x + (size_t)(n0 + t) * x_stride + (size_t)h * x_head + k, v);
+                store4(xs + t * KP + k, v);
+            }
+        } else {
+            for (int i = threadIdx.x; i < TOK * K; i += blockDim.x) {
+                const int t = i / K, k = i % K;
+                xs[t * KP + k] = t < nt ? to_f32(x[(size_t)(n0 + t) * x_stride + (size_t)h * x_head + k]) : 0.f;
+            }
         }
+        if constexpr (STAGED) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
         const int j = j0 + lane;
         const int kq = (K + 3) / 4;
@@ -92,21 +119,28 @@ __global__ void __launch_bounds__(128) head_matmul_kernel(const T* __restrict__ 
 #pragma unroll
         for (int t = 0; t < TOK; ++t) acc[t] = 0.f;
         if (j < J) {
-            const T* col = M + (size_t)h * K * J + j;
+            const T* col = STAGED ? ms + lane : M + (size_t)h * K * J + j;
+            const size_t step = STAGED ? 32 : J;
             int k = k_lo;
-            for (; k + 8 <= k_hi; k += 8) {   // eight loads in flight
-                float w[8];
+            if ((kq & 3) == 0) {
+                for (; k + 8 <= k_hi; k += 8) {   // eight loads in flight; a token's entries four at a time
+                    float w[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) w[u] = to_f32(col[(size_t)(k + u) * J]);
+                    for (int u = 0; u < 8; ++u) w[u] = to_f32(col[(size_t)(k + u) * step]);
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-#pragma unroll
-                    for (int t = 0; t < TOK; ++t) acc[t] = fmaf(xs[t * K + k + u], w[u], acc[t]);
+                    for (int t = 0; t < TOK; ++t) {
+                        if (t < nt) {
+                            const float4 a = *reinterpret_cast<const float4*>(xs + t * KP + k), b = *reinterpret_cast<const float4*>(xs + t * KP + k + 4);
+                            acc[t] = fmaf(a.x, w[0], acc[t]); acc[t] = fmaf(a.y, w[1], acc[t]); acc[t] = fmaf(a.z, w[2], acc[t]); acc[t] = fmaf(a.w, w[3], acc[t]);
+                            acc[t] = fmaf(b.x, w[4], acc[t]); acc[t] = fmaf(b.y, w[5], acc[t]); acc[t] = fmaf(b.z, w[6], acc[t]); acc[t] = fmaf(b.w, w[7], acc[t]);
+                        }
+                    }
+                }
             }
             for (; k < k_hi; ++k) {
-                const float w = to_f32(col[(size_t)k * J]);
+                const float w = to_f32(col[(size_t)k * step]);
 #pragma unroll
-                for (int t = 0; t < TOK; ++t) acc[t] = fmaf(xs[t * K + k], w, acc[t]);
+                for (int t = 0; t < TOK; ++t) acc[t] = fmaf(xs[t * KP + k], w, acc[t]);
             }
         }
 #pragma unroll
@@ -150,11 +184,15 @@ int prepare(const T* z, int z_stride, int q_rank, int kv_rank, int rot_dim, int 
 template <typename T>
 int head_matmul(const T* x, int x_stride, int x_head, const T* M, T* out, int out_stride, int out_head, int N, int H, int K, int J, int mode,
                 int R, int rot_dims, const float* cos_t, const float* sin_t, const T* gate, int gate_stride, cudaStream_t s) {
-    const size_t smem = sizeof(float) * (TOK * (size_t)K + 4 * TOK * 32);
+    const size_t rows = sizeof(float) * (TOK * (size_t)((K + 3) & ~3) + 4 * TOK * 32), columns = (size_t)K * 32 * sizeof(T);
     const int jchunks = mode == MODE_ABSORB_TAIL ? 1 : (J + 31) / 32;   // the tail alone is one block's work per tokens and head
-    if (smem > 200 * 1024 || H > 65535 || jchunks > 65535) return LLMIE_ERR_BAD_ARGUMENT;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(head_matmul_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_kernel(head_matmul_kernel<T>, dim3((N + TOK - 1) / TOK, H, jchunks), dim3(128), smem, s, x, x_stride, x_head, M, out, out_stride,
+    if (rows > 200 * 1024 || H > 65535 || jchunks > 65535) return LLMIE_ERR_BAD_ARGUMENT;
+    const bool product = mode != MODE_ABSORB_TAIL && mode != MODE_GATE_ONLY;
+    const bool staged = product && J % (int)(16 / sizeof(T)) == 0 && ((uintptr_t)M & 15) == 0 && rows + columns <= 200 * 1024;
+    const size_t smem = rows + (staged ? columns : 0);
+    auto kernel = staged ? head_matmul_kernel<T, true> : head_matmul_kernel<T, false>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return launch_kernel(kernel, dim3((N + TOK - 1) / TOK, H, jchunks), dim3(128), smem, s, x, x_stride, x_head, M, out, out_stride,
                          out_head, N, K, J, mode, R, rot_dims, cos_t, sin_t, gate, gate_stride);
 }
 
