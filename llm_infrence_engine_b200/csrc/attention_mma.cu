@@ -40,6 +40,8 @@ struct Params {
     float* part_ml;         // [tiles][nkv][splits][ROWS][2]
     int* counters;          // [tiles * nkv], zero between launches
     int q_stride, max_blocks, nq, nkv, page_size, window, num_splits;
+    // decode kernel, tile i is token i, not as clusters: > 0: the launch's blocks are dealt out by the tokens' lengths (see deal), this many tokens
+    int balanced = 0;
     int page_shift;         // log2(page_size), or -1 if that is no power of two
     int cluster;            // 1: the slices of a tile are one thread-block cluster and merge through distributed shared memory
     float scale_log2;       // softmax scale * log2(e)
@@ -404,6 +406,82 @@ __device__ __forceinline__ void attend_chunk_t8(const uint32_t (&qb)[D / 16][2],
 // T8: every tile has at most 8 rows and one token (a decode step of a model with up to 8 heads per group): the transposed form.
 // SIG: sigmoid weights; TURN: results are turned back (each compiled in only where it is asked for)
 // EXT: the extras of ExtTerms (T8 only); SHARED: keys are values, a chunk is one tile of the ring
+// Which token and slice a launch's item is, when `items` of them are dealt out by the tokens' lengths: a token gets as many slices as its
+// chunks fill at the smallest length of a slice for which all slices fit the items (no token more than num_splits). The launch is made
+// once for every length a step may bring, and without this it lasts as long as the longest token takes one block. Every warp finds
+// it by itself, from the positions alone, before the wait for the kernel ahead. False: nothing to do for this item.
+constexpr int DEAL_TOKENS = 96;
+template <int BN, bool EXT>
+__device__ __forceinline__ bool deal(const Params& p, int item, int items, int lane, int& token, int& split, int& slices, int& pos_of_token) {
+    constexpr int GROUPS = DEAL_TOKENS / 32;
+    int c[GROUPS], pos[GROUPS];   // chunks and position of token lane + 32 j
+    int most = 1, total = 0;
+#pragma unroll
+    for (int j = 0; j < GROUPS; ++j) pos[j] = lane + 32 * j < p.balanced ? p.positions[lane + 32 * j] : -1;
+#pragma unroll
+    for (int j = 0; j < GROUPS; ++j) {
+        int lo = p.window > 0 ? max(0, pos[j] - p.window + 1) : 0;
+        if (EXT && p.chunk > 0) lo = max(lo, pos[j] / p.chunk * p.chunk);
+        c[j] = pos[j] < 0 ? 0 : (pos[j] + 1 - lo + BN - 1) / BN;
+        most = max(most, c[j]);
+        total += c[j];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+        total += __shfl_xor_sync(0xffffffffu, total, o);
+    }
+    // slices of x chunks at `each` chunks a slice (exact: numbers of a few thousand)
+    auto slices_at = [](int x, int each) { return (int)(((float)(x + each - 1) + 0.5f) * (1.0f / (float)each)); };
+    int enough = most;   // chunks of a slice: this always fits (a slice per token)
+    // no slice can be shorter than an even share of all chunks; where the longest token is near that, nothing is cut
+    int least = max((total + items - 1) / items, (most + p.num_splits - 1) / p.num_splits);
+    if (4 * most <= 5 * least) {
+        if (item >= p.balanced) return false;
+        token = item;
+        split = 0;
+        slices = 1;
+    } else {
+        while (least < enough) {
+            const int mid = (least + enough) / 2;
+            int n = 0;
+#pragma unroll
+            for (int j = 0; j < GROUPS; ++j) n += slices_at(c[j], mid);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+            if (n <= items) enough = mid;
+            else least = mid + 1;
+        }
+        int before = 0;
+        token = -1;
+#pragma unroll
+        for (int j = 0; j < GROUPS; ++j) {
+            const int mine = slices_at(c[j], enough);
+            int upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            const uint32_t behind = __ballot_sync(0xffffffffu, before + upto > item);
+            if (behind && token < 0) {
+                const int at = __ffs(behind) - 1;
+                token = at + 32 * j;
+                slices = __shfl_sync(0xffffffffu, mine, at);
+                split = item - before - (__shfl_sync(0xffffffffu, upto, at) - slices);
+            }
+            before += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (token < 0) return false;
+    }
+#pragma unroll
+    for (int j = 0; j < GROUPS; ++j) {
+        const int v = __shfl_sync(0xffffffffu, pos[j], token & 31);
+        if (token >> 5 == j) pos_of_token = v;
+    }
+    return true;
+}
+
 template <int D, int BN, int STAGES, int DW, bool T8, bool SIG, bool TURN, bool EXT = false, bool SHARED = false>
 __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -416,8 +494,15 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
     float* my_numbers = reinterpret_cast<float*>(smem_raw + (size_t)DW * STAGES * SLOT * sizeof(bf16)) + warp * STAGES * BN;   // SHARED: [STAGES][BN]
     __shared__ int flag;
 
-    const int tile = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
+    int tile = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, slices = p.num_splits, dealt_pos = 0;
     pdl_trigger();
+    if (p.balanced > 0) {
+        kvh = blockIdx.x % p.nkv;
+        if (!deal<BN, EXT>(p, blockIdx.x / p.nkv, gridDim.x / p.nkv, lane, tile, split, slices, dealt_pos)) {
+            pdl_wait();
+            return;
+        }
+    }
     // What this block needs of the step's own integers (positions, table rows, block tables) was copied to the device
     // before the step's first kernel, and keys and values of earlier positions were written by earlier steps: none of it
     // depends on the kernels just before this one. So when tile i is simply token i, the block finds its key range and
@@ -429,28 +514,62 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
     const int ntok = p.tile_info ? p.tile_info[2 * tile + 1] : 1;
     const int G = p.nq / p.nkv;
     const int nrows = ntok * G;  // <= 16
-    const int pos0 = p.positions[n0];
+    const int pos0 = p.balanced > 0 ? dealt_pos : p.positions[n0];
     const int* table = p.block_table + (size_t)p.token_seq[n0] * p.max_blocks;
     const int hi = pos0 + ntok;  // one past the last visible key
     int lo = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
     if (EXT && p.chunk > 0) lo = max(lo, pos0 / p.chunk * p.chunk);
     const int chunks = (hi - lo + BN - 1) / BN;
-    const int per = (chunks + p.num_splits - 1) / p.num_splits;
+    const int per = (chunks + slices - 1) / slices;
     const int c_begin = split * per, c_end = min(chunks, c_begin + per);
 
     // this warp's chunks: c_begin + warp, + DW, ...
     const int first = c_begin + warp;
     const int mine = first < c_end ? (c_end - first + DW - 1) / DW : 0;
+    // Where the first chunks lie is looked up before the wait for all of them. (From the projection's sums) a chunk that holds the
+    // token's own position is fetched early too: the rows that the cache does not hold yet are replaced below by the warp that owns it.
+    const bool own_here = T8 && p.qkv_acc && p.slots;
+    int own_it = -1;
+    if (own_here) {
+        const int c_p = (pos0 - lo) / BN;   // the chunk that holds the token's own position
+        if (c_p >= c_begin && c_p < c_end && (c_p - c_begin) % DW == warp) own_it = (c_p - first) / DW;
+    }
+    PoolRows<BN> rows_at[STAGES];
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s)
+        if (s < mine) rows_at[s] = find_rows_warp<BN>(p, table, kvh, lo + (first + s * DW) * BN, hi - 1, lane);
     // All STAGES slots of the ring are filled up front; a slot is filled again right AFTER its chunk has been used, so the
     // instructions that issue a copy never stand between a landed chunk and its arithmetic.
     bool fetched[STAGES];
 #pragma unroll
     for (int s = 0; s < STAGES; ++s) {
         const int key0 = lo + (first + s * DW) * BN;
-        fetched[s] = early && s < mine && key0 + BN <= pos0;  // wholly before the first new position
-        if (fetched[s]) load_rows_warp<D, BN, SHARED>(p, table, kvh, key0, hi - 1, 0, my + s * SLOT, my + s * SLOT + V_AT, lane, my_numbers + s * BN);
+        fetched[s] = early && s < mine && (own_here || key0 + BN <= pos0);  // wholly before the first new position
+        if (fetched[s]) copy_rows_warp<D, BN, SHARED>(p, rows_at[s], 0, my + s * SLOT, my + s * SLOT + V_AT, lane, my_numbers + s * BN);
     }
+    // the biases of the projection are weights: they are asked for before the wait as well
+    float q_bias[T8 ? D / 16 : 1][4];
+    if constexpr (T8) {
+        const int head = kvh * G + ((lane >> 2) < nrows ? lane >> 2 : 0);
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+            q_bias[kk][0] = q_bias[kk][1] = q_bias[kk][2] = q_bias[kk][3] = 0.f;
+            if (p.qkv_acc && p.bias) {
+                const int col = kk * 16 + ((lane & 3) << 1);
+                const float2 ba = *reinterpret_cast<const float2*>(p.bias + (size_t)head * D + col);
+                const float2 bc = *reinterpret_cast<const float2*>(p.bias + (size_t)head * D + col + 8);
+                q_bias[kk][0] = ba.x; q_bias[kk][1] = ba.y; q_bias[kk][2] = bc.x; q_bias[kk][3] = bc.y;
+            }
+        }
+    }
+    const int own_slot = own_it >= 0 ? p.slots[n0] : -1;   // (of the step's own integers)
     if (early) pdl_wait();
+    // what the kernels just before have written: the chunks' copies and every load below leave together, one trip to memory for all
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s) {
+        if (s < mine && !fetched[s]) copy_rows_warp<D, BN, SHARED>(p, rows_at[s], 0, my + s * SLOT, my + s * SLOT + V_AT, lane, my_numbers + s * BN);
+        cp_async_commit();  // stage 0's group may also hold later stages' early fetches: it then completes a little later, never too early
+    }
 
     int row_pos[2];
     bool row_ok[2];
@@ -460,7 +579,6 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
     // (from the projection's sums) the token's own key and value, finished by the warp that owns its position: pairs
     // (j, j + D / 2) for j = lane, lane + 32, ...
     constexpr int NP = D / 64;
-    int own_it = -1;
     uint32_t own_k[NP], own_v[NP];   // (element j, element j + D / 2) as two bfloat16
     if constexpr (T8) {
         const int row = lane >> 2;
@@ -470,63 +588,74 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
             const float* src = p.qkv_acc + (size_t)n0 * p.acc_stride + (size_t)head * D;
             const float* ct = p.cos_t + (size_t)n0 * (D / 2);
             const float* sn = p.sin_t + (size_t)n0 * (D / 2);
-            float x[D / 16][4];
+            // the loads first, all of them (no branch between them, or each would wait for the one before)
+            float x[D / 16][4], cs[D / 32][4], ss[D / 32][4];
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
                 const int col = kk * 16 + ((lane & 3) << 1);
                 const float2 a = __ldcg(reinterpret_cast<const float2*>(src + col)), c = __ldcg(reinterpret_cast<const float2*>(src + col + 8));
                 x[kk][0] = a.x; x[kk][1] = a.y; x[kk][2] = c.x; x[kk][3] = c.y;
-                if (p.bias) {
-                    const float2 ba = *reinterpret_cast<const float2*>(p.bias + (size_t)head * D + col);
-                    const float2 bc = *reinterpret_cast<const float2*>(p.bias + (size_t)head * D + col + 8);
-                    x[kk][0] += ba.x; x[kk][1] += ba.y; x[kk][2] += bc.x; x[kk][3] += bc.y;
-                }
             }
 #pragma unroll
-            for (int kk = 0; kk < D / 32; ++kk) {   // dims of the first half and their partners D / 2 further on, both in this lane
+            for (int kk = 0; kk < D / 32; ++kk) {
                 const int col = kk * 16 + ((lane & 3) << 1);
                 const float2 c0 = *reinterpret_cast<const float2*>(ct + col), c1 = *reinterpret_cast<const float2*>(ct + col + 8);
                 const float2 s0 = *reinterpret_cast<const float2*>(sn + col), s1 = *reinterpret_cast<const float2*>(sn + col + 8);
-                const float cs[4] = {c0.x, c0.y, c1.x, c1.y}, ss[4] = {s0.x, s0.y, s1.x, s1.y};
+                cs[kk][0] = c0.x; cs[kk][1] = c0.y; cs[kk][2] = c1.x; cs[kk][3] = c1.y;
+                ss[kk][0] = s0.x; ss[kk][1] = s0.y; ss[kk][2] = s1.x; ss[kk][3] = s1.y;
+            }
+            if (own_it >= 0) {
+                const float* ks_ = p.qkv_acc + (size_t)n0 * p.acc_stride + (size_t)(p.nq + kvh) * D;
+                const float* vs_ = p.qkv_acc + (size_t)n0 * p.acc_stride + (size_t)(p.nq + p.nkv + kvh) * D;
+                float raw[NP][4], c[NP], sv[NP], b[NP][4];
+#pragma unroll
+                for (int i = 0; i < NP; ++i) {
+                    const int j = lane + 32 * i;
+                    raw[i][0] = __ldcg(ks_ + j); raw[i][1] = __ldcg(ks_ + j + D / 2); raw[i][2] = __ldcg(vs_ + j); raw[i][3] = __ldcg(vs_ + j + D / 2);
+                    c[i] = ct[j]; sv[i] = sn[j];
+                    b[i][0] = b[i][1] = b[i][2] = b[i][3] = 0.f;
+                }
+                if (p.bias) {
+                    const float *kb = p.bias + (size_t)(p.nq + kvh) * D, *vb = p.bias + (size_t)(p.nq + p.nkv + kvh) * D;
+#pragma unroll
+                    for (int i = 0; i < NP; ++i) {
+                        const int j = lane + 32 * i;
+                        b[i][0] = kb[j]; b[i][1] = kb[j + D / 2]; b[i][2] = vb[j]; b[i][3] = vb[j + D / 2];
+                    }
+                }
+                const int page = own_slot >= 0 ? own_slot / p.page_size : 0, off = own_slot >= 0 ? own_slot - page * p.page_size : 0;
+                const size_t dst = (((size_t)page * p.nkv + kvh) * p.page_size + off) * D;
+#pragma unroll
+                for (int i = 0; i < NP; ++i) {
+                    const int j = lane + 32 * i;
+                    const float k1 = raw[i][0] + b[i][0], k2 = raw[i][1] + b[i][1], v1 = raw[i][2] + b[i][2], v2 = raw[i][3] + b[i][3];
+                    const __nv_bfloat16 r1 = __float2bfloat16_rn(k1 * c[i] - k2 * sv[i]), r2 = __float2bfloat16_rn(k2 * c[i] + k1 * sv[i]);
+                    const __nv_bfloat16 w1 = __float2bfloat16_rn(v1), w2 = __float2bfloat16_rn(v2);
+                    own_k[i] = (uint32_t)__bfloat16_as_ushort(r1) | ((uint32_t)__bfloat16_as_ushort(r2) << 16);
+                    own_v[i] = (uint32_t)__bfloat16_as_ushort(w1) | ((uint32_t)__bfloat16_as_ushort(w2) << 16);
+                    if (own_slot >= 0) {
+                        p.k_pool_w[dst + j] = r1; p.k_pool_w[dst + j + D / 2] = r2;
+                        p.v_pool_w[dst + j] = w1; p.v_pool_w[dst + j + D / 2] = w2;
+                    }
+                }
+            }
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[kk][e] += q_bias[kk][e];
+#pragma unroll
+            for (int kk = 0; kk < D / 32; ++kk) {   // dims of the first half and their partners D / 2 further on, both in this lane
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float x1 = x[kk][e], x2 = x[kk + D / 32][e];
-                    x[kk][e] = x1 * cs[e] - x2 * ss[e];
-                    x[kk + D / 32][e] = x2 * cs[e] + x1 * ss[e];
+                    x[kk][e] = x1 * cs[kk][e] - x2 * ss[kk][e];
+                    x[kk + D / 32][e] = x2 * cs[kk][e] + x1 * ss[kk][e];
                 }
             }
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
                 qb[kk][0] = ok ? pack_bf16(x[kk][0], x[kk][1]) : 0u;
                 qb[kk][1] = ok ? pack_bf16(x[kk][2], x[kk][3]) : 0u;
-            }
-            if (p.slots) {
-                const int c_p = (pos0 - lo) / BN;   // the chunk that holds the token's own position
-                if (c_p >= c_begin && c_p < c_end && (c_p - c_begin) % DW == warp) own_it = (c_p - first) / DW;
-            }
-            if (own_it >= 0) {
-                const float* ks_ = p.qkv_acc + (size_t)n0 * p.acc_stride + (size_t)(p.nq + kvh) * D;
-                const float* vs_ = p.qkv_acc + (size_t)n0 * p.acc_stride + (size_t)(p.nq + p.nkv + kvh) * D;
-                const float* kb = p.bias ? p.bias + (size_t)(p.nq + kvh) * D : nullptr;
-                const float* vb = p.bias ? p.bias + (size_t)(p.nq + p.nkv + kvh) * D : nullptr;
-                const int slot = p.slots[n0];
-                const int page = slot >= 0 ? slot / p.page_size : 0, off = slot >= 0 ? slot - page * p.page_size : 0;
-                const size_t dst = (((size_t)page * p.nkv + kvh) * p.page_size + off) * D;
-#pragma unroll
-                for (int i = 0; i < NP; ++i) {
-                    const int j = lane + 32 * i;
-                    float k1 = __ldcg(ks_ + j), k2 = __ldcg(ks_ + j + D / 2), v1 = __ldcg(vs_ + j), v2 = __ldcg(vs_ + j + D / 2);
-                    if (p.bias) { k1 += kb[j]; k2 += kb[j + D / 2]; v1 += vb[j]; v2 += vb[j + D / 2]; }
-                    const float c = ct[j], sv = sn[j];
-                    const __nv_bfloat16 r1 = __float2bfloat16_rn(k1 * c - k2 * sv), r2 = __float2bfloat16_rn(k2 * c + k1 * sv);
-                    const __nv_bfloat16 w1 = __float2bfloat16_rn(v1), w2 = __float2bfloat16_rn(v2);
-                    own_k[i] = (uint32_t)__bfloat16_as_ushort(r1) | ((uint32_t)__bfloat16_as_ushort(r2) << 16);
-                    own_v[i] = (uint32_t)__bfloat16_as_ushort(w1) | ((uint32_t)__bfloat16_as_ushort(w2) << 16);
-                    if (slot >= 0) {
-                        p.k_pool_w[dst + j] = r1; p.k_pool_w[dst + j + D / 2] = r2;
-                        p.v_pool_w[dst + j] = w1; p.v_pool_w[dst + j + D / 2] = w2;
-                    }
-                }
             }
         } else {
             const bf16* qp = p.q + (size_t)n0 * p.q_stride + (size_t)(kvh * G + (ok ? row : 0)) * D;
@@ -566,12 +695,6 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
         }
     }
 
-#pragma unroll
-    for (int s = 0; s < STAGES; ++s) {
-        if (s < mine && !fetched[s])
-            load_rows_warp<D, BN, SHARED>(p, table, kvh, lo + (first + s * DW) * BN, hi - 1, 0, my + s * SLOT, my + s * SLOT + V_AT, lane, my_numbers + s * BN);
-        cp_async_commit();  // stage 0's group may also hold later stages' early fetches: it then completes a little later, never too early
-    }
     // where the chunk lies that refills the first slot: the block table is read now, not between a chunk's arithmetic and the
     // copies that refill its slot
     PoolRows<BN> refill;
@@ -780,7 +903,7 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
         cluster_sync_all();  // the other blocks' shared memory stays until block 0 has read it
         return;
     }
-    finish_tile<D, 16, DW * 32>(p, fm, fl, fo, p.num_splits, ((size_t)tile * p.nkv + kvh) * p.num_splits, 1, tile * p.nkv + kvh, kvh, split, n0, nrows, G, &flag, wo);
+    finish_tile<D, 16, DW * 32>(p, fm, fl, fo, slices, ((size_t)tile * p.nkv + kvh) * p.num_splits, 1, tile * p.nkv + kvh, kvh, split, n0, nrows, G, &flag, wo);
 }
 
 // ---------------------------------------------------------------------------------------------- prefill
@@ -952,8 +1075,8 @@ int launch_decode(const Params& p, dim3 grid, cudaStream_t s) {
 }
 
 template <int D>
-int launch(const Params& p, int num_tiles, int decode_mode, cudaStream_t s) {
-    const dim3 grid(num_tiles, p.nkv, p.num_splits);
+int launch(const Params& p, int num_tiles, int items, int decode_mode, cudaStream_t s) {
+    const dim3 grid = p.balanced > 0 ? dim3(items * p.nkv) : dim3(num_tiles, p.nkv, p.num_splits);
     if (decode_mode) {
         // tiles of one token with up to 8 heads per group: the transposed form, which spends nothing on padding rows
         const bool t8 = p.tile_info == nullptr && p.nq / p.nkv <= 8;
@@ -985,6 +1108,8 @@ LLMIE_API int llmie_attn_plan(const int* seq_starts, int num_seqs, int tokens_pe
     return launch_kernel(attn_plan_kernel, dim3(1), dim3(32), 0, s, seq_starts, num_seqs, tokens_per_tile, tile_info, max_tiles);
 }
 
+// balanced (0, or the number of tokens: decode modes without tile_info, not as clusters): one block per multiprocessor, dealt out by the
+// tokens' lengths; num_splits is then the most slices that a token may have.
 // decode_mode 1 or 2: every tile has at most 16 rows (tokens * group); 2 asks for blocks of four warps instead of eight when
 // nothing is cut into slices. 0: at most 64 rows.
 // turn_cos / turn_sin (or null), sig_bias (or null), log_r1 / log_r2 (or null): decode modes only.
@@ -995,7 +1120,7 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
                    bf16* out, float* scratch_o, float* scratch_ml, int* counters, int nq, int nkv, int d,
                    int page_size, float scale, int window, int num_splits, int decode_mode, int cluster, const float* qkv_acc,
                    int acc_stride, const float* bias, const float* cos_t, const float* sin_t, const int* slots, const float* turn_cos, const float* turn_sin,
-                   const float* sig_bias, const float* log_r1, const float* log_r2, cudaStream_t s, const Params* extras = nullptr) {
+                   const float* sig_bias, const float* log_r1, const float* log_r2, int balanced, int num_sms, cudaStream_t s, const Params* extras = nullptr) {
     if (num_tiles <= 0) return 0;
     if ((turn_cos == nullptr) != (turn_sin == nullptr) || (log_r1 == nullptr) != (log_r2 == nullptr) || (log_r1 && !sig_bias) ||
         ((turn_cos || sig_bias) && !decode_mode))
@@ -1004,6 +1129,8 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
                     (acc_stride & 1) || ((uintptr_t)qkv_acc & 7) || ((uintptr_t)bias & 7) || ((uintptr_t)cos_t & 7) || ((uintptr_t)sin_t & 7)))
         return LLMIE_ERR_BAD_ARGUMENT;
     if (cluster && (!decode_mode || num_splits > 8)) return LLMIE_ERR_BAD_ARGUMENT;
+    if (balanced && (balanced != num_tiles || balanced > DEAL_TOKENS || !decode_mode || cluster || tile_info || nkv < 1 || num_tiles > num_sms / nkv))
+        return LLMIE_ERR_BAD_ARGUMENT;
     if ((d != 64 && d != 128) || nkv <= 0 || nq % nkv || page_size <= 0 || num_splits < 1 || q_stride % 8 || nkv > 65535 ||
         num_splits > 64 || (num_splits > 1 && !cluster && (!scratch_o || !scratch_ml || !counters)))
         return LLMIE_ERR_BAD_ARGUMENT;
@@ -1014,7 +1141,7 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
     p.tile_info = tile_info; p.out = out; p.part_o = scratch_o; p.part_ml = scratch_ml; p.counters = counters;
     p.q_stride = q_stride; p.max_blocks = max_blocks; p.nq = nq; p.nkv = nkv; p.page_size = page_size; p.window = window;
     p.page_shift = (page_size & (page_size - 1)) == 0 ? __builtin_ctz((unsigned)page_size) : -1;
-    p.num_splits = num_splits; p.scale_log2 = scale * LOG2E; p.cluster = cluster;
+    p.num_splits = num_splits; p.balanced = balanced; p.scale_log2 = scale * LOG2E; p.cluster = cluster;
     p.qkv_acc = qkv_acc; p.acc_stride = acc_stride; p.bias = bias; p.cos_t = cos_t; p.sin_t = sin_t; p.slots = slots;
     p.turn_cos = turn_cos; p.turn_sin = turn_sin; p.sig_bias = sig_bias; p.log_r1 = log_r1; p.log_r2 = log_r2;
     if (extras) {
@@ -1023,17 +1150,18 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
         p.key_scale = extras->key_scale;
     }
     p.k_pool_w = const_cast<bf16*>(k_pool); p.v_pool_w = const_cast<bf16*>(v_pool);
-    return d == 64 ? launch<64>(p, num_tiles, decode_mode, s) : launch<128>(p, num_tiles, decode_mode, s);
+    return d == 64 ? launch<64>(p, num_tiles, num_sms / nkv, decode_mode, s) : launch<128>(p, num_tiles, num_sms / nkv, decode_mode, s);
 }
 
 LLMIE_API int llmie_paged_attention_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* v_pool, const int* block_table,
                                         int max_blocks, const int* token_seq, const int* positions, const int* tile_info, int num_tiles,
                                         bf16* out, float* scratch_o, float* scratch_ml, int* counters, int nq, int nkv, int d,
                                         int page_size, float scale, int window, int num_splits, int decode_mode, int cluster, const float* turn_cos,
-                                        const float* turn_sin, const float* sig_bias, const float* log_r1, const float* log_r2, cudaStream_t s) {
+                                        const float* turn_sin, const float* sig_bias, const float* log_r1, const float* log_r2, int balanced,
+                                        int num_sms, cudaStream_t s) {
     return run_mma(q, q_stride, k_pool, v_pool, block_table, max_blocks, token_seq, positions, tile_info, num_tiles, out, scratch_o, scratch_ml,
                    counters, nq, nkv, d, page_size, scale, window, num_splits, decode_mode, cluster, nullptr, 0, nullptr, nullptr, nullptr,
-                   nullptr, turn_cos, turn_sin, sig_bias, log_r1, log_r2, s);
+                   nullptr, turn_cos, turn_sin, sig_bias, log_r1, log_r2, balanced, num_sms, s);
 }
 
 // Decode steps (tile i is token i, at most 8 query heads per key/value head) with chunks, a soft cap, a bias by distance (rel [rel_rows][nq],
@@ -1043,7 +1171,7 @@ LLMIE_API int llmie_paged_attention_mma_ext(const bf16* q, int q_stride, const b
                                             const int* token_seq, const int* positions, int num_tokens, bf16* out, float* scratch_o, float* scratch_ml,
                                             int* counters, int nq, int nkv, int d, int page_size, float scale, int window, int num_splits, int cluster,
                                             int four_warps, int chunk, float softcap, const float* rel, const int* rows_of, int n_rows_of, int rel_rows,
-                                            const bf16* gate, int gate_stride, const float* key_scale, cudaStream_t s) {
+                                            const bf16* gate, int gate_stride, const float* key_scale, int balanced, int num_sms, cudaStream_t s) {
     if (num_tokens <= 0) return 0;
     if (nkv <= 0 || nq / nkv > 8 || chunk < 0 || softcap < 0.f || scale == 0.f || (rel && (!rows_of || rel_rows < 1 || n_rows_of < 0)) ||
         (v_pool == nullptr) != (key_scale != nullptr))
@@ -1053,7 +1181,7 @@ LLMIE_API int llmie_paged_attention_mma_ext(const bf16* q, int q_stride, const b
     e.rel = rel; e.rows_of = rows_of; e.n_rows_of = n_rows_of; e.rel_rows = rel_rows; e.gate = gate; e.gate_stride = gate_stride; e.key_scale = key_scale;
     return run_mma(q, q_stride, k_pool, v_pool, block_table, max_blocks, token_seq, positions, nullptr, num_tokens, out, scratch_o, scratch_ml, counters,
                    nq, nkv, d, page_size, scale, window, num_splits, four_warps ? 2 : 1, cluster, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr,
-                   nullptr, nullptr, nullptr, nullptr, s, &e);
+                   nullptr, nullptr, nullptr, nullptr, balanced, num_sms, s, &e);
 }
 
 // Decode steps (every tile one token, at most 8 query heads per key/value head): the same attention, with the queries, keys and
@@ -1064,9 +1192,9 @@ LLMIE_API int llmie_paged_attention_mma_acc(const float* qkv_acc, int acc_stride
                                             const int* slots, bf16* k_pool, bf16* v_pool, const int* block_table, int max_blocks,
                                             const int* token_seq, const int* positions, int num_tokens, bf16* out, float* scratch_o,
                                             float* scratch_ml, int* counters, int nq, int nkv, int d, int page_size, float scale, int window,
-                                            int num_splits, int cluster, int four_warps, cudaStream_t s) {
+                                            int num_splits, int cluster, int four_warps, int balanced, int num_sms, cudaStream_t s) {
     if (!qkv_acc) return LLMIE_ERR_BAD_ARGUMENT;
     return run_mma(nullptr, 8, k_pool, v_pool, block_table, max_blocks, token_seq, positions, nullptr, num_tokens, out, scratch_o, scratch_ml,
                    counters, nq, nkv, d, page_size, scale, window, num_splits, four_warps ? 2 : 1, cluster, qkv_acc, acc_stride, bias, cos_t, sin_t, slots,
-                   nullptr, nullptr, nullptr, nullptr, nullptr, s);
+                   nullptr, nullptr, nullptr, nullptr, nullptr, balanced, num_sms, s);
 }

@@ -431,6 +431,30 @@ def test_decode_attention_with_many_key_slices(K, monkeypatch, cluster, nq, nkv,
     assert K._attn_counters is None or K._attn_counters.abs().sum().item() == 0
 
 
+@pytest.mark.parametrize("nq,nkv,d,ps,window,lens", [
+    (12, 2, 128, 16, 0, [int(20 * 1.09 ** i) for i in range(60)]),        # lengths of 20 to 3,200: the longest are cut into many slices
+    (14, 2, 64, 16, 0, [3201] + [1] * 73),                                 # one long request; as many tokens as the device has room for
+    (14, 2, 64, 16, 0, [3100 + i for i in range(40)]),                     # all alike: none is cut
+    (8, 4, 128, 32, 1600, [3000, 5, 1601, 1599] + [100 + 13 * i for i in range(33)]),   # a window: lengths beyond it count as the window
+    (32, 2, 64, 16, 0, [900 + 400 * (i % 7) for i in range(50)]),          # 16 heads per key/value head: not the transposed form
+    (16, 8, 64, 16, 0, [200 * i + 1 for i in range(18)]),
+])
+def test_decode_attention_dealt_out_by_length(K, monkeypatch, nq, nkv, d, ps, window, lens):
+    """Nearly a block per multiprocessor: the blocks are dealt out by the tokens' lengths, on the device, and agree with one block per token
+    and with plain torch. Twice in a row: the counters must be back at zero."""
+    qlens = [1] * len(lens)
+    qkv, kp, vp, table, tseq, pos = _attention_case(torch.bfloat16, nq, nkv, d, ps, lens, qlens, window, 23, True)
+    scale = 1.0 / math.sqrt(d)
+    want = REF.paged_attention(qkv, kp, vp, table, tseq, pos, nq, nkv, d, ps, scale, window, max(lens))
+    dev = [t.cuda() for t in (qkv, kp, vp, table, tseq, pos)]
+    for balance in (True, True, False):
+        monkeypatch.setattr(K, "balance_decode", balance)
+        got = K.paged_attention(*dev, nq, nkv, d, ps, scale, window, max(lens), batch=_Batch(qlens))
+        assert K._decode_balanced == (len(lens) if balance else 0)
+        close(got, want, 1e-2)
+    assert K._attn_counters is None or K._attn_counters.abs().sum().item() == 0
+
+
 @pytest.mark.parametrize("cluster", [True, False])
 @pytest.mark.parametrize("nq,nkv,d,ps,H,lens,window,bias,write", [
     (14, 2, 64, 16, 896, [300, 700, 5, 64, 65, 1, 33, 32], 0, True, True),   # page edges, a request of one token, chunk edges
