@@ -63,6 +63,7 @@ class DecodeGraphs:
         self.max_shapes = 6
         self.capture_after = 3   # a capture costs about a hundred eager steps: only shapes that keep coming are worth it
         self.max_shape_tokens = 8192
+        self.max_shape_entries = 64   # (decoded tokens beside a prompt portion: a busy server's step)
         self.pool = None
         self._stream = None
         self.replays = 0
@@ -77,7 +78,7 @@ class DecodeGraphs:
         if not self.usable:
             return None
         n = sum(len(e.tokens) for e in entries)
-        if n > self.max_shape_tokens or len(entries) > 8:
+        if n > self.max_shape_tokens or len(entries) > self.max_shape_entries:
             return None
         return tuple((len(e.tokens), len(e.want)) for e in entries)
 
@@ -110,7 +111,8 @@ class DecodeGraphs:
             cap.static_in = static_in
             self.shapes[key] = cap
             while len(self.shapes) > self.max_shapes:
-                self.shapes.popitem(last=False)
+                gone, _ = self.shapes.popitem(last=False)
+                self.seen.pop(gone, None)   # to be captured again it has to keep coming again
         else:
             self.shapes.move_to_end(key)
             full = r._upload(packed)
