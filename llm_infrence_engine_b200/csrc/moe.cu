@@ -25,13 +25,14 @@ constexpr int SORT_MAX_EXPERTS = 4096;
 // `scoring` 1 instead: s = sigmoid(logits), every output by itself, and the weights are the chosen s as they are (not renormalised).
 // `scoring` 2: the `top` largest logits are chosen, and their weights are the softmax over the chosen ones alone.
 // `bias` [total] or null is added to the logits first.
-__device__ __forceinline__ void route_token(const float* __restrict__ row, const float* __restrict__ correction, int* __restrict__ ids,
-                                            float* __restrict__ weights, int n, int total, int top, int lane, int scoring,
-                                            const float* __restrict__ bias) {
-    float s[ROUTE_MAX_PER_LANE], c[ROUTE_MAX_PER_LANE];
+template <int PER_LANE>
+__device__ __forceinline__ void route_token_as(const float* __restrict__ row, const float* __restrict__ correction, int* __restrict__ ids,
+                                               float* __restrict__ weights, int n, int total, int top, int lane, int scoring,
+                                               const float* __restrict__ bias) {
+    float s[PER_LANE], c[PER_LANE];
     float mx = -INFINITY;
 #pragma unroll
-    for (int j = 0; j < ROUTE_MAX_PER_LANE; ++j) {
+    for (int j = 0; j < PER_LANE; ++j) {
         const int e = lane + 32 * j;
         s[j] = e < total ? row[e] + (bias ? bias[e] : 0.f) : -INFINITY;
         c[j] = s[j];
@@ -40,7 +41,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ row, const
     mx = warp_max(mx);
     float sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < ROUTE_MAX_PER_LANE; ++j) {
+    for (int j = 0; j < PER_LANE; ++j) {
         const int e = lane + 32 * j;
         if (scoring == 1) s[j] = e < total ? 1.0f / (1.0f + expf(-s[j])) : 0.f;
         else s[j] = e < total ? expf(s[j] - mx) : 0.f;
@@ -48,7 +49,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ row, const
     }
     sum = scoring != 0 ? 1.f : warp_sum(sum);
 #pragma unroll
-    for (int j = 0; j < ROUTE_MAX_PER_LANE; ++j) {
+    for (int j = 0; j < PER_LANE; ++j) {
         const int e = lane + 32 * j;
         s[j] = s[j] / sum;
         if (scoring != 2) c[j] = e < total ? s[j] + (correction ? correction[e] : 0.f) : -INFINITY;
@@ -60,7 +61,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ row, const
         float best = -INFINITY;
         int best_e = 0x7fffffff;
 #pragma unroll
-        for (int j = 0; j < ROUTE_MAX_PER_LANE; ++j) {
+        for (int j = 0; j < PER_LANE; ++j) {
             const int e = lane + 32 * j;
             if (c[j] > best) { best = c[j]; best_e = e; }   // (ascending e within a lane: the lower index wins a tie)
         }
@@ -72,7 +73,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ row, const
         }
         float w = 0.f;
 #pragma unroll
-        for (int j = 0; j < ROUTE_MAX_PER_LANE; ++j)
+        for (int j = 0; j < PER_LANE; ++j)
             if (lane + 32 * j == best_e) { w = s[j]; c[j] = -INFINITY; }
         w = warp_sum(w);   // only the owner's lane holds it
         chosen_sum += w;
@@ -86,6 +87,14 @@ __device__ __forceinline__ void route_token(const float* __restrict__ row, const
     __syncwarp();
     const float inv = scoring == 1 ? 1.0f : 1.0f / (chosen_sum + (scoring == 0 ? 1e-20f : 0.f));   // (2: the largest logit's share is 1)
     for (int k = lane; k < top; k += 32) weights[(size_t)n * top + k] *= inv;
+}
+// (a lane's share of the outputs as a compile-time number: with room for 512 outputs, 16 of them spend sixteen times the instructions)
+__device__ __forceinline__ void route_token(const float* __restrict__ row, const float* __restrict__ correction, int* __restrict__ ids,
+                                            float* __restrict__ weights, int n, int total, int top, int lane, int scoring,
+                                            const float* __restrict__ bias) {
+    if (total <= 32) route_token_as<1>(row, correction, ids, weights, n, total, top, lane, scoring, bias);
+    else if (total <= 128) route_token_as<4>(row, correction, ids, weights, n, total, top, lane, scoring, bias);
+    else route_token_as<ROUTE_MAX_PER_LANE>(row, correction, ids, weights, n, total, top, lane, scoring, bias);
 }
 
 // Rows of `total + extra` logits; the extra ones are gates of their own: gates[n][j] = sigmoid(logit).
@@ -105,8 +114,11 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
 // The router's product and its choice in one kernel, a block per token: the token's row lies in shared memory as floats, the warps
 // share the router's outputs (a warp's lanes walk an output's weight row in 16-byte pieces; the sum runs over K in one order whatever
 // the step holds), and the first warp chooses from the logits in shared memory. For the few rows of a decode step, where the product
-// alone would be a kernel that walks K in one block.
-constexpr int ROUTER_THREADS = 256;
+// alone would be a kernel that walks K in one block. It is a chain of trips to memory, and the matrix is nobody's result: a warp's first
+// ROUTER_EARLY pieces of it are asked for before the kernel ahead has finished, the others that many at a time (a trip per piece was
+// most of the kernel: 8 rows, K = 1,024, 18 outputs: 10.5 -> 6.1 us).
+constexpr int ROUTER_THREADS = 512;
+constexpr int ROUTER_EARLY = 8;
 template <typename T>
 __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(const T* __restrict__ h, const T* __restrict__ w, const float* __restrict__ correction,
                                                                     int* __restrict__ ids, float* __restrict__ weights, int K, int total, int top, int scoring,
@@ -118,6 +130,19 @@ __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(const T* __r
     pdl_trigger();
     const int n = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool vec = (K % VN) == 0 && ((uintptr_t)h & 15) == 0 && ((uintptr_t)w & 15) == 0;
+    // a warp's pieces of the matrix: outputs warp, warp + ROUTER_THREADS / 32, ..., each in steps of 32 * VN entries
+    const int steps = (K + 32 * VN - 1) / (32 * VN), outputs = total + extra;
+    const int pieces = warp < outputs ? ((outputs - 1 - warp) / (ROUTER_THREADS / 32) + 1) * steps : 0;
+    uint4 early[ROUTER_EARLY];
+    auto ask = [&](int i0) {
+#pragma unroll
+        for (int i = 0; i < ROUTER_EARLY; ++i) {
+            const int e = warp + (i0 + i) / steps * (ROUTER_THREADS / 32), k = (i0 + i) % steps * 32 * VN + lane * VN;
+            early[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (i0 + i < pieces && k < K) early[i] = *reinterpret_cast<const uint4*>(w + (size_t)e * K + k);
+        }
+    };
+    if (vec) ask(0);
     pdl_wait();
     const T* src = h + (size_t)n * K;
     if (vec) {
@@ -131,21 +156,36 @@ __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(const T* __r
         for (int k = threadIdx.x; k < K; k += ROUTER_THREADS) row[k] = to_f32(src[k]);
     }
     __syncthreads();
-    for (int e = warp; e < total + extra; e += ROUTER_THREADS / 32) {
-        const T* we = w + (size_t)e * K;
+    if (vec) {
         float acc = 0.f;
-        if (vec) {
-            for (int k = lane * VN; k < K; k += 32 * VN) {
-                float v[VN];
-                Vec16<T>::load(we + k, v);
+        for (int i0 = 0; i0 < pieces; i0 += ROUTER_EARLY) {
+            if (i0 > 0) ask(i0);
 #pragma unroll
-                for (int i = 0; i < VN; ++i) acc = fmaf(row[k + i], v[i], acc);
+            for (int i = 0; i < ROUTER_EARLY; ++i) {
+                if (i0 + i < pieces) {
+                    const int step = (i0 + i) % steps, k = step * 32 * VN + lane * VN;
+                    if (k < K) {
+                        float v[VN];
+                        Vec16<T>::load(reinterpret_cast<const T*>(&early[i]), v);
+#pragma unroll
+                        for (int c = 0; c < VN; ++c) acc = fmaf(row[k + c], v[c], acc);
+                    }
+                    if (step == steps - 1) {
+                        acc = warp_sum(acc);
+                        if (lane == 0) logits[warp + (i0 + i) / steps * (ROUTER_THREADS / 32)] = acc;
+                        acc = 0.f;
+                    }
+                }
             }
-        } else {
-            for (int k = lane; k < K; k += 32) acc = fmaf(row[k], to_f32(we[k]), acc);
         }
-        acc = warp_sum(acc);
-        if (lane == 0) logits[e] = acc;
+    } else {
+        for (int e = warp; e < outputs; e += ROUTER_THREADS / 32) {
+            const T* we = w + (size_t)e * K;
+            float acc = 0.f;
+            for (int k = lane; k < K; k += 32) acc = fmaf(row[k], to_f32(we[k]), acc);
+            acc = warp_sum(acc);
+            if (lane == 0) logits[e] = acc;
+        }
     }
     __syncthreads();
     if (warp == 1)
@@ -222,6 +262,27 @@ __global__ void __launch_bounds__(256, 2) moe_rows_kernel(const T* __restrict__ 
     const int e = tiles[1 + 2 * blockIdx.y], p0 = tiles[2 + 2 * blockIdx.y];
     const int count = min(offsets[e + 1] - p0, tile_rows);
     const bool vec = (K % VN) == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const T* we = w + (size_t)e * (GATED ? 2 : 1) * F * K;
+    constexpr int CPW = MOE_COLS / 8;   // a warp's outputs, taken together: their weight rows are in flight at once
+    const int j0 = blockIdx.x * MOE_COLS + warp * CPW;
+    const T* wrow[CPW];
+#pragma unroll
+    for (int c = 0; c < CPW; ++c) wrow[c] = we + (size_t)min(j0 + c, F - 1) * K;   // (an output past the end repeats the last: not stored)
+    const size_t up = (size_t)F * K;   // from an output's gate row to its up row (read only when GATED)
+    // a step's 16-byte pieces of all the warp's weight rows. GATED: the next step's are asked for before this one's are used, the first
+    // step's before the tile's rows are fetched (2 rows, 16 experts of 512 x 1,024: 8.5 -> 7.8 us, 8 rows: equal; without a gate, with half the pieces, the
+    // registers cost more than it gains: 7.0 -> 7.6 at 8 rows)
+    struct Pieces { uint4 g[CPW], u[GATED ? CPW : 1]; };
+    auto ask = [&](int k, Pieces& p) {
+#pragma unroll
+        for (int c = 0; c < CPW; ++c) {
+            p.g[c] = *reinterpret_cast<const uint4*>(wrow[c] + k);
+            if constexpr (GATED) p.u[c] = *reinterpret_cast<const uint4*>(wrow[c] + up + k);
+        }
+    };
+    Pieces now;
+    if (GATED && vec && lane * VN < K) ask(lane * VN, now);
     for (int r = 0; r < count; ++r) {
         const int p = p0 + r;
         const T* src = x + (size_t)(row_map ? row_map[p] / row_div : p) * K;
@@ -239,44 +300,39 @@ __global__ void __launch_bounds__(256, 2) moe_rows_kernel(const T* __restrict__ 
         }
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const T* we = w + (size_t)e * (GATED ? 2 : 1) * F * K;
-    constexpr int CPW = MOE_COLS / 8;   // a warp's outputs, taken together: their weight rows are in flight at once
-    const int j0 = blockIdx.x * MOE_COLS + warp * CPW;
     if (j0 >= F) return;
-    const T* wrow[CPW];
-#pragma unroll
-    for (int c = 0; c < CPW; ++c) wrow[c] = we + (size_t)min(j0 + c, F - 1) * K;   // (an output past the end repeats the last: not stored)
-    const size_t up = (size_t)F * K;   // from an output's gate row to its up row (read only when GATED)
     float ag[CPW][MOE_TM] = {}, au[GATED ? CPW : 1][MOE_TM] = {};
     if (vec) {
         for (int k = lane * VN; k < K; k += 32 * VN) {
-            float g[CPW][VN], u[GATED ? CPW : 1][VN];
+            Pieces next;
+            if constexpr (!GATED) ask(k, now);
+            else if (k + 32 * VN < K) ask(k + 32 * VN, next);
 #pragma unroll
-            for (int c = 0; c < CPW; ++c) {
-                Vec16<T>::load(wrow[c] + k, g[c]);
-                if (GATED) Vec16<T>::load(wrow[c] + up + k, u[GATED ? c : 0]);
-            }
+            for (int i = 0; i < VN; i += 4) {   // (four entries of every piece at a time as floats: all of them would not fit the registers)
+                float g[CPW][4], u[GATED ? CPW : 1][4];
 #pragma unroll
-            for (int r = 0; r < MOE_TM; ++r) {
-                if (r < count) {
-                    const float* a = moe_rows_smem + (size_t)r * K + k;
+                for (int c = 0; c < CPW; ++c) {
+                    load4(reinterpret_cast<const T*>(&now.g[c]) + i, g[c]);
+                    if constexpr (GATED) load4(reinterpret_cast<const T*>(&now.u[c]) + i, u[c]);
+                }
 #pragma unroll
-                    for (int i = 0; i < VN; i += 4) {
-                        const float4 av = *reinterpret_cast<const float4*>(a + i);
+                for (int r = 0; r < MOE_TM; ++r) {
+                    if (r < count) {
+                        const float4 av = *reinterpret_cast<const float4*>(moe_rows_smem + (size_t)r * K + k + i);
 #pragma unroll
                         for (int c = 0; c < CPW; ++c) {
-                            ag[c][r] = fmaf(av.x, g[c][i], ag[c][r]); ag[c][r] = fmaf(av.y, g[c][i + 1], ag[c][r]);
-                            ag[c][r] = fmaf(av.z, g[c][i + 2], ag[c][r]); ag[c][r] = fmaf(av.w, g[c][i + 3], ag[c][r]);
-                            if (GATED) {
-                                float& s = au[GATED ? c : 0][r];
-                                s = fmaf(av.x, u[GATED ? c : 0][i], s); s = fmaf(av.y, u[GATED ? c : 0][i + 1], s);
-                                s = fmaf(av.z, u[GATED ? c : 0][i + 2], s); s = fmaf(av.w, u[GATED ? c : 0][i + 3], s);
+                            ag[c][r] = fmaf(av.x, g[c][0], ag[c][r]); ag[c][r] = fmaf(av.y, g[c][1], ag[c][r]);
+                            ag[c][r] = fmaf(av.z, g[c][2], ag[c][r]); ag[c][r] = fmaf(av.w, g[c][3], ag[c][r]);
+                            if constexpr (GATED) {
+                                float& s = au[c][r];
+                                s = fmaf(av.x, u[c][0], s); s = fmaf(av.y, u[c][1], s);
+                                s = fmaf(av.z, u[c][2], s); s = fmaf(av.w, u[c][3], s);
                             }
                         }
                     }
                 }
             }
+            if constexpr (GATED) now = next;
         }
     } else {
         for (int k = lane; k < K; k += 32) {
