@@ -92,6 +92,17 @@ def test_layernorm_and_the_norm_of_a_result(K, dtype, N, H):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("gs,groups,shared", [(260, 2, False), (512, 1, True), (1020, 3, False), (1024, 2, True), (1028, 1, False), (4096, 1, False), (4100, 1, False)])
+def test_group_norm_with_gate_on_whole_groups_in_registers(K, dtype, gs, groups, shared):
+    """Groups that a block holds in registers (aligned rows of 257 to 4,096 channels), one piece per thread, several, and one group too long."""
+    ref, T, C, N = TorchKernels(), TD[dtype], gs * groups, 3
+    x, gate, w = rnd(N, C, seed=1, scale=2.0), rnd(N, C + 8, seed=2).to(T), 1 + rnd(gs if shared else C, seed=3, scale=0.2)
+    for gate_first, act in ((True, "sigmoid"), (False, "sigmoid"), (False, "silu")):
+        got = K.group_rmsnorm_gate(x.cuda(), gate.cuda(), 8, w.cuda(), gs, 1e-5, gate_first, T, gate_act=act)
+        close(got, ref.group_rmsnorm_gate(x, gate, 8, w, gs, 1e-5, gate_first, T, gate_act=act), dtype, f"{gs} x {groups}, gate first {gate_first}, {act}")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_group_norm_with_gate_mix_of_two_and_gated_unit(K, dtype):
     ref, T = TorchKernels(), TD[dtype]
     for N, C, gs, shared in ((7, 96, 32, False), (3, 120, 40, True), (40, 512, 512, False), (2, 66, 33, True), (5, 2048, 1024, False)):
@@ -180,6 +191,31 @@ def test_short_convolution_over_ragged_steps(K, dtype, C, taps, bias, act):
         want = ref.causal_conv(z, 4, C, w, b, state, host, act)
         close(got, want, dtype, f"causal_conv step {step}", f32=4e-6)
         assert torch.equal(dstate.cpu(), state), "the convolution's state is a copy of inputs"
+
+
+@pytest.mark.parametrize("taps", [1, 2, 4, 8])
+def test_short_convolution_whatever_the_cut(K, taps):
+    """Portions whose lengths end inside and at the end of the kernel's batches of 8 and chunks of 32 tokens: the same bits, and the same state."""
+    C, N = 70, 101
+    z, w, b = rnd(N, C, seed=1), rnd(C, taps, seed=2), rnd(C, seed=3)
+
+    def run(cuts):
+        state = torch.zeros(2, taps - 1, C).cuda()
+        outs = []
+        for lo, hi in cuts:
+            _, dev = ragged([hi - lo], [1])
+            outs.append(K.causal_conv(z[lo:hi].contiguous().cuda(), 0, C, w.cuda(), b.cuda(), state, dev, "silu"))
+        return torch.cat(outs), state
+
+    whole, end = run([(0, N)])
+    for sizes in ([1], [8], [7, 1, 9], [32, 33], [3, 40]):
+        cuts, at = [], 0
+        while at < N:
+            n = min(sizes[len(cuts) % len(sizes)], N - at)
+            cuts.append((at, at + n))
+            at += n
+        got, state = run(cuts)
+        assert torch.equal(got, whole) and torch.equal(state, end), f"{taps} taps, portions of {sizes}"
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
