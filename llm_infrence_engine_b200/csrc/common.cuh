@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "per_device.h"
+
 #define LLMIE_API extern "C" __attribute__((visibility("default")))
 
 // Return codes of the exported functions (0 and CUDA's own codes are passed through unchanged).
@@ -137,6 +139,15 @@ __device__ __forceinline__ float gated_unit(float g, float u, float limit, float
 
 static inline int launch_status() {
     return (int)cudaGetLastError();
+}
+
+// Room in shared memory beyond 48 KB: the runtime keeps it per kernel AND per device. `granted` belongs to the kernel.
+template <typename Kernel>
+static inline int grant_shared(OncePerDevice& granted, Kernel kernel, int bytes) {
+    int device = 0;
+    const int rc = (int)cudaGetDevice(&device);
+    if (rc) return rc;
+    return granted.run(device, [&] { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -367,8 +367,8 @@ int run_small(const F32Args& p, cudaStream_t s) {
     const Slices sl = slices_of(p.K);
     const int warps = (p.M + R - 1) / R, stages = min(SMALL_STAGES, (sl.length + CHUNK - 1) / CHUNK);
     constexpr int most = SMALL_STAGES * (32 + SMALL_ROWS) * CHUNK_PITCH * 4;
-    static const int set = (int)cudaFuncSetAttribute(small_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    if (set) return set;
+    static OncePerDevice granted;
+    if (const int rc = grant_shared(granted, small_kernel<R>, most)) return rc;
     return launch_sliced(small_kernel<R>, dim3((p.N + 31) / 32, sl.count), dim3(32 * warps), dim3(1, sl.count, 1),
                          (size_t)stages * (32 + warps * R) * CHUNK_PITCH * 4, s, p, stages);
 }
@@ -376,8 +376,8 @@ int run_small(const F32Args& p, cudaStream_t s) {
 template <int COLS>
 int run_tiles(const F32Args& p, cudaStream_t s) {
     constexpr int smem = TILE_STAGES * (TILE_M + 16 * COLS) * TILE_PITCH * 4;
-    static const int set = (int)cudaFuncSetAttribute(tile_kernel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (set) return set;
+    static OncePerDevice granted;
+    if (const int rc = grant_shared(granted, tile_kernel<COLS>, smem)) return rc;
     const Slices sl = slices_of(p.K);
     return launch_sliced(tile_kernel<COLS>, dim3((p.N + 16 * COLS - 1) / (16 * COLS), (p.M + TILE_M - 1) / TILE_M, sl.count), dim3(128),
                          dim3(1, 1, sl.count), smem, s, p, 0);

@@ -318,8 +318,8 @@ int launch_scan_as(const T* v, int v_stride, int v_col, const float* qf, const f
     constexpr int COLS = ML_THREADS / ml_parts(DM) * CPL;
     constexpr int smem = 4 * 2 * ML_TILE * (2 * DM + COLS + 2);
     if (smem > 48 * 1024) {
-        static const int set = (int)cudaFuncSetAttribute(mlstm_scan_kernel<T, DM, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (set) return set;
+        static OncePerDevice granted;
+        if (const int rc = grant_shared(granted, mlstm_scan_kernel<T, DM, CPL>, smem)) return rc;
     }
     const dim3 grid((DV + 1 + COLS - 1) / COLS, H, R);
     return launch_kernel_on(alone, mlstm_scan_kernel<T, DM, CPL>, grid, dim3(ML_THREADS + 32), (size_t)smem, s, v, v_stride, v_col, qf, kf, ig, fg, state,
