@@ -50,6 +50,7 @@ struct Params {
     // keys include the token's own position finishes that key and value, puts them into its chunk and into the cache.
     const float* qkv_acc;   // [tokens][acc_stride]: query heads, key heads, value heads; or null
     const float* bias;      // [(nq + 2 nkv) * D] or null
+    int bias_at_rest = 0;   // it may be read before the kernels ahead have finished
     const float* cos_t;     // [tokens][D / 2]
     const float* sin_t;
     const int* slots;       // [tokens] cache slot (page * page_size + offset) of the token's own key and value; null: already cached
@@ -547,9 +548,10 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
         fetched[s] = early && s < mine && (own_here || key0 + BN <= pos0);  // wholly before the first new position
         if (fetched[s]) copy_rows_warp<D, BN, SHARED>(p, rows_at[s], 0, my + s * SLOT, my + s * SLOT + V_AT, lane, my_numbers + s * BN);
     }
-    // the biases of the projection are weights: they are asked for before the wait as well
+    // biases at rest are asked for before the wait as well
     float q_bias[T8 ? D / 16 : 1][4];
     if constexpr (T8) {
+        if (early && p.qkv_acc && p.bias) pdl_wait_unless(p.bias_at_rest);
         const int head = kvh * G + ((lane >> 2) < nrows ? lane >> 2 : 0);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
@@ -1120,7 +1122,8 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
                    bf16* out, float* scratch_o, float* scratch_ml, int* counters, int nq, int nkv, int d,
                    int page_size, float scale, int window, int num_splits, int decode_mode, int cluster, const float* qkv_acc,
                    int acc_stride, const float* bias, const float* cos_t, const float* sin_t, const int* slots, const float* turn_cos, const float* turn_sin,
-                   const float* sig_bias, const float* log_r1, const float* log_r2, int balanced, int num_sms, cudaStream_t s, const Params* extras = nullptr) {
+                   const float* sig_bias, const float* log_r1, const float* log_r2, int balanced, int num_sms, cudaStream_t s, const Params* extras = nullptr,
+                   int bias_at_rest = 0) {
     if (num_tiles <= 0) return 0;
     if ((turn_cos == nullptr) != (turn_sin == nullptr) || (log_r1 == nullptr) != (log_r2 == nullptr) || (log_r1 && !sig_bias) ||
         ((turn_cos || sig_bias) && !decode_mode))
@@ -1142,7 +1145,7 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
     p.q_stride = q_stride; p.max_blocks = max_blocks; p.nq = nq; p.nkv = nkv; p.page_size = page_size; p.window = window;
     p.page_shift = (page_size & (page_size - 1)) == 0 ? __builtin_ctz((unsigned)page_size) : -1;
     p.num_splits = num_splits; p.balanced = balanced; p.scale_log2 = scale * LOG2E; p.cluster = cluster;
-    p.qkv_acc = qkv_acc; p.acc_stride = acc_stride; p.bias = bias; p.cos_t = cos_t; p.sin_t = sin_t; p.slots = slots;
+    p.qkv_acc = qkv_acc; p.acc_stride = acc_stride; p.bias = bias; p.bias_at_rest = bias_at_rest; p.cos_t = cos_t; p.sin_t = sin_t; p.slots = slots;
     p.turn_cos = turn_cos; p.turn_sin = turn_sin; p.sig_bias = sig_bias; p.log_r1 = log_r1; p.log_r2 = log_r2;
     if (extras) {
         p.chunk = extras->chunk; p.cap_log2 = extras->cap_log2; p.x_scale = extras->x_scale; p.rel = extras->rel; p.rows_of = extras->rows_of;
@@ -1192,9 +1195,9 @@ LLMIE_API int llmie_paged_attention_mma_acc(const float* qkv_acc, int acc_stride
                                             const int* slots, bf16* k_pool, bf16* v_pool, const int* block_table, int max_blocks,
                                             const int* token_seq, const int* positions, int num_tokens, bf16* out, float* scratch_o,
                                             float* scratch_ml, int* counters, int nq, int nkv, int d, int page_size, float scale, int window,
-                                            int num_splits, int cluster, int four_warps, int balanced, int num_sms, cudaStream_t s) {
+                                            int num_splits, int cluster, int four_warps, int balanced, int num_sms, int bias_at_rest, cudaStream_t s) {
     if (!qkv_acc) return LLMIE_ERR_BAD_ARGUMENT;
     return run_mma(nullptr, 8, k_pool, v_pool, block_table, max_blocks, token_seq, positions, nullptr, num_tokens, out, scratch_o, scratch_ml,
                    counters, nq, nkv, d, page_size, scale, window, num_splits, four_warps ? 2 : 1, cluster, qkv_acc, acc_stride, bias, cos_t, sin_t, slots,
-                   nullptr, nullptr, nullptr, nullptr, nullptr, balanced, num_sms, s);
+                   nullptr, nullptr, nullptr, nullptr, nullptr, balanced, num_sms, s, nullptr, bias_at_rest);
 }

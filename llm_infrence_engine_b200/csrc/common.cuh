@@ -159,6 +159,9 @@ static inline int grant_shared(OncePerDevice& granted, Kernel kernel, int bytes)
 // stays ordered along the stream. pdl_trigger() lets the next kernel's blocks be scheduled from now on.
 // Without the launch attribute both are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// Parameters that lie at rest (a model's weights, written when it was loaded) may be read before the wait. Only the caller knows whether they
+// do: a matrix that a kernel has just made is one of the things that kernel wrote.
+__device__ __forceinline__ void pdl_wait_unless(int at_rest) { if (!at_rest) pdl_wait(); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
 extern "C" int llmie_pdl_flag;  // 1: launch with the programmatic-serialization attribute (set by llmie_set_pdl)

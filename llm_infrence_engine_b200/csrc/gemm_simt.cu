@@ -11,7 +11,7 @@
 //
 //   small_kernel    M <= 16: weights stream at memory speed. A block owns 32 outputs (one per lane) of ONE slice and fetches its
 //                   32 rows of it with asynchronous 16-byte copies, up to SMALL_STAGES chunks of 128 k in flight, the first ones
-//                   before the kernel ahead has finished; a warp takes up to 4 token rows. The slices of an output are a cluster.
+//                   before the kernel ahead has finished (weights at rest); a warp takes up to 4 token rows. The slices of an output are a cluster.
 //   tile_kernel     more rows: bound by the multiply-adds. 64 x 64 or 64 x 128 outputs of one slice per block, 8 x 4 or 8 x 8 per
 //                   thread, both operands row-major in shared memory (rows 36 floats apart: eight lanes' 16-byte reads fall into
 //                   eight different bank groups), so nothing is transposed; the slices of a tile are a cluster, which adds
@@ -145,6 +145,7 @@ struct F32Args {
     const float *A, *W, *bias;
     float* C;
     int M, N, K, accumulate;
+    int at_rest;   // W was written before the kernels that may still be running: see pdl_wait_unless
 };
 
 __device__ __forceinline__ void put(const F32Args& p, int m, int n, float v) {
@@ -181,7 +182,8 @@ __global__ void __launch_bounds__(128) small_kernel(F32Args p, int stages) {
     };
     pdl_trigger();
     const int early = min(stages, chunks);
-    for (int c = 0; c < early; ++c) fetch_weights(c);   // nobody writes the weights: they are fetched while the kernel ahead still runs
+    pdl_wait_unless(p.at_rest);
+    for (int c = 0; c < early; ++c) fetch_weights(c);   // weights at rest are fetched while the kernel ahead still runs
     pdl_wait();
     for (int c = 0; c < early; ++c) fetch_tokens(c);
     copies_commit();
@@ -274,6 +276,7 @@ __global__ void __launch_bounds__(128) tile_kernel(F32Args p) {
 #pragma unroll
         for (int j = 0; j < COLS; ++j) acc[i][j] = make_float2(0.f, 0.f);
     pdl_trigger();
+    pdl_wait_unless(p.at_rest);
     for (int t = 0; t < TILE_STAGES - 1; ++t)
         if (t < steps) fetch(t, true, false);
     pdl_wait();
@@ -399,16 +402,16 @@ int run_f32(const F32Args& p, cudaStream_t s) {
 
 }  // namespace
 
-// in_dtype / out_dtype: 0 float32, 1 bfloat16; bias (or null) in in_dtype. Beyond K the tiles are padded with zeros, which add nothing.
+// in_dtype / out_dtype: 0 float32, 1 bfloat16; bias (or null) in in_dtype; at_rest: W may be read before the kernels ahead have finished. Beyond K the tiles are padded with zeros, which add nothing.
 LLMIE_API int llmie_gemm_simt(const void* A, const void* W, void* C, int M, int N, int K, int in_dtype, int out_dtype,
-                              int accumulate, const void* bias, cudaStream_t s) {
+                              int accumulate, const void* bias, int at_rest, cudaStream_t s) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return LLMIE_ERR_BAD_ARGUMENT;
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     const int vec = (K % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
     if (in_dtype == DT_F32 && out_dtype == DT_F32) {
         if (vec && (M + TILE_M - 1) / TILE_M <= 65535)
-            return run_f32({(const float*)A, (const float*)W, (const float*)bias, (float*)C, M, N, K, accumulate}, s);
+            return run_f32({(const float*)A, (const float*)W, (const float*)bias, (float*)C, M, N, K, accumulate, at_rest}, s);
         gemm_simt_kernel<float, float><<<grid, 256, 0, s>>>((const float*)A, (const float*)W, (float*)C, M, N, K, vec, accumulate, (const float*)bias);
     } else if (in_dtype == DT_BF16 && out_dtype == DT_F32)
         gemm_simt_kernel<bf16, float><<<grid, 256, 0, s>>>((const bf16*)A, (const bf16*)W, (float*)C, M, N, K, vec, accumulate, (const bf16*)bias);

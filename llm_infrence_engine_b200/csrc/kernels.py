@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from typing import Optional
 
 import torch
@@ -37,6 +38,20 @@ def _ptr(t: Optional[torch.Tensor]):
 
 class KernelError(RuntimeError):
     pass
+
+
+class AtRest(threading.local):
+    """``with kernels.at_rest:`` around calls whose weights were all written long before, as a loaded model's are: kernels that can then
+    fetch them while the kernel before is still running. Everywhere else a weight may be what that kernel is just writing. A thread's
+    own, and it nests."""
+
+    depth = 0
+
+    def __enter__(self):
+        self.depth += 1
+
+    def __exit__(self, *exc):
+        self.depth -= 1
 
 
 class CudaKernels:
@@ -121,6 +136,7 @@ class CudaKernels:
         self._decode_four_warps = False         # the last decode plan asked for blocks of four warps
         self._decode_balanced = 0               # ... and for blocks dealt out by the lengths of this many tokens
         self.balance_decode = True
+        self.at_rest = AtRest()
         for fn in ("llmie_embed", "llmie_feed_tokens", "llmie_zero_fresh_state", "llmie_rope_tables", "llmie_add_rmsnorm", "llmie_rope_kv_write", "llmie_silu_mul",
                    "llmie_gemm_simt", "llmie_gemm_tc", "llmie_gateup_silu_tc", "llmie_qkv_rope_tc", "llmie_add_into", "llmie_attn_plan", "llmie_attn_tc_plan", "llmie_paged_attention_mma", "llmie_paged_attention_mma_acc", "llmie_paged_attention_tc", "llmie_paged_attention_f32", "llmie_paged_attention_bf16", "llmie_argmax", "llmie_sample",
                    "llmie_streams_expand", "llmie_streams_update", "llmie_streams_norm", "llmie_latent_prepare", "llmie_head_matmul",
@@ -189,6 +205,9 @@ class CudaKernels:
         if rc == _ERR_BAD_ARGUMENT:
             raise KernelError(f"{what}: the kernel refused its arguments")
         raise KernelError(f"{what}: CUDA error {rc}")
+
+    def _weights_at_rest(self) -> int:
+        return int(self.at_rest.depth > 0)
 
     @staticmethod
     def _need(t: torch.Tensor, name: str, dtype=None, dims: Optional[int] = None) -> None:
@@ -419,7 +438,8 @@ class CudaKernels:
         nothing is returned. ``transient``: the caller hands the result straight to ``rope_kv_write`` or ``silu_mul``
         and nowhere else; for small bfloat16 batches it is then a float32 view of the library's accumulation buffer,
         which those kernels read and set back to zero. ``x`` may be a run of columns of wider rows (unit column stride): the
-        library product takes it as it is, every other path gets a copy."""
+        library product takes it as it is, every other path gets a copy. In float32 ``w`` may be the result of a kernel launched
+        just before; the tensor cores' small-batch product (bfloat16) fetches ``w`` ahead of the kernel before, so there it has to lie at rest."""
         if x.dim() == 2 and not x.is_contiguous():
             as_it_is = (x.stride(1) == 1 and x.dtype == torch.bfloat16 and self.use_cublas and add_to is None and not transient
                         and (out_dtype or x.dtype) == torch.bfloat16 and x.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0)
@@ -452,8 +472,8 @@ class CudaKernels:
                 self.launches += 1
                 self._pending_add = (add_to, torch.nn.functional.linear(x, w, bias))  # added by the norm that follows, or by flush()
             else:
-                self._check(self.lib.llmie_gemm_simt(_ptr(x), _ptr(w), _ptr(add_to), M, N, K, self._dt(x, "x"), 0, 1, _ptr(bias), self._stream()),
-                            "linear (accumulate)")
+                self._check(self.lib.llmie_gemm_simt(_ptr(x), _ptr(w), _ptr(add_to), M, N, K, self._dt(x, "x"), 0, 1, _ptr(bias), self._weights_at_rest(),
+                                                     self._stream()), "linear (accumulate)")
             return None
         out_dtype = out_dtype or x.dtype
         if small and transient:
@@ -468,7 +488,7 @@ class CudaKernels:
             return torch.nn.functional.linear(x, w, bias)
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
         self._check(self.lib.llmie_gemm_simt(_ptr(x), _ptr(w), _ptr(out), M, N, K, self._dt(x, "x"), self._dt(out, "out"), 0,
-                                             _ptr(bias), self._stream()), "linear")
+                                             _ptr(bias), self._weights_at_rest(), self._stream()), "linear")
         return out
 
     def _check_bias(self, bias, x, w) -> None:
@@ -877,7 +897,7 @@ class CudaKernels:
                 _ptr(sums), width, _ptr(bias), _ptr(cos), _ptr(sin), _ptr(slot_mapping if write_kv else None), _ptr(k_pool), _ptr(v_pool),
                 _ptr(block_table), block_table.shape[1], _ptr(token_seq), _ptr(positions), M, _ptr(out), _ptr(scratch_o), _ptr(scratch_ml),
                 _ptr(counters), num_heads, num_kv_heads, head_dim, page_size, ctypes.c_float(scale), int(window), num_splits, cluster,
-                int(self._decode_four_warps), self._decode_balanced, self.num_sms, self._stream()), "qkv_attention (tensor cores)")
+                int(self._decode_four_warps), self._decode_balanced, self.num_sms, self._weights_at_rest(), self._stream()), "qkv_attention (tensor cores)")
             self._dirty_qkv = sums
             return out
         qkv = self.qkv_rope(x, w, bias, cos, sin, slot_mapping, k_pool, v_pool, num_heads, num_kv_heads, head_dim, page_size, write_kv,
@@ -1586,7 +1606,8 @@ class CudaKernels:
         out = torch.empty((N, C), dtype=out_dtype, device=x.device)
         self._check(self.lib.llmie_group_rmsnorm_gate(_ptr(x), ctypes.c_void_p(gate.data_ptr() + gate_col * gate.element_size()), gate.stride(0),
                                                       self._dt(gate, "gate"), _ptr(weight), weight.shape[0], _ptr(out), _DT[out_dtype], N, C,
-                                                      group_size, ctypes.c_float(eps), 0 if gate_first else (2 if gate_act == "silu" else 1), self._stream()), "group_rmsnorm_gate")
+                                                      group_size, ctypes.c_float(eps), 0 if gate_first else (2 if gate_act == "silu" else 1), self._weights_at_rest(), self._stream()),
+                    "group_rmsnorm_gate")
         return out
 
     def dual_rmsnorm_mix(self, a, b, weight_a, weight_b, eps, coef, add_to):
@@ -1940,7 +1961,7 @@ class CudaKernels:
         weights = torch.empty((N, top), dtype=torch.float32, device=h.device)
         out_gates = torch.empty((N, gates), dtype=torch.float32, device=h.device)
         self._check(self.lib.llmie_moe_router(_ptr(h), _ptr(w_router), _ptr(correction), _ptr(ids), _ptr(weights), N, K, total, top, self._SCORING[scoring],
-                                              _ptr(bias), int(gates), _ptr(out_gates if gates else None), self._dt(h, "h"), self._stream()), "moe_router")
+                                              _ptr(bias), int(gates), _ptr(out_gates if gates else None), self._weights_at_rest(), self._dt(h, "h"), self._stream()), "moe_router")
         return (ids, weights, out_gates) if bias is not None or gates else (ids, weights)
 
     def moe_experts(self, h, ids, weights, w_gate_up, w_down, add_to, glu=None, weight_inputs=False):
@@ -2053,7 +2074,7 @@ class CudaKernels:
             mode = 3
         self._check(self.lib.llmie_head_matmul(_ptr(q), q.shape[1], head_dim + rot_dim, _ptr(w_uk), _ptr(out), out.shape[1], kv_rank + rot_dim,
                                                N, num_heads, head_dim, kv_rank, mode, rot_dim, rot_dims, _ptr(cos), _ptr(sin), _ptr(None), 0,
-                                               self._dt(q, "q"), self._stream()), "latent_absorb")
+                                               self._weights_at_rest(), self._dt(q, "q"), self._stream()), "latent_absorb")
         return out
 
     def latent_expand(self, o_lat, w_uv, gate, gate_col, num_heads, kv_rank, v_head_dim):
@@ -2080,12 +2101,12 @@ class CudaKernels:
         if gate is None:
             self._check(self.lib.llmie_head_matmul(_ptr(o_lat), o_lat.shape[1], kv_rank, _ptr(w_uv), _ptr(out), out.shape[1], v_head_dim, N,
                                                    num_heads, kv_rank, v_head_dim, mode, 0, 0, _ptr(None), _ptr(None), _ptr(None), 0,
-                                                   self._dt(o_lat, "o_lat"), self._stream()), "latent_expand")
+                                                   self._weights_at_rest(), self._dt(o_lat, "o_lat"), self._stream()), "latent_expand")
             return out
         self._check(self.lib.llmie_head_matmul(_ptr(o_lat), o_lat.shape[1], kv_rank, _ptr(w_uv), _ptr(out), out.shape[1], v_head_dim, N,
                                                num_heads, kv_rank, v_head_dim, mode, 0, 0, _ptr(None), _ptr(None),
                                                ctypes.c_void_p(gate.data_ptr() + gate_col * gate.element_size()), gate.shape[1],
-                                               self._dt(o_lat, "o_lat"), self._stream()), "latent_expand")
+                                               self._weights_at_rest(), self._dt(o_lat, "o_lat"), self._stream()), "latent_expand")
         return out
 
     def argmax(self, logits):

@@ -59,13 +59,13 @@ enum { MODE_PLAIN = 0, MODE_ABSORB = 1, MODE_EXPAND = 2, MODE_ABSORB_TAIL = 3, M
 // each, in order, and their partial sums are added in the order of the warps: every result is one fixed sequence of 32-bit
 // multiply-adds, whatever the batch holds.
 // STAGED: the block's 32 columns of the matrix are copied to shared memory first, all of them on their way before the kernel ahead
-// has finished (the matrix is a weight): read from global memory 8 rows at a time, a trip to memory per 8 was most of what the
+// has finished (a matrix at rest): read from global memory 8 rows at a time, a trip to memory per 8 was most of what the
 // kernel took for a few decoded tokens (14 heads, 64 x 256 and 256 x 64: 9.7 -> 4.9 us). Needs columns in whole 16-byte pieces.
 template <typename T, bool STAGED>
 __global__ void __launch_bounds__(128) head_matmul_kernel(const T* __restrict__ x, int x_stride, int x_head, const T* __restrict__ M,
                                                          T* __restrict__ out, int out_stride, int out_head, int N, int K, int J, int mode,
                                                          int R, int rot_dims, const float* __restrict__ cos_t,
-                                                         const float* __restrict__ sin_t, const T* __restrict__ gate, int gate_stride) {
+                                                         const float* __restrict__ sin_t, const T* __restrict__ gate, int gate_stride, int at_rest) {
     extern __shared__ __align__(16) float xs[];   // [TOK][KP], then [4][TOK][32] partial sums, then (STAGED) [K][32] of the matrix
     const int KP = (K + 3) & ~3;
     float* part = xs + TOK * KP;
@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(128) head_matmul_kernel(const T* __restrict__ 
     pdl_trigger();
     if constexpr (STAGED) {   // (launched so for modes with a product only)
         constexpr int PIECE = 16 / sizeof(T), PER_ROW = 32 / PIECE;
+        pdl_wait_unless(at_rest);
         const T* from = M + (size_t)blockIdx.y * K * J + blockIdx.z * 32;
         for (int i = threadIdx.x; i < K * PER_ROW; i += blockDim.x) {
             const int k = i / PER_ROW, c = i % PER_ROW * PIECE;
@@ -183,7 +184,7 @@ int prepare(const T* z, int z_stride, int q_rank, int kv_rank, int rot_dim, int 
 
 template <typename T>
 int head_matmul(const T* x, int x_stride, int x_head, const T* M, T* out, int out_stride, int out_head, int N, int H, int K, int J, int mode,
-                int R, int rot_dims, const float* cos_t, const float* sin_t, const T* gate, int gate_stride, cudaStream_t s) {
+                int R, int rot_dims, const float* cos_t, const float* sin_t, const T* gate, int gate_stride, int at_rest, cudaStream_t s) {
     const size_t rows = sizeof(float) * (TOK * (size_t)((K + 3) & ~3) + 4 * TOK * 32), columns = (size_t)K * 32 * sizeof(T);
     const int jchunks = mode == MODE_ABSORB_TAIL ? 1 : (J + 31) / 32;   // the tail alone is one block's work per tokens and head
     if (rows > 200 * 1024 || H > 65535 || jchunks > 65535) return LLMIE_ERR_BAD_ARGUMENT;
@@ -193,7 +194,7 @@ int head_matmul(const T* x, int x_stride, int x_head, const T* M, T* out, int ou
     auto kernel = staged ? head_matmul_kernel<T, true> : head_matmul_kernel<T, false>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return launch_kernel(kernel, dim3((N + TOK - 1) / TOK, H, jchunks), dim3(128), smem, s, x, x_stride, x_head, M, out, out_stride,
-                         out_head, N, K, J, mode, R, rot_dims, cos_t, sin_t, gate, gate_stride);
+                         out_head, N, K, J, mode, R, rot_dims, cos_t, sin_t, gate, gate_stride, at_rest);
 }
 
 }  // namespace
@@ -211,15 +212,15 @@ LLMIE_API int llmie_latent_prepare(const void* z, int z_stride, int q_rank, int 
 }
 
 // mode 0: plain; 1: absorb (R further entries of every head of x are copied behind the J results, the first rot_dims of them
-// turned); 2: expand (results times sigmoid(gate)).
+// turned); 2: expand (results times sigmoid(gate)). at_rest: M may be read before the kernels ahead have finished.
 LLMIE_API int llmie_head_matmul(const void* x, int x_stride, int x_head, const void* M, void* out, int out_stride, int out_head, int N, int H,
                                 int K, int J, int mode, int R, int rot_dims, const float* cos_t, const float* sin_t, const void* gate,
-                                int gate_stride, int dtype, cudaStream_t s) {
+                                int gate_stride, int at_rest, int dtype, cudaStream_t s) {
     if (N <= 0) return 0;
     if (K < 1 || J < 1 || H < 1 || mode < 0 || mode > 4 || ((mode == 1 || mode == 3) && (rot_dims > R || (rot_dims & 1) || (rot_dims && (!cos_t || !sin_t)))) ||
         ((mode == 2 || mode == 4) && !gate))
         return LLMIE_ERR_BAD_ARGUMENT;
     if (dtype == DT_F32)
-        return head_matmul<float>((const float*)x, x_stride, x_head, (const float*)M, (float*)out, out_stride, out_head, N, H, K, J, mode, R, rot_dims, cos_t, sin_t, (const float*)gate, gate_stride, s);
-    return head_matmul<bf16>((const bf16*)x, x_stride, x_head, (const bf16*)M, (bf16*)out, out_stride, out_head, N, H, K, J, mode, R, rot_dims, cos_t, sin_t, (const bf16*)gate, gate_stride, s);
+        return head_matmul<float>((const float*)x, x_stride, x_head, (const float*)M, (float*)out, out_stride, out_head, N, H, K, J, mode, R, rot_dims, cos_t, sin_t, (const float*)gate, gate_stride, at_rest, s);
+    return head_matmul<bf16>((const bf16*)x, x_stride, x_head, (const bf16*)M, (bf16*)out, out_stride, out_head, N, H, K, J, mode, R, rot_dims, cos_t, sin_t, (const bf16*)gate, gate_stride, at_rest, s);
 }

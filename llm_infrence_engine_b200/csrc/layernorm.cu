@@ -127,15 +127,16 @@ int launch_layernorm(float* x, void* y, const float* w_post, int clear_y, const 
 //   mode 2: out = x / rms(x) * w * silu(gate)
 // w has w_len entries and channel c uses w[c % w_len] (one weight per channel, or one vector shared by all groups).
 // Rows that a block's threads hold at once (four neighbouring channels each, GROUP_HELD pieces): x and gate in one trip to memory, the
-// weights before the wait for the kernel ahead. Read again after the sum, and one channel at a time, they were two more trips and most of the
+// weights, at rest, before the wait for the kernel ahead. Read again after the sum, and one channel at a time, they were two more trips and most of the
 // kernel (1,024 channels, 16 rows: 5.0 -> 2.3 us).
 constexpr int GROUP_HELD = 4;
 template <typename TG, typename TO>
 __global__ void __launch_bounds__(256) group_rmsnorm_gate_held_kernel(const float* __restrict__ x, const TG* __restrict__ gate, int gate_stride,
                                                                       const float* __restrict__ w, int w_len, TO* __restrict__ out, int C, int gs,
-                                                                      float eps, int mode) {
+                                                                      float eps, int mode, int at_rest) {
     __shared__ float scratch[36];
     pdl_trigger();
+    pdl_wait_unless(at_rest);
     const int n = blockIdx.x, c0 = blockIdx.y * gs, step = blockDim.x * 4;
     float v[GROUP_HELD][4], z[GROUP_HELD][4], wt[GROUP_HELD][4];
 #pragma unroll
@@ -316,7 +317,7 @@ LLMIE_API int llmie_layernorm(float* x, void* y, int y_dtype, const float* w_pos
 }
 
 LLMIE_API int llmie_group_rmsnorm_gate(const float* x, const void* gate, int gate_stride, int gate_dtype, const float* w, int w_len,
-                                       void* out, int out_dtype, int N, int C, int gs, float eps, int mode, cudaStream_t s) {
+                                       void* out, int out_dtype, int N, int C, int gs, float eps, int mode, int at_rest, cudaStream_t s) {
     if (N <= 0) return 0;
     if (C <= 0 || gs <= 0 || C % gs || w_len <= 0 || C / gs > 65535 || mode < 0 || mode > 2) return LLMIE_ERR_BAD_ARGUMENT;
     int threads = 32;
@@ -335,7 +336,7 @@ LLMIE_API int llmie_group_rmsnorm_gate(const float* x, const void* gate, int gat
                                  gate_stride, w, w_len, (TO*)out, N, C, gs, eps, mode);                                                          \
         if (held)                                                                                                                                \
             return launch_kernel(group_rmsnorm_gate_held_kernel<TG, TO>, grid, dim3(held_threads), 0, s, x, (const TG*)gate, gate_stride, w,     \
-                                 w_len, (TO*)out, C, gs, eps, mode);                                                                             \
+                                 w_len, (TO*)out, C, gs, eps, mode, at_rest);                                                                    \
         return launch_kernel(group_rmsnorm_gate_kernel<TG, TO>, grid, dim3(threads), 0, s, x, (const TG*)gate, gate_stride, w, w_len, (TO*)out,  \
                              C, gs, eps, mode);                                                                                                  \
     }

@@ -114,15 +114,15 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
 // The router's product and its choice in one kernel, a block per token: the token's row lies in shared memory as floats, the warps
 // share the router's outputs (a warp's lanes walk an output's weight row in 16-byte pieces; the sum runs over K in one order whatever
 // the step holds), and the first warp chooses from the logits in shared memory. For the few rows of a decode step, where the product
-// alone would be a kernel that walks K in one block. It is a chain of trips to memory, and the matrix is nobody's result: a warp's first
-// ROUTER_EARLY pieces of it are asked for before the kernel ahead has finished, the others that many at a time (a trip per piece was
+// alone would be a kernel that walks K in one block. It is a chain of trips to memory: a warp's first ROUTER_EARLY pieces of a
+// matrix at rest are asked for before the kernel ahead has finished, the others that many at a time (a trip per piece was
 // most of the kernel: 8 rows, K = 1,024, 18 outputs: 10.5 -> 6.1 us).
 constexpr int ROUTER_THREADS = 512;
 constexpr int ROUTER_EARLY = 8;
 template <typename T>
 __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(const T* __restrict__ h, const T* __restrict__ w, const float* __restrict__ correction,
                                                                     int* __restrict__ ids, float* __restrict__ weights, int K, int total, int top, int scoring,
-                                                                    const float* __restrict__ bias, int extra, float* __restrict__ gates) {
+                                                                    const float* __restrict__ bias, int extra, float* __restrict__ gates, int at_rest) {
     extern __shared__ __align__(16) float router_smem[];   // [K] the row, then [total + extra] the logits
     constexpr int VN = Vec16<T>::N;
     float* row = router_smem;
@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(const T* __r
             if (i0 + i < pieces && k < K) early[i] = *reinterpret_cast<const uint4*>(w + (size_t)e * K + k);
         }
     };
+    pdl_wait_unless(at_rest);
     if (vec) ask(0);
     pdl_wait();
     const T* src = h + (size_t)n * K;
@@ -457,9 +458,9 @@ LLMIE_API int llmie_moe_route(const float* logits, const float* correction, int*
 }
 
 // ids, weights [N, top] from the rows h [N, K] and the router's matrix w [total + extra, K] of the same type (float or bfloat16): the product in
-// 32-bit and the choice, one launch. The row and the logits must fit the shared memory (K + total floats: up to about 50,000).
+// 32-bit and the choice, one launch. at_rest: w may be read before the kernels ahead have finished. The row and the logits must fit the shared memory (K + total floats: up to about 50,000).
 LLMIE_API int llmie_moe_router(const void* h, const void* w, const float* correction, int* ids, float* weights, int N, int K, int total, int top,
-                               int scoring, const float* bias, int extra, float* gates, int dtype, cudaStream_t s) {
+                               int scoring, const float* bias, int extra, float* gates, int at_rest, int dtype, cudaStream_t s) {
     if (N <= 0) return 0;
     if (K <= 0 || total <= 0 || total > 32 * ROUTE_MAX_PER_LANE || top <= 0 || top > total || extra < 0 || (extra && !gates)) return LLMIE_ERR_BAD_ARGUMENT;
     const size_t smem = ((size_t)((K + 3) & ~3) + total + extra) * sizeof(float);
@@ -472,7 +473,7 @@ LLMIE_API int llmie_moe_router(const void* h, const void* w, const float* correc
             allowed_f = 200 * 1024;
         }
         return launch_kernel(moe_router_kernel<float>, dim3(N), dim3(ROUTER_THREADS), smem, s, (const float*)h, (const float*)w, correction, ids, weights, K,
-                             total, top, scoring, bias, extra, gates);
+                             total, top, scoring, bias, extra, gates, at_rest);
     }
     if (smem > allowed_b) {
         cudaError_t e = cudaFuncSetAttribute(moe_router_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -480,7 +481,7 @@ LLMIE_API int llmie_moe_router(const void* h, const void* w, const float* correc
         allowed_b = 200 * 1024;
     }
     return launch_kernel(moe_router_kernel<bf16>, dim3(N), dim3(ROUTER_THREADS), smem, s, (const bf16*)h, (const bf16*)w, correction, ids, weights, K, total,
-                         top, scoring, bias, extra, gates);
+                         top, scoring, bias, extra, gates, at_rest);
 }
 
 // Rows per tile of the grouped product on the CUDA cores for rows of K numbers: as many as fit the shared memory, at most MOE_TM;

@@ -666,8 +666,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
     T pre_b[BPT], pre_c[BPT], pre_x[XPT], pre_dt[XPT], pre_z[XPT];   // (as they are stored: see above)
     // (a thread stages the same channel of the block in all its pieces: COLS divides the block)
     const int stage_c = blockIdx.x * COLS + threadIdx.x % COLS;
-    const float bias = stage_c < C ? dt_bias[stage_c] : 0.f;
     pdl_wait();
+    const float bias = stage_c < C ? dt_bias[stage_c] : 0.f;
     const int s0 = seq_starts[r], s1 = seq_starts[r + 1];
     float* st = state + ((size_t)seq_slots[r] * C + (live ? col : 0)) * NS;
     float S[DPL];

@@ -14,6 +14,7 @@ there, and hands ``step`` a list of ``StepEntry``.
 """
 from __future__ import annotations
 
+from contextlib import nullcontext
 from dataclasses import dataclass, field
 from typing import Dict, Hashable, List, Optional, Sequence
 
@@ -388,7 +389,8 @@ class ModelRunner:
         """The model on the step's batch. If anything raises in the middle, the kernels object is told to drop what the
         unfinished step left with it (``abandon_step``), so that the next step, of whatever request or runner, starts clean."""
         try:
-            return self._forward(ctx, logit_rows)
+            with getattr(self.K, "at_rest", None) or nullcontext():   # (every matrix of a step is a loaded weight)
+                return self._forward(ctx, logit_rows)
         except BaseException:
             abandon = getattr(self.K, "abandon_step", None)
             if abandon is not None:
