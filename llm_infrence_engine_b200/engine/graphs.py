@@ -10,13 +10,17 @@ rows carry token 0 at position 0, point at a table row of null pages and write t
 into the null page, which nobody reads.
 
 A graph fixes the launch shapes, so the number of key slices per token is planned for ``max_len``;
-the kernel cuts each token's own keys into that many slices on the device, whatever its length.
+the kernel cuts each token's own keys into that many slices on the device, whatever its length. (A launch of nearly a
+block per multiprocessor deals its blocks out by the lengths of all the step's tokens instead: how a token's keys are cut,
+and with it the rounding of its bfloat16 result, then follows from its neighbours too. ``balance_decode = False`` on the
+kernels object leaves every token whole there.)
 
 Steps that bring prompt portions are launched kernel by kernel from Python, a few hundred launches that take the host
-longer than the device needs to run them. Their shape, the tuple of (tokens, wanted rows) per request, often comes
-again: a prompt cut under the token budget gives step after step of exactly the budget. So a shape that is seen a
-third time is captured too (a handful are kept, the least recently used goes), and from then on such a step is one
-launch.
+longer than the device needs to run them. Their shape, the tuple of (tokens, wanted rows) per request, in order, may come
+again: a long prompt cut under the token budget gives step after step of exactly the budget, alone or beside steady
+conversations. So a shape that is seen a third time is captured too (a handful are kept, the least recently used goes), and
+from then on such a step is one launch. A shape that comes once or twice, which is what prompts of any length beside
+conversations that come and go bring, costs what it always did.
 """
 from __future__ import annotations
 
@@ -59,9 +63,19 @@ class DecodeGraphs:
         self.buckets = bucket_sizes(runner.max_seqs)
         self.captured: Dict[int, _Captured] = {}
         self.shapes: "OrderedDict[tuple, _Captured]" = OrderedDict()  # captured prompt-portion steps, least recently used first
-        self.seen: Dict[tuple, int] = {}
+        # how often a shape came, the one that has not come for longest first; steps of many requests hardly ever come again, and are counted
+        # apart so that they push out no others
+        self.seen: "OrderedDict[tuple, int]" = OrderedDict()
+        self.seen_busy: "OrderedDict[tuple, int]" = OrderedDict()
+        self.max_seen = 256
+        self.busy_entries = 9    # from so many requests on
         self.max_shapes = 6
-        self.capture_after = 3   # a capture costs about a hundred eager steps: only shapes that keep coming are worth it
+        # A capture costs 10 to 20 ms in a process whose graph pool is warm (the first ones, that grow it, up to 170), three to five launches of
+        # the step kernel by kernel, and a replay saves 1.2 to 2.5 ms: only shapes that keep coming are worth it. Measured with 0.5B weights: five
+        # prompts of 9,000 to 14,000 tokens beside 32 conversations, budget 512: 2 captures, 114 replays, 0.92 -> 0.73 s, longest pause
+        # 9 -> 40 ms; budget 2,048: one capture, 24 replays, 0.60 s both; 64 prompts of any lengths at once, or arriving one by one: no shape
+        # comes three times, 0.65 and 1.07 s both.
+        self.capture_after = 3
         self.max_shape_tokens = 8192
         self.max_shape_entries = 64   # (decoded tokens beside a prompt portion: a busy server's step)
         self.pool = None
@@ -82,19 +96,23 @@ class DecodeGraphs:
             return None
         return tuple((len(e.tokens), len(e.want)) for e in entries)
 
+    def _came(self, key: tuple) -> int:
+        """Counts one more coming of a shape; how often it came, as far as that is remembered."""
+        seen = self.seen if len(key) < self.busy_entries else self.seen_busy
+        seen[key] = times = seen.pop(key, 0) + 1
+        if len(seen) > self.max_seen:
+            seen.popitem(last=False)
+        return times
+
     def run_shape(self, entries: Sequence[StepEntry], previous_tokens: Optional[torch.Tensor] = None):
-        """Replays (capturing first, if this is the second time) the graph of this step's shape; returns ``(handled, logits)``."""
+        """Replays (capturing first, if it has now come ``capture_after`` times) the graph of this step's shape; returns ``(handled, logits)``."""
         key = self.shape_key(entries)
         if key is None:
             return False, None
         r = self.runner
         cap = self.shapes.get(key)
-        if cap is None:
-            self.seen[key] = self.seen.get(key, 0) + 1
-            if self.seen[key] < self.capture_after:
-                if len(self.seen) > 256:
-                    self.seen.clear()
-                return False, None
+        if cap is None and self._came(key) < self.capture_after:
+            return False, None
         packed, N, R, M, changed, starts, lens, ctxs, slots = r._build(entries)
         static_len = step_layout(N, R, M, len(r.cache.groups))["end"][0]
         if cap is None:
@@ -112,7 +130,7 @@ class DecodeGraphs:
             self.shapes[key] = cap
             while len(self.shapes) > self.max_shapes:
                 gone, _ = self.shapes.popitem(last=False)
-                self.seen.pop(gone, None)   # to be captured again it has to keep coming again
+                (self.seen if len(gone) < self.busy_entries else self.seen_busy).pop(gone, None)   # to be captured again it has to keep coming again
         else:
             self.shapes.move_to_end(key)
             full = r._upload(packed)

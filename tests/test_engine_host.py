@@ -168,3 +168,40 @@ def test_a_step_that_raises_loses_nothing(folders):
     for i in (0, 2):
         assert reqs[i].output_ids == plain_generate(cfg, w, prompts[i], 10) and reqs[i].finish_reason == "length"
     assert all(pool.num_free == pool.capacity for pool in eng.cache.pools) and eng.cache.num_free_slots() == 3
+
+
+def test_shapes_of_steps_are_counted_within_bounds():
+    """Steps of many requests, which hardly ever repeat, take no count from the shapes that do; the counts are bounded, and a shape whose
+    graph was dropped has to come as often again."""
+    from types import SimpleNamespace
+
+    from llm_infrence_engine_b200.engine.graphs import DecodeGraphs
+
+    class Capture(Exception):
+        pass
+
+    def build(entries):
+        raise Capture
+
+    g = DecodeGraphs(SimpleNamespace(device=torch.device("cpu"), max_seqs=64, _build=build))
+    g.usable = True
+
+    def step(*portions):
+        entries = [SimpleNamespace(tokens=[0] * n, want=(0,)) for n in portions]
+        try:
+            handled, _ = g.run_shape(entries)
+        except Capture:
+            return "captured"
+        assert not handled
+        return "eager"
+
+    assert step(512) == step(512) == "eager"
+    for i in range(600):                                   # a busy server's steps, every one its own
+        assert step(*([1] * 20 + [100 + i])) == "eager"
+    assert step(512) == "captured"                         # the third time
+    assert step(*([1] * 20 + [700 - 1])) == "eager" and step(*([1] * 20 + [700 - 1])) == "captured"   # (it came once above)
+    for i in range(600):
+        step(1000 + i)
+    assert len(g.seen) <= 256 and len(g.seen_busy) <= 256
+    assert step(512) == "eager"                            # forgotten: 600 others came since
+    assert step(*([1] * 65 + [9])) == step(*([1] * 65 + [9])) == step(*([1] * 65 + [9])) == "eager"   # too many requests to capture
