@@ -89,15 +89,18 @@ __device__ __forceinline__ void route_token_as(const float* __restrict__ row, co
     for (int k = lane; k < top; k += 32) weights[(size_t)n * top + k] *= inv;
 }
 // (a lane's share of the outputs as a compile-time number: with room for 512 outputs, 16 of them spend sixteen times the instructions)
+static inline __host__ __device__ int route_per_lane(int total) { return total <= 32 ? 1 : (total <= 128 ? 4 : ROUTE_MAX_PER_LANE); }
 __device__ __forceinline__ void route_token(const float* __restrict__ row, const float* __restrict__ correction, int* __restrict__ ids,
                                             float* __restrict__ weights, int n, int total, int top, int lane, int scoring,
                                             const float* __restrict__ bias) {
-    if (total <= 32) route_token_as<1>(row, correction, ids, weights, n, total, top, lane, scoring, bias);
-    else if (total <= 128) route_token_as<4>(row, correction, ids, weights, n, total, top, lane, scoring, bias);
+    const int per_lane = route_per_lane(total);
+    if (per_lane == 1) route_token_as<1>(row, correction, ids, weights, n, total, top, lane, scoring, bias);
+    else if (per_lane == 4) route_token_as<4>(row, correction, ids, weights, n, total, top, lane, scoring, bias);
     else route_token_as<ROUTE_MAX_PER_LANE>(row, correction, ids, weights, n, total, top, lane, scoring, bias);
 }
 
 // Rows of `total + extra` logits; the extra ones are gates of their own: gates[n][j] = sigmoid(logit).
+template <int PER_LANE>
 __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict__ logits, const float* __restrict__ correction,
                                                         int* __restrict__ ids, float* __restrict__ weights, int N, int total, int top, int scoring,
                                                         const float* __restrict__ bias, int extra, float* __restrict__ gates) {
@@ -108,18 +111,19 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
     const float* row = logits + (size_t)n * (total + extra);
     const int lane = threadIdx.x & 31;
     for (int j = lane; j < extra; j += 32) gates[(size_t)n * extra + j] = 1.0f / (1.0f + expf(-row[total + j]));
-    route_token(row, correction, ids, weights, n, total, top, lane, scoring, bias);
+    route_token_as<PER_LANE>(row, correction, ids, weights, n, total, top, lane, scoring, bias);
 }
 
 // The router's product and its choice in one kernel, a block per token: the token's row lies in shared memory as floats, the warps
 // share the router's outputs (a warp's lanes walk an output's weight row in 16-byte pieces; the sum runs over K in one order whatever
 // the step holds), and the first warp chooses from the logits in shared memory. For the few rows of a decode step, where the product
-// alone would be a kernel that walks K in one block. It is a chain of trips to memory: a warp's first ROUTER_EARLY pieces of a
-// matrix at rest are asked for before the kernel ahead has finished, the others that many at a time (a trip per piece was
-// most of the kernel: 8 rows, K = 1,024, 18 outputs: 10.5 -> 6.1 us).
+// alone would be a kernel that walks K in one block. EARLY: no warp has more than ROUTER_EARLY pieces of the matrix, and (at rest) they are
+// all asked for before the kernel ahead has finished. More pieces that many at a time cost more in counting than they save (64 outputs of 1,024
+// in float32: output by output 7.0 us, in four rounds of pieces 9.6), and with more blocks than multiprocessors eight warps each do better than
+// sixteen. (8 rows, K = 1,024, 18 outputs, float32: 10.5 us with eight warps and the choice's room for 512 outputs, 4.1 now.)
 constexpr int ROUTER_THREADS = 512;
 constexpr int ROUTER_EARLY = 8;
-template <typename T>
+template <typename T, bool EARLY>
 __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(const T* __restrict__ h, const T* __restrict__ w, const float* __restrict__ correction,
                                                                     int* __restrict__ ids, float* __restrict__ weights, int K, int total, int top, int scoring,
                                                                     const float* __restrict__ bias, int extra, float* __restrict__ gates, int at_rest) {
@@ -130,60 +134,69 @@ __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(const T* __r
     pdl_trigger();
     const int n = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool vec = (K % VN) == 0 && ((uintptr_t)h & 15) == 0 && ((uintptr_t)w & 15) == 0;
-    // a warp's pieces of the matrix: outputs warp, warp + ROUTER_THREADS / 32, ..., each in steps of 32 * VN entries
-    const int steps = (K + 32 * VN - 1) / (32 * VN), outputs = total + extra;
-    const int pieces = warp < outputs ? ((outputs - 1 - warp) / (ROUTER_THREADS / 32) + 1) * steps : 0;
+    // a warp's pieces of the matrix: outputs warp, warp + warps, ..., each in steps of 32 * VN entries
+    const int warps = blockDim.x >> 5, steps = (K + 32 * VN - 1) / (32 * VN), outputs = total + extra;
     uint4 early[ROUTER_EARLY];
-    auto ask = [&](int i0) {
+    if constexpr (EARLY) {
+        pdl_wait_unless(at_rest);
+        int e = warp, step = 0;   // (counted on: a division per piece costs more than its multiply-adds)
 #pragma unroll
         for (int i = 0; i < ROUTER_EARLY; ++i) {
-            const int e = warp + (i0 + i) / steps * (ROUTER_THREADS / 32), k = (i0 + i) % steps * 32 * VN + lane * VN;
+            const int k = (step * 32 + lane) * VN;
             early[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (i0 + i < pieces && k < K) early[i] = *reinterpret_cast<const uint4*>(w + (size_t)e * K + k);
+            if (e < outputs && k < K) early[i] = *reinterpret_cast<const uint4*>(w + (size_t)e * K + k);
+            if (++step == steps) { step = 0; e += warps; }
         }
-    };
-    pdl_wait_unless(at_rest);
-    if (vec) ask(0);
+    }
     pdl_wait();
     const T* src = h + (size_t)n * K;
     if (vec) {
-        for (int k = threadIdx.x * VN; k < K; k += ROUTER_THREADS * VN) {
+        for (int k = threadIdx.x * VN; k < K; k += blockDim.x * VN) {
             float v[VN];
             Vec16<T>::load(src + k, v);
 #pragma unroll
             for (int i = 0; i < VN; ++i) row[k + i] = v[i];
         }
     } else {
-        for (int k = threadIdx.x; k < K; k += ROUTER_THREADS) row[k] = to_f32(src[k]);
+        for (int k = threadIdx.x; k < K; k += blockDim.x) row[k] = to_f32(src[k]);
     }
     __syncthreads();
-    if (vec) {
+    if constexpr (EARLY) {
         float acc = 0.f;
-        for (int i0 = 0; i0 < pieces; i0 += ROUTER_EARLY) {
-            if (i0 > 0) ask(i0);
+        int e = warp, step = 0;
 #pragma unroll
-            for (int i = 0; i < ROUTER_EARLY; ++i) {
-                if (i0 + i < pieces) {
-                    const int step = (i0 + i) % steps, k = step * 32 * VN + lane * VN;
-                    if (k < K) {
-                        float v[VN];
-                        Vec16<T>::load(reinterpret_cast<const T*>(&early[i]), v);
+        for (int i = 0; i < ROUTER_EARLY; ++i) {
+            if (e < outputs) {
+                const int k = (step * 32 + lane) * VN;
+                if (k < K) {
+                    float v[VN];
+                    Vec16<T>::load(reinterpret_cast<const T*>(&early[i]), v);
 #pragma unroll
-                        for (int c = 0; c < VN; ++c) acc = fmaf(row[k + c], v[c], acc);
-                    }
-                    if (step == steps - 1) {
-                        acc = warp_sum(acc);
-                        if (lane == 0) logits[warp + (i0 + i) / steps * (ROUTER_THREADS / 32)] = acc;
-                        acc = 0.f;
-                    }
+                    for (int c = 0; c < VN; ++c) acc = fmaf(row[k + c], v[c], acc);
+                }
+                if (++step == steps) {
+                    acc = warp_sum(acc);
+                    if (lane == 0) logits[e] = acc;
+                    acc = 0.f;
+                    step = 0;
+                    e += warps;
                 }
             }
         }
     } else {
-        for (int e = warp; e < outputs; e += ROUTER_THREADS / 32) {
+        for (int e = warp; e < outputs; e += warps) {
             const T* we = w + (size_t)e * K;
             float acc = 0.f;
-            for (int k = lane; k < K; k += 32) acc = fmaf(row[k], to_f32(we[k]), acc);
+            if (vec) {
+                for (int k = lane * VN; k < K; k += 32 * VN) {
+                    float v[VN];
+                    Vec16<T>::load(we + k, v);
+#pragma unroll
+                    for (int i = 0; i < VN; ++i) acc = fmaf(row[k + i], v[i], acc);
+                }
+            } else {
+                for (int k = lane; k < K; k += 32) acc = fmaf(row[k], to_f32(we[k]), acc);
+            }
             acc = warp_sum(acc);
             if (lane == 0) logits[e] = acc;
         }
@@ -453,8 +466,34 @@ LLMIE_API int llmie_moe_route(const float* logits, const float* correction, int*
                               const float* bias, int extra, float* gates, cudaStream_t s) {
     if (N <= 0) return 0;
     if (total <= 0 || total > 32 * ROUTE_MAX_PER_LANE || top <= 0 || top > total || extra < 0 || (extra && !gates)) return LLMIE_ERR_BAD_ARGUMENT;
-    return launch_kernel(moe_route_kernel, dim3((N + 3) / 4), dim3(128), 0, s, logits, correction, ids, weights, N, total, top, scoring, bias, extra,
+    const int per_lane = route_per_lane(total);
+    auto kernel = per_lane == 1 ? moe_route_kernel<1> : (per_lane == 4 ? moe_route_kernel<4> : moe_route_kernel<ROUTE_MAX_PER_LANE>);
+    return launch_kernel(kernel, dim3((N + 3) / 4), dim3(128), 0, s, logits, correction, ids, weights, N, total, top, scoring, bias, extra,
                          gates);
+}
+
+template <typename T, bool EARLY>
+static int launch_router_as(const void* h, const void* w, const float* correction, int* ids, float* weights, int N, int K, int total, int top, int scoring,
+                            const float* bias, int extra, float* gates, int at_rest, size_t smem, int threads, cudaStream_t s) {
+    if (smem > 48 * 1024) {
+        static OncePerDevice granted;
+        if (const int rc = grant_shared(granted, moe_router_kernel<T, EARLY>, 200 * 1024)) return rc;
+    }
+    return launch_kernel(moe_router_kernel<T, EARLY>, dim3(N), dim3(threads), smem, s, (const T*)h, (const T*)w, correction, ids, weights, K, total, top, scoring,
+                         bias, extra, gates, at_rest);
+}
+
+template <typename T>
+static int launch_router(const void* h, const void* w, const float* correction, int* ids, float* weights, int N, int K, int total, int top, int scoring,
+                         const float* bias, int extra, float* gates, int at_rest, size_t smem, cudaStream_t s) {
+    constexpr int VN = Vec16<T>::N, WARPS = ROUTER_THREADS / 32;
+    const bool vec = K % VN == 0 && ((uintptr_t)h & 15) == 0 && ((uintptr_t)w & 15) == 0;
+    const int pieces = (total + extra + WARPS - 1) / WARPS * ((K + 32 * VN - 1) / (32 * VN));
+    const bool few = N <= 148;
+#define LLMIE_ROUTER_ARGS(THREADS) h, w, correction, ids, weights, N, K, total, top, scoring, bias, extra, gates, at_rest, smem, THREADS, s
+    if (vec && few && pieces <= ROUTER_EARLY) return launch_router_as<T, true>(LLMIE_ROUTER_ARGS(ROUTER_THREADS));
+    return launch_router_as<T, false>(LLMIE_ROUTER_ARGS(few ? ROUTER_THREADS : 256));
+#undef LLMIE_ROUTER_ARGS
 }
 
 // ids, weights [N, top] from the rows h [N, K] and the router's matrix w [total + extra, K] of the same type (float or bfloat16): the product in
@@ -465,23 +504,8 @@ LLMIE_API int llmie_moe_router(const void* h, const void* w, const float* correc
     if (K <= 0 || total <= 0 || total > 32 * ROUTE_MAX_PER_LANE || top <= 0 || top > total || extra < 0 || (extra && !gates)) return LLMIE_ERR_BAD_ARGUMENT;
     const size_t smem = ((size_t)((K + 3) & ~3) + total + extra) * sizeof(float);
     if (smem > 200 * 1024) return LLMIE_ERR_BAD_ARGUMENT;
-    static size_t allowed_f = 48 * 1024, allowed_b = 48 * 1024;
-    if (dtype == DT_F32) {
-        if (smem > allowed_f) {
-            cudaError_t e = cudaFuncSetAttribute(moe_router_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            if (e != cudaSuccess) return (int)e;
-            allowed_f = 200 * 1024;
-        }
-        return launch_kernel(moe_router_kernel<float>, dim3(N), dim3(ROUTER_THREADS), smem, s, (const float*)h, (const float*)w, correction, ids, weights, K,
-                             total, top, scoring, bias, extra, gates, at_rest);
-    }
-    if (smem > allowed_b) {
-        cudaError_t e = cudaFuncSetAttribute(moe_router_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e != cudaSuccess) return (int)e;
-        allowed_b = 200 * 1024;
-    }
-    return launch_kernel(moe_router_kernel<bf16>, dim3(N), dim3(ROUTER_THREADS), smem, s, (const bf16*)h, (const bf16*)w, correction, ids, weights, K, total,
-                         top, scoring, bias, extra, gates, at_rest);
+    if (dtype == DT_F32) return launch_router<float>(h, w, correction, ids, weights, N, K, total, top, scoring, bias, extra, gates, at_rest, smem, s);
+    return launch_router<bf16>(h, w, correction, ids, weights, N, K, total, top, scoring, bias, extra, gates, at_rest, smem, s);
 }
 
 // Rows per tile of the grouped product on the CUDA cores for rows of K numbers: as many as fit the shared memory, at most MOE_TM;

@@ -661,3 +661,23 @@ def test_transient_products_are_consumed_and_cleared(K):
     assert K.linear(a, wd.cuda(), add_to=r) is None
     close(r, res.double() + a.double().cpu() @ wd.double().T, 2e-5)
     K.check_device_errors()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("N,W,E,top,gates", [(1, 512, 8, 2, 0), (3, 1024, 16, 4, 2), (64, 1024, 64, 6, 0), (5, 2048, 128, 8, 1), (148, 896, 300, 2, 0), (149, 512, 18, 2, 0), (2, 300, 17, 3, 0)])
+def test_router_forms_agree(K, monkeypatch, dtype, N, W, E, top, gates):
+    """All pieces asked for at once or output by output, sixteen warps or eight (more rows than multiprocessors): the same sums in the same order."""
+    h, w = torch.randn(N, W, generator=torch.Generator().manual_seed(1)).to(dtype), torch.randn(E + gates, W, generator=torch.Generator().manual_seed(2)).to(dtype)
+    monkeypatch.setattr(K, "tc_max_rows", 1 << 20)
+    hd, wd = h.cuda(), w.cuda()
+    apart = torch.empty(w.numel() + 1, dtype=dtype, device="cuda")[1:].view_as(wd)   # not on a 16-byte boundary
+    apart.copy_(wd)
+    many = K.moe_router(hd.repeat(150, 1), wd, None, top, gates=gates)
+    outs = [K.moe_router(hd, wd, None, top, gates=gates), [o[:N] for o in many]]
+    with K.at_rest:
+        outs.append(K.moe_router(hd, wd, None, top, gates=gates))
+    for o in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(outs[0], o))
+    want = REF.moe_router(h, w, None, top, gates=gates)
+    for o in (outs[0], K.moe_router(hd, apart, None, top, gates=gates)):
+        close(o[1].sort().values, want[1].sort().values, 2e-5)   # (logits of a scale of 45: 32-bit sums of 2,048 products in another order)
