@@ -284,9 +284,10 @@ __global__ void __launch_bounds__(256, 2) moe_rows_kernel(const T* __restrict__ 
 #pragma unroll
     for (int c = 0; c < CPW; ++c) wrow[c] = we + (size_t)min(j0 + c, F - 1) * K;   // (an output past the end repeats the last: not stored)
     const size_t up = (size_t)F * K;   // from an output's gate row to its up row (read only when GATED)
-    // a step's 16-byte pieces of all the warp's weight rows. GATED: the next step's are asked for before this one's are used, the first
-    // step's before the tile's rows are fetched (2 rows, 16 experts of 512 x 1,024: 8.5 -> 7.8 us, 8 rows: equal; without a gate, with half the pieces, the
-    // registers cost more than it gains: 7.0 -> 7.6 at 8 rows)
+    // a step's 16-byte pieces of all the warp's weight rows. GATED in bfloat16: the next step's are asked for before this one's are used, the
+    // first step's before the tile's rows are fetched (2 rows, 16 experts of 512 x 1,024: 8.5 -> 7.8 us, 8 rows: equal; without a gate, with half the
+    // pieces, the registers cost more than it gains: 7.0 -> 7.6 at 8 rows; so they do in float32: both products 24.2 -> 25.2 at 16 rows of 512, 8 experts)
+    constexpr bool AHEAD = GATED && sizeof(T) == 2;
     struct Pieces { uint4 g[CPW], u[GATED ? CPW : 1]; };
     auto ask = [&](int k, Pieces& p) {
 #pragma unroll
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(256, 2) moe_rows_kernel(const T* __restrict__ 
         }
     };
     Pieces now;
-    if (GATED && vec && lane * VN < K) ask(lane * VN, now);
+    if (AHEAD && vec && lane * VN < K) ask(lane * VN, now);
     for (int r = 0; r < count; ++r) {
         const int p = p0 + r;
         const T* src = x + (size_t)(row_map ? row_map[p] / row_div : p) * K;
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(256, 2) moe_rows_kernel(const T* __restrict__ 
     if (vec) {
         for (int k = lane * VN; k < K; k += 32 * VN) {
             Pieces next;
-            if constexpr (!GATED) ask(k, now);
+            if constexpr (!AHEAD) ask(k, now);
             else if (k + 32 * VN < K) ask(k + 32 * VN, next);
 #pragma unroll
             for (int i = 0; i < VN; i += 4) {   // (four entries of every piece at a time as floats: all of them would not fit the registers)
@@ -346,7 +347,7 @@ __global__ void __launch_bounds__(256, 2) moe_rows_kernel(const T* __restrict__ 
                     }
                 }
             }
-            if constexpr (GATED) now = next;
+            if constexpr (AHEAD) now = next;
         }
     } else {
         for (int k = lane; k < K; k += 32) {
