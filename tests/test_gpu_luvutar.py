@@ -312,3 +312,18 @@ def test_random_weights_and_the_command_line(tmp_path):
     for _ in range(6):
         seq.append(int(plain_logits(cfg, tensors, seq)[-1].argmax()))
     assert tokens == seq[5:]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("N,H,K_,J", [(1, 14, 64, 256), (9, 14, 256, 64), (5, 3, 30, 40), (8, 2, 250, 40), (3, 2, 90, 31), (2, 1, 1500, 64), (600, 2, 512, 128)])
+def test_per_head_products(K, dtype, N, H, K_, J):
+    """Inner sizes of whole groups of 16 and not, columns copied to shared memory and not (columns in no whole 16-byte pieces, a matrix too tall,
+    a launch too long for it); a matrix at rest and one just made: the same bits."""
+    ref, T = TorchKernels(), TD[dtype]
+    x, w = rnd(N, H * K_, seed=1).to(T), rnd(H, K_, J, seed=2, scale=K_ ** -0.5).to(T)
+    want = ref.latent_expand(x, w, None, 0, H, K_, J)
+    xd, wd = x.cuda(), w.cuda()
+    got = K.latent_expand(xd, wd, None, 0, H, K_, J)
+    close(got, want, dtype, "latent_expand", scale=2.0 if dtype == "float32" else None)   # (32-bit sums of up to 1,500 products in another order: twice what the short ones are given)
+    with K.at_rest:
+        assert torch.equal(K.latent_expand(xd, wd, None, 0, H, K_, J), got)
