@@ -522,11 +522,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
             pre_x[n] = (j < count * COLS && c < DV) ? xbc[(size_t)(base + t) * x_stride + x_col + h * DV + c] : from_f32<T>(0.f);
         }
     };
-    auto store_tile = [&](int buf) {
+    auto store_tile = [&](int buf, int count) {   // (tokens that are not there cost nothing: decoded tokens come one to a tile)
 #pragma unroll
         for (int n = 0; n < QPT; ++n) {
             const int i = threadIdx.x + n * SCAN_THREADS;
-            if (i < SCAN_TILE * NMAX / 4) {
+            if (i < count * (NMAX / 4)) {
                 float b4[4], c4[4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {   // (silu(0) = 0: the padding stays)
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
                 store4(c_s + buf * SCAN_TILE * NMAX + 4 * i, c4);
             }
         }
-        if (!FIXED && threadIdx.x < SCAN_TILE) {
+        if (!FIXED && threadIdx.x < count) {
             const float dt = softplus_f(to_f32(pre_dt) + bias);
             dt_s[buf * SCAN_TILE + threadIdx.x] = dt;
             a_s[buf * SCAN_TILE + threadIdx.x] = expf(-rate * dt);
@@ -546,14 +546,14 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
 #pragma unroll
         for (int n = 0; n < XPT; ++n) {
             const int j = SCAN_THREADS - 1 - threadIdx.x + n * SCAN_THREADS;
-            if (j < SCAN_TILE * COLS) x_s[buf * SCAN_TILE * COLS + j] = FIXED ? silu_f(to_f32(pre_x[n])) : to_f32(pre_x[n]);
+            if (j < count * COLS) x_s[buf * SCAN_TILE * COLS + j] = FIXED ? silu_f(to_f32(pre_x[n])) : to_f32(pre_x[n]);
         }
     };
     if (s0 < s1) load_tile(s0);
     int buf = 0;
     for (int base = s0; base < s1; base += SCAN_TILE, buf ^= 1) {
         const int count = min(SCAN_TILE, s1 - base);
-        store_tile(buf);                       // (this stage's last readers passed the barrier of the tile between)
+        store_tile(buf, count);                       // (this stage's last readers passed the barrier of the tile between)
         __syncthreads();                       // this tile is in shared memory
         if (base + SCAN_TILE < s1) load_tile(base + SCAN_TILE);
         const float* bb = b_s + buf * SCAN_TILE * NMAX + 4 * part;
@@ -635,20 +635,21 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
 // The layout is the one above with a channel in the place of a column: PARTS lanes share a channel, each with its entries of S and
 // of A in registers; a block owns SCAN_THREADS / PARTS channels; tiles of SCAN_TILE tokens are loaded into registers a tile ahead.
 // 2,048 channels, 16 states, eight prompts of 64 to 511 tokens (bfloat16), with step sizes waited for as they were loaded and a reduction per token before: 214 -> 105 us.
-template <typename T, int NMAX>
+template <typename T, int NMAX, int PARTS, int TILE>
 __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* __restrict__ x, int x_stride, const T* __restrict__ dt_raw, int dt_stride,
                                                                       const T* __restrict__ bc, int bc_stride, int b_col, int c_col,
                                                                       const T* __restrict__ z, int z_stride, const float* __restrict__ A_log,
                                                                       const float* __restrict__ dt_bias, const float* __restrict__ Dskip,
                                                                       float* __restrict__ state, const int* __restrict__ seq_starts,
                                                                       const int* __restrict__ seq_slots, T* __restrict__ out, int C, int NS) {
-    constexpr int PARTS = delta_parts(NMAX), DPL = NMAX / PARTS, COLS = SCAN_THREADS / PARTS;
+    constexpr int DPL = NMAX / PARTS, COLS = SCAN_THREADS / PARTS;
+    constexpr bool WHOLE = TILE % PARTS == 0;   // a full tile's sums are added up PARTS at a time
     extern __shared__ __align__(16) float scan_smem[];
-    float* b_s = scan_smem;                              // [2][SCAN_TILE][NMAX]
-    float* c_s = b_s + 2 * SCAN_TILE * NMAX;
-    float* x_s = c_s + 2 * SCAN_TILE * NMAX;             // [2][SCAN_TILE][COLS]
-    float* dt_s = x_s + 2 * SCAN_TILE * COLS;
-    float* z_s = dt_s + 2 * SCAN_TILE * COLS;
+    float* b_s = scan_smem;                              // [2][TILE][NMAX]
+    float* c_s = b_s + 2 * TILE * NMAX;
+    float* x_s = c_s + 2 * TILE * NMAX;             // [2][TILE][COLS]
+    float* dt_s = x_s + 2 * TILE * COLS;
+    float* z_s = dt_s + 2 * TILE * COLS;
     const int part = threadIdx.x % PARTS;
     const int my_col = threadIdx.x / PARTS;
     const int col = blockIdx.x * COLS + my_col;
@@ -661,8 +662,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
 #pragma unroll
     for (int i = 0; i < DPL; ++i) A[i] = -expf(A[i]);
     const float skip = live ? Dskip[col] : 0.f;
-    constexpr int BPT = (SCAN_TILE * NMAX + SCAN_THREADS - 1) / SCAN_THREADS;
-    constexpr int XPT = (SCAN_TILE * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
+    constexpr int BPT = (TILE * NMAX + SCAN_THREADS - 1) / SCAN_THREADS;
+    constexpr int XPT = (TILE * COLS + SCAN_THREADS - 1) / SCAN_THREADS;
     T pre_b[BPT], pre_c[BPT], pre_x[XPT], pre_dt[XPT], pre_z[XPT];   // (as they are stored: see above)
     // (a thread stages the same channel of the block in all its pieces: COLS divides the block)
     const int stage_c = blockIdx.x * COLS + threadIdx.x % COLS;
@@ -673,7 +674,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
     float S[DPL];
     load_column<DPL, PARTS>(S, st, part, NS, live, vec);
     auto load_tile = [&](int base) {
-        const int count = min(SCAN_TILE, s1 - base);
+        const int count = min(TILE, s1 - base);
 #pragma unroll
         for (int n = 0; n < BPT; ++n) {
             const int i = threadIdx.x + n * SCAN_THREADS;
@@ -693,37 +694,37 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
             pre_dt[n] = in ? dt_raw[(size_t)(base + t) * dt_stride + c] : from_f32<T>(0.f);
         }
     };
-    auto store_tile = [&](int buf) {   // step sizes and gates are taken here, a tile behind their loads, which nobody waits for
+    auto store_tile = [&](int buf, int count) {   // step sizes and gates are taken here, a tile behind their loads, which nobody waits for
 #pragma unroll
         for (int n = 0; n < BPT; ++n) {
             const int i = threadIdx.x + n * SCAN_THREADS;
-            if (i < SCAN_TILE * NMAX) {
-                b_s[buf * SCAN_TILE * NMAX + i] = to_f32(pre_b[n]);
-                c_s[buf * SCAN_TILE * NMAX + i] = to_f32(pre_c[n]);
+            if (i < count * NMAX) {
+                b_s[buf * TILE * NMAX + i] = to_f32(pre_b[n]);
+                c_s[buf * TILE * NMAX + i] = to_f32(pre_c[n]);
             }
         }
 #pragma unroll
         for (int n = 0; n < XPT; ++n) {
             const int j = threadIdx.x + n * SCAN_THREADS;
-            if (j < SCAN_TILE * COLS) {
-                x_s[buf * SCAN_TILE * COLS + j] = to_f32(pre_x[n]);
-                dt_s[buf * SCAN_TILE * COLS + j] = softplus_f(to_f32(pre_dt[n]) + bias);
-                z_s[buf * SCAN_TILE * COLS + j] = silu_f(to_f32(pre_z[n]));
+            if (j < count * COLS) {
+                x_s[buf * TILE * COLS + j] = to_f32(pre_x[n]);
+                dt_s[buf * TILE * COLS + j] = softplus_f(to_f32(pre_dt[n]) + bias);
+                z_s[buf * TILE * COLS + j] = silu_f(to_f32(pre_z[n]));
             }
         }
     };
     if (s0 < s1) load_tile(s0);
     int buf = 0;
-    for (int base = s0; base < s1; base += SCAN_TILE, buf ^= 1) {
-        const int count = min(SCAN_TILE, s1 - base);
-        store_tile(buf);                       // (this stage's last readers passed the barrier of the tile between)
+    for (int base = s0; base < s1; base += TILE, buf ^= 1) {
+        const int count = min(TILE, s1 - base);
+        store_tile(buf, count);                       // (this stage's last readers passed the barrier of the tile between)
         __syncthreads();                       // this tile is in shared memory
-        if (base + SCAN_TILE < s1) load_tile(base + SCAN_TILE);
-        const float* bb = b_s + buf * SCAN_TILE * NMAX + 4 * part;
-        const float* cb = c_s + buf * SCAN_TILE * NMAX + 4 * part;
+        if (base + TILE < s1) load_tile(base + TILE);
+        const float* bb = b_s + buf * TILE * NMAX + 4 * part;
+        const float* cb = c_s + buf * TILE * NMAX + 4 * part;
         auto token = [&](int t) {   // returns this lane's share of the channel's sum
-            const float xv = x_s[(buf * SCAN_TILE + t) * COLS + my_col];
-            const float dt = dt_s[(buf * SCAN_TILE + t) * COLS + my_col];
+            const float xv = x_s[(buf * TILE + t) * COLS + my_col];
+            const float dt = dt_s[(buf * TILE + t) * COLS + my_col];
             const float u = dt * xv;
             float y0 = 0.f, y1 = 0.f;
 #pragma unroll
@@ -739,12 +740,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
             return y0 + y1;
         };
         auto put = [&](int t, float y) {
-            const int at = (buf * SCAN_TILE + t) * COLS + my_col;
+            const int at = (buf * TILE + t) * COLS + my_col;
             out[(size_t)(base + t) * C + col] = from_f32<T>(fmaf(skip, x_s[at], y) * z_s[at]);
         };
-        if (count == SCAN_TILE) {
+        if (WHOLE && count == TILE) {
 #pragma unroll
-            for (int t0 = 0; t0 < SCAN_TILE; t0 += PARTS) {
+            for (int t0 = 0; t0 < TILE; t0 += PARTS) {
                 float y[PARTS];
 #pragma unroll
                 for (int t = 0; t < PARTS; ++t) y[t] = token(t0 + t);
@@ -773,6 +774,8 @@ int launch_conv(const T* z, int z_stride, int C, const float* w, const float* bi
 // Several columns to a lane as soon as one each would be more warps than the device has schedulers: the step's columns decide (a lane
 // with more of them makes each token longer, but reads the token's rows once for all).
 static inline bool many_columns(long long columns, int parts) { return columns * parts > 148LL * SCAN_THREADS * 2; }
+// (but not where a block would then be wider than the columns there are: its lanes beyond them idle)
+static inline int padded(int columns, int block) { return (columns + block - 1) / block * block; }
 
 template <typename T, int DM, int CPL, bool SCALAR>
 int launch_delta_scan_one(const T* v, int v_stride, int v_col, const float* qn, const float* kn, const float* kq, const float* decay,
@@ -814,10 +817,15 @@ int launch_ssm_scan_as(const T* xbc, int x_stride, int x_col, int b_col, int c_c
                        const float* dt_bias, const float* Dskip, float* state, const int* seq_starts, const int* seq_slots, float* out, int H,
                        int G, int NS, int DV, int R, bool alone, cudaStream_t s) {
 #define LLMIE_SSM_ARGS xbc, x_stride, x_col, b_col, c_col, dt_raw, dt_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, out, H, G, NS, DV, R, alone, s
-    const bool many = many_columns((long long)R * H * DV, scan_parts(NM));
-    if (!dt_raw)   // no step sizes: the fixed decays of linear attention
-        return many ? launch_ssm_scan_one<T, NM, 4, true>(LLMIE_SSM_ARGS) : launch_ssm_scan_one<T, NM, 2, true>(LLMIE_SSM_ARGS);
-    return many ? launch_ssm_scan_one<T, NM, 4, false>(LLMIE_SSM_ARGS) : launch_ssm_scan_one<T, NM, 2, false>(LLMIE_SSM_ARGS);
+    constexpr int one = SCAN_THREADS / scan_parts(NM);   // a block's columns with one to a lane
+    const bool fixed = !dt_raw;                          // no step sizes: the fixed decays of linear attention
+    if constexpr (NM <= 32) {
+        if (padded(DV, one) < padded(DV, 2 * one) || (long long)R * H * DV * scan_parts(NM) <= 148LL * SCAN_THREADS)   // (or not even a block per multiprocessor)
+            return fixed ? launch_ssm_scan_one<T, NM, 1, true>(LLMIE_SSM_ARGS) : launch_ssm_scan_one<T, NM, 1, false>(LLMIE_SSM_ARGS);
+    }
+    if (many_columns((long long)R * H * DV, scan_parts(NM)) && padded(DV, 4 * one) == padded(DV, 2 * one))
+        return fixed ? launch_ssm_scan_one<T, NM, 4, true>(LLMIE_SSM_ARGS) : launch_ssm_scan_one<T, NM, 4, false>(LLMIE_SSM_ARGS);
+    return fixed ? launch_ssm_scan_one<T, NM, 2, true>(LLMIE_SSM_ARGS) : launch_ssm_scan_one<T, NM, 2, false>(LLMIE_SSM_ARGS);
 #undef LLMIE_SSM_ARGS
 }
 
@@ -846,24 +854,36 @@ int launch_ssm_scan(const T* xbc, int x_stride, int x_col, int b_col, int c_col,
                         seq_slots, out, H, G, NS, DV, R, alone, s)
 }
 
-template <typename T, int NM>
+template <typename T, int NM, int PARTS, int TILE>
 int launch_selective_scan_as(const T* x, int x_stride, const T* dt_raw, int dt_stride, const T* bc, int bc_stride, int b_col, int c_col, const T* z,
                              int z_stride, const float* A_log, const float* dt_bias, const float* Dskip, float* state, const int* seq_starts,
                              const int* seq_slots, T* out, int C, int NS, int R, bool alone, cudaStream_t s) {
-    constexpr int cols = SCAN_THREADS / delta_parts(NM);
+    constexpr int cols = SCAN_THREADS / PARTS;
     const dim3 grid((C + cols - 1) / cols, 1, R);
-    const size_t smem = sizeof(float) * (2 * SCAN_TILE * (2 * NM + 3 * cols));
-    if (smem > 48 * 1024) cudaFuncSetAttribute(selective_scan_kernel<T, NM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_kernel_on(alone, selective_scan_kernel<T, NM>, grid, dim3(SCAN_THREADS), smem, s, x, x_stride, dt_raw, dt_stride, bc, bc_stride,
+    const size_t smem = sizeof(float) * (2 * TILE * (2 * NM + 3 * cols));
+    if (smem > 48 * 1024) cudaFuncSetAttribute(selective_scan_kernel<T, NM, PARTS, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return launch_kernel_on(alone, selective_scan_kernel<T, NM, PARTS, TILE>, grid, dim3(SCAN_THREADS), smem, s, x, x_stride, dt_raw, dt_stride, bc, bc_stride,
                             b_col, c_col, z, z_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, out, C, NS);
 }
 
+constexpr long long SELECTIVE_FEW = 32768;
 template <typename T>
 int launch_selective_scan(const T* x, int x_stride, const T* dt_raw, int dt_stride, const T* bc, int bc_stride, int b_col, int c_col, const T* z,
                           int z_stride, const float* A_log, const float* dt_bias, const float* Dskip, float* state, const int* seq_starts,
-                          const int* seq_slots, T* out, int C, int NS, int R, bool alone, cudaStream_t s) {
-    LLMIE_SCAN_DISPATCH(launch_selective_scan_as, NS, x, x_stride, dt_raw, dt_stride, bc, bc_stride, b_col, c_col, z, z_stride, A_log, dt_bias, Dskip,
-                        state, seq_starts, seq_slots, out, C, NS, R, alone, s)
+                          const int* seq_slots, T* out, int C, int NS, int R, bool alone, bool short_rows, cudaStream_t s) {
+#define LLMIE_SELECTIVE_ARGS x, x_stride, dt_raw, dt_stride, bc, bc_stride, b_col, c_col, z, z_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, out, C, NS, R, alone, s
+    // (decoded tokens come one to a tile: a tile of SCAN_TILE would only take the room that more blocks at once need)
+#define LLMIE_SELECTIVE(NM, PARTS) (short_rows ? launch_selective_scan_as<T, NM, PARTS, 4>(LLMIE_SELECTIVE_ARGS) : launch_selective_scan_as<T, NM, PARTS, SCAN_TILE>(LLMIE_SELECTIVE_ARGS))
+    // An exponential per entry and token is most of the work, so a channel's entries are shared out among more lanes than a head's column would
+    // be, the more the fewer channels there are (the model's sizes alone decide, never the batch: see scan_parts).
+    const bool few = (long long)C * 16 <= SELECTIVE_FEW;
+    if (NS <= 16) return LLMIE_SELECTIVE(16, 4);
+    if (NS <= 32) return LLMIE_SELECTIVE(32, 8);
+    if (NS <= 64) return few ? LLMIE_SELECTIVE(64, 16) : LLMIE_SELECTIVE(64, 8);
+    if (NS <= 128) return few ? LLMIE_SELECTIVE(128, 16) : LLMIE_SELECTIVE(128, 8);
+    return LLMIE_SELECTIVE(256, 16);
+#undef LLMIE_SELECTIVE
+#undef LLMIE_SELECTIVE_ARGS
 }
 
 }  // namespace
@@ -945,7 +965,7 @@ LLMIE_API int llmie_selective_scan(const void* x, int x_stride, const void* dt_r
     const bool alone = max_rows >= SCAN_ALONE_ROWS;
     if (dtype == DT_F32)
         return launch_selective_scan<float>((const float*)x, x_stride, (const float*)dt_raw, dt_stride, (const float*)bc, bc_stride, b_col, c_col,
-                                            (const float*)z, z_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, (float*)out, C, NS, R, alone, s);
+                                            (const float*)z, z_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, (float*)out, C, NS, R, alone, max_rows <= 4, s);
     return launch_selective_scan<bf16>((const bf16*)x, x_stride, (const bf16*)dt_raw, dt_stride, (const bf16*)bc, bc_stride, b_col, c_col,
-                                       (const bf16*)z, z_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, (bf16*)out, C, NS, R, alone, s);
+                                       (const bf16*)z, z_stride, A_log, dt_bias, Dskip, state, seq_starts, seq_slots, (bf16*)out, C, NS, R, alone, max_rows <= 4, s);
 }

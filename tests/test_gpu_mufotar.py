@@ -371,3 +371,25 @@ def test_random_weights_and_the_command_line(tmp_path):
     for t in tokens:
         assert t == int(plain_logits(cfg, tensors, seq)[-1].argmax())
         seq.append(t)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("C,NS", [(40, 17), (2100, 40), (40, 64), (2100, 100), (40, 128), (4, 200)])
+def test_selective_scan_with_few_channels_and_with_many(K, dtype, C, NS):
+    """More lanes share a channel's states where there are few channels: against plain torch, decoded tokens after a portion that ends inside
+    a tile, and the same bits as the whole."""
+    ref, T = TorchKernels(), TD[dtype]
+    N = 21
+    x, dt, bc, z = rnd(N, C, seed=1).to(T), rnd(N, C, seed=2).to(T), rnd(N, 2 * NS, seed=3).to(T), rnd(N, C, seed=4).to(T)
+    A_log, dt_bias, skip = rnd(C, NS, seed=5, scale=0.3), rnd(C, seed=6) - 1, rnd(C, seed=7)
+    outs = {}
+    for how, cuts in (("whole", [(0, N)]), ("cut", [(0, 18), (18, 19), (19, 20), (20, N)])):
+        st, rows = rnd(2, C, NS, seed=8, scale=0.3).cuda(), []
+        for lo, hi in cuts:
+            rows.append(K.selective_scan(x[lo:hi].cuda(), dt[lo:hi].cuda(), bc[lo:hi].cuda(), 0, NS, z[lo:hi].cuda(), 0, A_log.cuda(), dt_bias.cuda(), skip.cuda(), st,
+                                         ragged([hi - lo], [1])[1]))
+        outs[how] = (torch.cat(rows), st)
+    st = rnd(2, C, NS, seed=8, scale=0.3)
+    want = ref.selective_scan(x, dt, bc, 0, NS, z, 0, A_log, dt_bias, skip, st, ragged([N], [1])[0])
+    close(outs["whole"][0], want, dtype, "selective_scan", scale=max(1.0, float(want.float().abs().max())), f32=1e-5)   # (as the state-space scan's)
+    assert all(torch.equal(a, b) for a, b in zip(outs["whole"], outs["cut"]))
