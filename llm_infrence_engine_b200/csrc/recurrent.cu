@@ -58,6 +58,20 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const T* __restrict__ 
         in[j] = 0.f;
         if (j >= skip) in[j] = t >= 0 ? to_f32(z[(size_t)(s0 + t) * z_stride + c]) : st[(size_t)(taps - 1 + t) * C];
     }
+    if (L == 1) {   // a decoded token: nothing to run in batches, and its window moves on by one (6,144 channels, 64 requests: as part of a batch 9.2 us)
+        const float u = to_f32(z[(size_t)s0 * z_stride + c]);
+        float y = b;
+#pragma unroll
+        for (int j = 0; j < H; ++j)
+            if (j >= skip) y = fmaf(w8[j], in[j], y);
+        y = fmaf(w8[H], u, y);
+        if (act == 1) y = silu_f(y);
+        out[(size_t)s0 * out_stride + c] = from_f32<T>(y);
+#pragma unroll
+        for (int j = 0; j < H; ++j)
+            if (j >= skip) st[(size_t)(j - skip) * C] = j + 1 < H ? in[j + 1] : u;
+        return;
+    }
     const int t1 = min(L, t0 + CONV_CHUNK);
     for (int t = t0; t < t1; t += CONV_BATCH) {
 #pragma unroll
