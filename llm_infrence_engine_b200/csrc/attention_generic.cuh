@@ -118,31 +118,7 @@ __global__ void __launch_bounds__(WARPS * 32) paged_attn_kernel(
             for (int i = 0; i < DPL; ++i) acc[g][i] *= corr[g];
         const int count = min(32, end - base);
         int j = max(0, lo - base);
-        // eight rows of values in flight at a time, for the same reason (float32 prompts of 33, 79 and 190 tokens, 14 heads of 64 over 2, a prompt's
-        // and a decoded token's launch: 41 -> 21 us on average); the keys one after the other, as below
-        for (; (j & 7) == 0 && j + 8 <= count; j += 8) {
-            float vv[8][DPL];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const T* vr = v_pool + (size_t)__shfl_sync(0xffffffffu, row, j + k) * d;
-#pragma unroll
-                for (int i = 0; i < DPL; ++i) {
-                    const int dim = lane + 32 * i;
-                    vv[k][i] = dim < d ? to_f32(vr[dim]) : 0.f;
-                }
-            }
-#pragma unroll
-            for (int g = 0; g < GC; ++g) {
-                float pj[8];
-                load4(&ps[warp][g][j], pj);
-                load4(&ps[warp][g][j + 4], pj + 4);
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-#pragma unroll
-                    for (int i = 0; i < DPL; ++i) acc[g][i] = fmaf(pj[k], vv[k][i], acc[g][i]);
-            }
-        }
-        for (; j < count; ++j) {
+        auto one = [&](int j) {
             const int rj = __shfl_sync(0xffffffffu, row, j);
             const T* vr = v_pool + (size_t)rj * d;
             float vv[DPL];
@@ -157,7 +133,36 @@ __global__ void __launch_bounds__(WARPS * 32) paged_attn_kernel(
 #pragma unroll
                 for (int i = 0; i < DPL; ++i) acc[g][i] = fmaf(pj, vv[i], acc[g][i]);
             }
+        };
+        // several rows of values in flight at a time, for the same reason (float32 prompts of 33, 79 and 190 tokens, 14 heads of 64 over 2, a prompt's
+        // and a decoded token's launch: 41 -> 21 us on average); the keys one after the other, as alone. (Heads of more than 128 have a row's worth
+        // of loads each anyway, and four rows of them take the registers that a second block needs: 8 heads of 256, 44 -> 51 us)
+        if constexpr (DPL <= 4) {
+            for (; (j & 7) != 0 && j < count; ++j) one(j);
+            for (; j + 8 <= count; j += 8) {
+                float vv[8][DPL];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const T* vr = v_pool + (size_t)__shfl_sync(0xffffffffu, row, j + k) * d;
+#pragma unroll
+                    for (int i = 0; i < DPL; ++i) {
+                        const int dim = lane + 32 * i;
+                        vv[k][i] = dim < d ? to_f32(vr[dim]) : 0.f;
+                    }
+                }
+#pragma unroll
+                for (int g = 0; g < GC; ++g) {
+                    float pj[8];
+                    load4(&ps[warp][g][j], pj);
+                    load4(&ps[warp][g][j + 4], pj + 4);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+#pragma unroll
+                        for (int i = 0; i < DPL; ++i) acc[g][i] = fmaf(pj[k], vv[k][i], acc[g][i]);
+                }
+            }
         }
+        for (; j < count; ++j) one(j);
         __syncwarp();
     }
 
