@@ -843,3 +843,45 @@ def test_decode_graphs_planned_for_a_long_context(models, tmp_path, which):
     check(torch.stack(got_a), want_a[40:90], "bfloat16", "request a", which)
     check(torch.stack(got_b), want_b[40:90], "bfloat16", "request b", which)
     runner.K.check_device_errors()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_captured_steps_of_a_prompt_portion_beside_many_conversations(models, dtype):
+    """Eleven requests in a step, ten of them decoding: captured when the shape comes again, replayed at other contexts, pages and tokens, and
+    after its graph was dropped for a newer shape's it is launched kernel by kernel again until it has come as often once more."""
+    from llm_infrence_engine_b200.config import EngineConfig
+    from llm_infrence_engine_b200.engine import StepEntry, build_runner
+
+    folder, cfg, w, prompts, want = models[("C", dtype)]
+    ec = EngineConfig(dtype=dtype, block_size=16, num_blocks=120, max_seqs=12, max_len=160, max_num_batched_tokens=512, cuda_graphs=True)
+    spec, cache, runner = build_runner(folder, ec)
+    runner.graphs.capture_after, runner.graphs.max_shapes = 2, 1
+    talking = [("a", i) for i in range(6)] + [("b", i) for i in range(4)]
+    pos = {k: 0 for k in talking + [("e", 0)]}
+    for k in pos:
+        cache.admit(k)
+
+    def entry(k, n, wanted=True):
+        cache.reserve(k, pos[k], pos[k] + n)
+        e = StepEntry(k, prompts[k[0]][pos[k]:pos[k] + n], pos[k], list(range(n)) if wanted else ())
+        pos[k] += n
+        return e
+
+    runner.step([entry(k, 5 + 7 * i, False) for i, k in enumerate(talking)])
+    order = talking[:3] + [("e", 0)] + talking[3:]
+
+    def busy(n):
+        at = dict(pos)
+        out = runner.step([entry(k, n if k[0] == "e" else 1) for k in order]).float().cpu()
+        expect = torch.cat([want[k[0]][at[k]:pos[k]] for k in order])
+        check(out, expect, dtype, f"contexts {sorted(at.values())}", "C")
+
+    for replays in (0, 1, 2, 3):
+        busy(7)
+        assert runner.graphs.shape_replays == replays
+    for replays in (3, 4):
+        busy(9)                                                  # a newer shape takes the only place ...
+        assert runner.graphs.shape_replays == replays and len(runner.graphs.shapes) == 1
+    for replays in (4, 5, 6):
+        busy(7)                                                  # ... and the first has to come twice again
+        assert runner.graphs.shape_replays == replays

@@ -681,3 +681,36 @@ def test_router_forms_agree(K, monkeypatch, dtype, N, W, E, top, gates):
     want = REF.moe_router(h, w, None, top, gates=gates)
     for o in (outs[0], K.moe_router(hd, apart, None, top, gates=gates)):
         close(o[1].sort().values, want[1].sort().values, 2e-5)   # (logits of a scale of 45: 32-bit sums of 2,048 products in another order)
+
+
+@pytest.mark.parametrize("inner", [5124, 8960, 18944])
+def test_linear_float32_slices_longer_than_the_ring(K, inner):
+    """Slices of more than five chunks of 128: the ring of the kernel for few rows is filled again. Against float64 and the general kernel's bits; the
+    bound is that of the shorter sums above (chains of inner / 16 roundings at most)."""
+    g = torch.Generator().manual_seed(inner)
+    x, w = torch.randn(17, inner, generator=g).cuda(), torch.randn(67, inner, generator=g).cuda()
+    shifted = torch.empty(x.numel() + 1, device="cuda")[1:].view_as(x)
+    shifted.copy_(x)
+    general = K.linear(shifted, w)
+    close(general.cpu(), (x.double() @ w.double().T).cpu(), 2e-6)
+    for M in (1, 3, 16, 17):
+        for at_rest in (False, True):
+            if at_rest:
+                with K.at_rest:
+                    got = K.linear(x[:M], w)
+            else:
+                got = K.linear(x[:M], w)
+            assert torch.equal(got, general[:M]), f"{M} rows, at rest {at_rest}"
+
+
+@pytest.mark.parametrize("rows,outputs,inner", [(3, 96, 896), (40, 200, 300)])
+def test_linear_float32_of_a_matrix_that_was_just_made(K, rows, outputs, inner):
+    """The matrix is the result of the product just before: nothing of it may be read before that kernel has finished."""
+    g = torch.Generator().manual_seed(rows)
+    x, made_of = torch.randn(rows, inner, generator=g).cuda(), torch.randn(inner, 512, generator=g).cuda()
+    for i in range(20):
+        left = torch.randn(outputs, 512, generator=g).cuda()
+        torch.cuda.synchronize()
+        w = K.linear(left, made_of)             # [outputs, inner]
+        got = K.linear(x, w)
+        assert torch.equal(got, K.linear(x, w.clone())), f"time {i}"
