@@ -1357,15 +1357,15 @@ class CudaKernels:
         work = torch.empty((2 * N * H * D + 2 * N * H,), dtype=torch.float32, device=dev)
         qf, kf = work[:N * H * D], work[N * H * D:2 * N * H * D]
         ig, fg = work[2 * N * H * D:2 * N * H * D + N * H], work[2 * N * H * D + N * H:]
-        readers = torch.empty((batch.num_seqs * H,), dtype=torch.int32, device=dev)
+        before = torch.empty((batch.num_seqs * H,), dtype=torch.float32, device=dev)   # the requests' m as the step finds it
         dt = self._dt(z, "z")
         self._check(self.lib.llmie_mlstm_prepare(_ptr(z), z.shape[1], q_col, k_col, _ptr(gates), gates.shape[1], _ptr(bias_i), _ptr(bias_f),
-                                                 ctypes.c_float(cap or 0.0), ctypes.c_float(D ** -0.5), _ptr(qf), _ptr(kf), _ptr(ig), _ptr(fg), _ptr(readers),
-                                                 readers.shape[0], N, H, D, dt, self._stream()), "mlstm (prepare)")
+                                                 ctypes.c_float(cap or 0.0), ctypes.c_float(D ** -0.5), _ptr(qf), _ptr(kf), _ptr(ig), _ptr(fg), _ptr(mstate),
+                                                 _ptr(batch.seq_slots), _ptr(before), batch.num_seqs, N, H, D, dt, self._stream()), "mlstm (prepare)")
         num = torch.empty((N, H, DV + 1), dtype=torch.float32, device=dev)
         m = torch.empty((N, H), dtype=torch.float32, device=dev)
         self._check(self.lib.llmie_mlstm_scan(_ptr(z), z.shape[1], v_col, _ptr(qf), _ptr(kf), _ptr(ig), _ptr(fg), _ptr(state), _ptr(mstate),
-                                              _ptr(batch.seq_starts_dev), _ptr(batch.seq_slots), _ptr(num), _ptr(m), _ptr(readers), H, D, DV, batch.num_seqs,
+                                              _ptr(batch.seq_starts_dev), _ptr(batch.seq_slots), _ptr(num), _ptr(m), _ptr(before), H, D, DV, batch.num_seqs,
                                               int(batch.max_seq_len), dt, self._stream()), "mlstm (scan)")
         return num, m
 

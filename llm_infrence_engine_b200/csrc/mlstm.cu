@@ -40,12 +40,16 @@ template <typename T>
 __global__ void __launch_bounds__(128) mlstm_prepare_kernel(const T* __restrict__ z, int z_stride, int q_col, int k_col, const float* __restrict__ gates,
                                                             int g_stride, const float* __restrict__ bias_i, const float* __restrict__ bias_f, float cap,
                                                             float q_scale, float* __restrict__ qf, float* __restrict__ kf, float* __restrict__ ig,
-                                                            float* __restrict__ fg, int H, int D, int* __restrict__ readers, int num_readers) {
+                                                            float* __restrict__ fg, int H, int D, const float* __restrict__ mstate, const int* __restrict__ seq_slots,
+                                                            float* __restrict__ before, int R) {
     pdl_trigger();
-    pdl_wait();
     const int n = blockIdx.x;
-    if (n == 0)   // the scan's counts of readers start from zero
-        for (int i = threadIdx.x; i < num_readers; i += blockDim.x) readers[i] = 0;
+    // the requests' m as the scan's blocks are to find it, whichever of them runs last: on its way while the block does its token (where the
+    // requests' states lie was sent before the step's first kernel)
+    const int mine = n * blockDim.x + threadIdx.x;
+    const float* at = mine < R * H ? mstate + (size_t)seq_slots[mine / H] * H + mine % H : nullptr;
+    pdl_wait();
+    const float kept = at ? *at : 0.f;
     const T* row = z + (size_t)n * z_stride;
     const int HD = H * D;
     for (int i = threadIdx.x; i < HD; i += blockDim.x) {
@@ -59,6 +63,8 @@ __global__ void __launch_bounds__(128) mlstm_prepare_kernel(const T* __restrict_
         ig[(size_t)n * H + h] = xi;
         fg[(size_t)n * H + h] = log_sigmoid_f(xf);
     }
+    if (at) before[mine] = kept;
+    for (int i = mine + gridDim.x * blockDim.x; i < R * H; i += gridDim.x * blockDim.x) before[i] = mstate[(size_t)seq_slots[i / H] * H + i % H];
 }
 
 // Block (x, h, r): COLS columns of head h of request r, PARTS lanes (D / 8) to CPL columns side by side, each lane holding DPL entries of
@@ -73,14 +79,14 @@ __global__ void __launch_bounds__(128) mlstm_prepare_kernel(const T* __restrict_
 // columns to a group of 16 lanes on 80 blocks, a branch per token and the gates between two tiles on the first of the four warps, a
 // prompt of 1,301 tokens (8 heads of 128 x 128, beside one of 700) took 659 us; this form 140 us.
 //
-// The request's m is read by every block of its (h, r) and written by one: the block that is the LAST to have read it, as `readers`
-// (zeroed by the prepare kernel) tells, so that no block that starts late reads what an early one left.
+// The request's m is read by every block of its (h, r) and written by one. They read it where the prepare kernel has put it (`before`), so that
+// no block that starts late reads what an early one left.
 template <typename T, int DMAX, int CPL>
 __global__ void __launch_bounds__(ML_THREADS + 32) mlstm_scan_kernel(const T* __restrict__ v, int v_stride, int v_col, const float* __restrict__ qf,
                                                                      const float* __restrict__ kf, const float* __restrict__ ig, const float* __restrict__ fg,
                                                                      float* __restrict__ state, float* mstate, const int* __restrict__ seq_starts,
                                                                      const int* __restrict__ seq_slots, float* __restrict__ num, float* __restrict__ m_out,
-                                                                     int* __restrict__ readers, int H, int D, int DV) {
+                                                                     const float* __restrict__ before, int H, int D, int DV) {
     constexpr int PARTS = ml_parts(DMAX), DPL = DMAX / PARTS, COLS = ML_THREADS / PARTS * CPL, Q = DMAX / 4, P2 = DPL / 2, BATCH = PARTS / CPL;
     extern __shared__ __align__(16) float ml_smem[];
     float* k_s = ml_smem;                          // [2][ML_TILE][DMAX]
@@ -95,16 +101,10 @@ __global__ void __launch_bounds__(ML_THREADS + 32) mlstm_scan_kernel(const T* __
     const int slot = seq_slots[r];
     if (threadIdx.x >= ML_THREADS) {      // the warp of the gates
         const int lane = threadIdx.x - ML_THREADS;
-        float m_carry = *(volatile float*)(mstate + (size_t)slot * H + h);
-        __syncwarp();
-        bool writes = false;
-        if (lane == 0 && s0 < s1) {
-            __threadfence();              // (the read above comes before the count)
-            writes = atomicAdd(readers + (size_t)r * H + h, 1) == (int)gridDim.x - 1;
-        }
+        float m_carry = before[(size_t)r * H + h];
         float pre_i, pre_f;
         auto load = [&](int base) {
-            pre_i = -INFINITY;            // a token past the end changes nothing: m -> max(0 + m, -inf)
+            pre_i = -INFINITY;
             pre_f = 0.f;
             if (lane < ML_TILE && base + lane < s1) {
                 pre_i = ig[(size_t)(base + lane) * H + h];
@@ -115,14 +115,26 @@ __global__ void __launch_bounds__(ML_THREADS + 32) mlstm_scan_kernel(const T* __
             // the chain m -> max(f + m, i) over the tile's tokens, walked by every lane of the warp in the tokens' order (each step
             // exactly as a token-by-token walk would take it, so the bits do not depend on where a tile begins); lane t keeps token t's
             float m_run = m_carry, m_prev = m_carry, m_t = m_carry;
-#pragma unroll
-            for (int t = 0; t < ML_TILE; ++t) {
+            const int count = min(ML_TILE, s1 - base);
+            auto walk = [&](int t) {
                 const float ft = __shfl_sync(0xffffffffu, pre_f, t), it = __shfl_sync(0xffffffffu, pre_i, t);
                 const float m_new = fmaxf(ft + m_run, it);
                 if (lane == t) { m_prev = m_run; m_t = m_new; }
                 m_run = m_new;
+            };
+            // (decoded tokens: the other warps wait for this tile's gates, so the walk ends with the tokens there are. Short keys leave the chain the
+            // longest part of a tile: there one run of instructions for both measured 8 to 11 % faster on prompts, longer keys two, by as much)
+            if constexpr (DMAX <= 32) {
+#pragma unroll
+                for (int t = 0; t < ML_TILE; ++t)
+                    if (t < count) walk(t);
+            } else if (count == ML_TILE) {
+#pragma unroll
+                for (int t = 0; t < ML_TILE; ++t) walk(t);
+            } else {
+                for (int t = 0; t < count; ++t) walk(t);
             }
-            if (lane < ML_TILE) {
+            if (lane < count) {
                 a_s[buf * ML_TILE + lane] = expf(pre_f + m_prev - m_t);
                 b_s[buf * ML_TILE + lane] = expf(pre_i - m_t);
                 if (blockIdx.x == 0 && base + lane < s1) m_out[(size_t)(base + lane) * H + h] = m_t;
@@ -143,12 +155,12 @@ __global__ void __launch_bounds__(ML_THREADS + 32) mlstm_scan_kernel(const T* __
             }
         }
         pdl_trigger();
-        if (writes) mstate[(size_t)slot * H + h] = m_carry;
+        if (blockIdx.x == 0 && lane == 0 && s0 < s1) mstate[(size_t)slot * H + h] = m_carry;
         return;
     }
     const int part = threadIdx.x % PARTS, my_col = threadIdx.x / PARTS * CPL;   // the first of the lane's CPL columns, within the block
     const int col = blockIdx.x * COLS + my_col;
-    const bool vec = (D & 3) == 0;
+    const bool vec = (D & 3) == 0, vec_state = vec && ((uintptr_t)state & 15) == 0;
     float* st = state + ((size_t)slot * H + h) * C * D;
     float2 S[CPL][P2];
 #pragma unroll
@@ -156,9 +168,14 @@ __global__ void __launch_bounds__(ML_THREADS + 32) mlstm_scan_kernel(const T* __
 #pragma unroll
         for (int i = 0; i < DPL / 4; ++i) {
             const int d = 4 * PARTS * i + 4 * part;
-            float x[4];
+            float x[4] = {0.f, 0.f, 0.f, 0.f};
+            if (DMAX != 128 && vec_state) {   // (16 bytes at a time the walk of 128 entries comes out 14 % slower on a prompt, 219 -> 252 us at 2,048 tokens)
+                if (col + u < C && d < D) load4(st + (size_t)(col + u) * D + d, x);
+            } else {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) x[c] = (col + u < C && d + c < D) ? st[(size_t)(col + u) * D + d + c] : 0.f;
+                for (int c = 0; c < 4; ++c)
+                    if (col + u < C && d + c < D) x[c] = st[(size_t)(col + u) * D + d + c];
+            }
             S[u][2 * i] = make_float2(x[0], x[1]);
             S[u][2 * i + 1] = make_float2(x[2], x[3]);
         }
@@ -285,9 +302,13 @@ __global__ void __launch_bounds__(ML_THREADS + 32) mlstm_scan_kernel(const T* __
         for (int i = 0; i < DPL / 4; ++i) {
             const int d = 4 * PARTS * i + 4 * part;
             const float x[4] = {S[u][2 * i].x, S[u][2 * i].y, S[u][2 * i + 1].x, S[u][2 * i + 1].y};
+            if (vec_state) {
+                if (col + u < C && d < D) store4(st + (size_t)(col + u) * D + d, x);
+            } else {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (col + u < C && d + c < D) st[(size_t)(col + u) * D + d + c] = x[c];
+                for (int c = 0; c < 4; ++c)
+                    if (col + u < C && d + c < D) st[(size_t)(col + u) * D + d + c] = x[c];
+            }
         }
 }
 
@@ -313,7 +334,7 @@ __global__ void __launch_bounds__(128) mlstm_finish_kernel(const float* __restri
 
 template <typename T, int DM, int CPL>
 int launch_scan_as(const T* v, int v_stride, int v_col, const float* qf, const float* kf, const float* ig, const float* fg, float* state, float* mstate,
-                   const int* seq_starts, const int* seq_slots, float* num, float* m_out, int* readers, int H, int D, int DV, int R, bool alone,
+                   const int* seq_starts, const int* seq_slots, float* num, float* m_out, const float* before, int H, int D, int DV, int R, bool alone,
                    cudaStream_t s) {
     constexpr int COLS = ML_THREADS / ml_parts(DM) * CPL;
     constexpr int smem = 4 * 2 * ML_TILE * (2 * DM + COLS + 2);
@@ -323,17 +344,18 @@ int launch_scan_as(const T* v, int v_stride, int v_col, const float* qf, const f
     }
     const dim3 grid((DV + 1 + COLS - 1) / COLS, H, R);
     return launch_kernel_on(alone, mlstm_scan_kernel<T, DM, CPL>, grid, dim3(ML_THREADS + 32), (size_t)smem, s, v, v_stride, v_col, qf, kf, ig, fg, state,
-                            mstate, seq_starts, seq_slots, num, m_out, readers, H, D, DV);
+                            mstate, seq_starts, seq_slots, num, m_out, before, H, D, DV);
 }
 
 // The lanes that share a column depend on the padded key size alone, never on the batch: the order of every sum, and with it every bit. How
 // many columns a lane has changes no sum: four where the step's columns are more than fill the device two at a time.
 template <typename T>
 int launch_scan(const T* v, int v_stride, int v_col, const float* qf, const float* kf, const float* ig, const float* fg, float* state, float* mstate,
-                const int* seq_starts, const int* seq_slots, float* num, float* m_out, int* readers, int H, int D, int DV, int R, bool alone,
+                const int* seq_starts, const int* seq_slots, float* num, float* m_out, const float* before, int H, int D, int DV, int R, bool alone,
                 cudaStream_t s) {
-#define ML_ARGS v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, readers, H, D, DV, R, alone, s
-#define ML_AS(DM) return (long long)R * H * (DV + 1) * ml_parts(DM) > 148LL * ML_THREADS * 2 ? launch_scan_as<T, DM, 4>(ML_ARGS) : launch_scan_as<T, DM, 2>(ML_ARGS)
+#define ML_ARGS v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, before, H, D, DV, R, alone, s
+    const long long columns = (long long)R * H * (DV + 1);
+#define ML_AS(DM) return columns * ml_parts(DM) > 148LL * ML_THREADS * 2 ? launch_scan_as<T, DM, 4>(ML_ARGS) : launch_scan_as<T, DM, 2>(ML_ARGS)
     if (D <= 16) ML_AS(16);
     if (D <= 32) ML_AS(32);
     if (D <= 64) ML_AS(64);
@@ -346,28 +368,29 @@ int launch_scan(const T* v, int v_stride, int v_col, const float* qf, const floa
 }  // namespace
 
 // z [N, z_stride] holds q (H * D from q_col) and k (from k_col); gates [N, g_stride] float = [W_i h | W_f h]; outputs qf, kf [N, H, D],
-// ig, fg [N, H], all float; readers [num_readers] is set to zero.
+// ig, fg [N, H], all float; before [R, H]: the m of each of the step's requests (mstate [slots, H]).
 LLMIE_API int llmie_mlstm_prepare(const void* z, int z_stride, int q_col, int k_col, const float* gates, int g_stride, const float* bias_i,
-                                  const float* bias_f, float cap, float q_scale, float* qf, float* kf, float* ig, float* fg, int* readers, int num_readers,
+                                  const float* bias_f, float cap, float q_scale, float* qf, float* kf, float* ig, float* fg, const float* mstate,
+                                  const int* seq_slots, float* before, int R,
                                   int N, int H, int D, int dtype, cudaStream_t s) {
     if (N <= 0) return 0;
-    if (H <= 0 || D <= 0 || g_stride < 2 * H || q_col < 0 || k_col < 0 || !bias_i || !bias_f || !readers) return LLMIE_ERR_BAD_ARGUMENT;
+    if (H <= 0 || D <= 0 || g_stride < 2 * H || q_col < 0 || k_col < 0 || !bias_i || !bias_f || !mstate || !seq_slots || !before || R < 0) return LLMIE_ERR_BAD_ARGUMENT;
     if (dtype == DT_F32)
         return launch_kernel(mlstm_prepare_kernel<float>, dim3(N), dim3(128), 0, s, (const float*)z, z_stride, q_col, k_col, gates, g_stride, bias_i, bias_f,
-                             cap, q_scale, qf, kf, ig, fg, H, D, readers, num_readers);
+                             cap, q_scale, qf, kf, ig, fg, H, D, mstate, seq_slots, before, R);
     return launch_kernel(mlstm_prepare_kernel<bf16>, dim3(N), dim3(128), 0, s, (const bf16*)z, z_stride, q_col, k_col, gates, g_stride, bias_i, bias_f, cap,
-                         q_scale, qf, kf, ig, fg, H, D, readers, num_readers);
+                         q_scale, qf, kf, ig, fg, H, D, mstate, seq_slots, before, R);
 }
 
-// v: DV columns per head from v_col of rows of v_stride; state [slots, H, DV + 1, D], mstate [slots, H]; num [N, H, DV + 1], m_out [N, H]; readers [R, H]: zeros.
+// v: DV columns per head from v_col of rows of v_stride; state [slots, H, DV + 1, D], mstate [slots, H]; num [N, H, DV + 1], m_out [N, H]; before [R, H]: from the prepare kernel.
 LLMIE_API int llmie_mlstm_scan(const void* v, int v_stride, int v_col, const float* qf, const float* kf, const float* ig, const float* fg, float* state,
-                               float* mstate, const int* seq_starts, const int* seq_slots, float* num, float* m_out, int* readers, int H, int D, int DV, int R,
+                               float* mstate, const int* seq_starts, const int* seq_slots, float* num, float* m_out, const float* before, int H, int D, int DV, int R,
                                int max_rows, int dtype, cudaStream_t s) {
     if (R <= 0) return 0;
     if (H <= 0 || H > 65535 || R > 65535 || D <= 0 || D > 256 || DV <= 0) return LLMIE_ERR_BAD_ARGUMENT;
     const bool alone = max_rows >= 64;   // a long walk: see launch_kernel_on
-    if (dtype == DT_F32) return launch_scan<float>((const float*)v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, readers, H, D, DV, R, alone, s);
-    return launch_scan<bf16>((const bf16*)v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, readers, H, D, DV, R, alone, s);
+    if (dtype == DT_F32) return launch_scan<float>((const float*)v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, before, H, D, DV, R, alone, s);
+    return launch_scan<bf16>((const bf16*)v, v_stride, v_col, qf, kf, ig, fg, state, mstate, seq_starts, seq_slots, num, m_out, before, H, D, DV, R, alone, s);
 }
 
 // gate: H * DV columns of rows of gate_stride (storage type); w [H * DV]; out [N, H * DV] of the storage type.
