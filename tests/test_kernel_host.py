@@ -108,7 +108,7 @@ def test_weights_are_fetched_ahead_of_the_wait_only_where_they_lie_at_rest(monke
 
 @pytest.mark.parametrize("name,kernel,first", [
     ("gemm_simt.cu", "small_kernel", "fetch_weights(c);"), ("gemm_simt.cu", "tile_kernel", "fetch(t, true, false);"),
-    ("moe.cu", "moe_router_kernel", "ask(0);"), ("latent.cu", "head_matmul_kernel", "cp.async.cg"),
+    ("moe.cu", "moe_router_kernel", "(w + (size_t)e * K + k)"), ("latent.cu", "head_matmul_kernel", "cp.async.cg"),
     ("layernorm.cu", "group_rmsnorm_gate_held_kernel", "load4(w + "), ("recurrent.cu", "selective_scan_kernel", "dt_bias[stage_c]"),
     ("attention_mma.cu", "attn_mma_decode_kernel", "p.bias + (size_t)head")])
 def test_a_wait_stands_before_the_first_read_of_a_weight(name, kernel, first):
