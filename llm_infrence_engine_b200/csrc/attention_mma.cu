@@ -42,6 +42,7 @@ struct Params {
     int q_stride, max_blocks, nq, nkv, page_size, window, num_splits;
     // decode kernel, tile i is token i, not as clusters: > 0: the launch's blocks are dealt out by the tokens' lengths (see deal), this many tokens
     int balanced = 0;
+    int deal_rounds = 0;    // ... where the longest is at least this many rounds
     int page_shift;         // log2(page_size), or -1 if that is no power of two
     int cluster;            // 1: the slices of a tile are one thread-block cluster and merge through distributed shared memory
     float scale_log2;       // softmax scale * log2(e)
@@ -404,19 +405,19 @@ __device__ __forceinline__ void attend_chunk_t8(const uint32_t (&qb)[D / 16][2],
 }
 
 // ---------------------------------------------------------------------------------------------- decode
-// T8: every tile has at most 8 rows and one token (a decode step of a model with up to 8 heads per group): the transposed form.
-// SIG: sigmoid weights; TURN: results are turned back (each compiled in only where it is asked for)
-// EXT: the extras of ExtTerms (T8 only); SHARED: keys are values, a chunk is one tile of the ring
 // Which token and slice a launch's item is, when `items` of them are dealt out by the tokens' lengths: a token gets as many slices as its
 // chunks fill at the smallest length of a slice for which all slices fit the items (no token more than num_splits). The launch is made
-// once for every length a step may bring, and without this it lasts as long as the longest token takes one block. Every warp finds
-// it by itself, from the positions alone, before the wait for the kernel ahead. False: nothing to do for this item.
+// once for every length a step may bring, and without this it lasts as long as the longest token takes one block. But slices have to be merged,
+// a trip through memory: where even the longest token is fewer than deal_rounds rounds of a block's DW warps over its chunks, every token
+// stays whole. Every warp finds it by itself, from the positions alone, before the wait for the kernel ahead. False: nothing to do
+// for this item.
 constexpr int DEAL_TOKENS = 96;
-template <int BN, bool EXT>
+template <int BN, int DW, bool EXT>
 __device__ __forceinline__ bool deal(const Params& p, int item, int items, int lane, int& token, int& split, int& slices, int& pos_of_token) {
     constexpr int GROUPS = DEAL_TOKENS / 32;
     int c[GROUPS], pos[GROUPS];   // chunks and position of token lane + 32 j
     int most = 1, total = 0;
+    const int same = item < p.balanced ? p.positions[item] : 0;   // (what it takes if no token is cut, beside the others' positions)
 #pragma unroll
     for (int j = 0; j < GROUPS; ++j) pos[j] = lane + 32 * j < p.balanced ? p.positions[lane + 32 * j] : -1;
 #pragma unroll
@@ -427,32 +428,34 @@ __device__ __forceinline__ bool deal(const Params& p, int item, int items, int l
         most = max(most, c[j]);
         total += c[j];
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-        total += __shfl_xor_sync(0xffffffffu, total, o);
-    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    total = __reduce_add_sync(0xffffffffu, total);
     // slices of x chunks at `each` chunks a slice (exact: numbers of a few thousand)
     auto slices_at = [](int x, int each) { return (int)(((float)(x + each - 1) + 0.5f) * (1.0f / (float)each)); };
     int enough = most;   // chunks of a slice: this always fits (a slice per token)
     // no slice can be shorter than an even share of all chunks; where the longest token is near that, nothing is cut
     int least = max((total + items - 1) / items, (most + p.num_splits - 1) / p.num_splits);
-    if (4 * most <= 5 * least) {
-        if (item >= p.balanced) return false;
-        token = item;
-        split = 0;
-        slices = 1;
-    } else {
+    auto rounds = [](int x) { return (x + DW - 1) / DW; };
+    bool cut = 4 * most > 5 * least && rounds(most) >= p.deal_rounds;
+    if (cut) {
         while (least < enough) {
             const int mid = (least + enough) / 2;
             int n = 0;
 #pragma unroll
             for (int j = 0; j < GROUPS; ++j) n += slices_at(c[j], mid);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+            n = __reduce_add_sync(0xffffffffu, n);
             if (n <= items) enough = mid;
             else least = mid + 1;
         }
+        cut = rounds(enough) < rounds(most);
+    }
+    if (!cut) {
+        if (item >= p.balanced) return false;
+        token = item;
+        split = 0;
+        slices = 1;
+        pos_of_token = same;
+    } else {
         int before = 0;
         token = -1;
 #pragma unroll
@@ -474,15 +477,18 @@ __device__ __forceinline__ bool deal(const Params& p, int item, int items, int l
             before += __shfl_sync(0xffffffffu, upto, 31);
         }
         if (token < 0) return false;
-    }
 #pragma unroll
-    for (int j = 0; j < GROUPS; ++j) {
-        const int v = __shfl_sync(0xffffffffu, pos[j], token & 31);
-        if (token >> 5 == j) pos_of_token = v;
+        for (int j = 0; j < GROUPS; ++j) {
+            const int v = __shfl_sync(0xffffffffu, pos[j], token & 31);
+            if (token >> 5 == j) pos_of_token = v;
+        }
     }
     return true;
 }
 
+// T8: every tile has at most 8 rows and one token (a decode step of a model with up to 8 heads per group): the transposed form.
+// SIG: sigmoid weights; TURN: results are turned back (each compiled in only where it is asked for)
+// EXT: the extras of ExtTerms (T8 only); SHARED: keys are values, a chunk is one tile of the ring
 template <int D, int BN, int STAGES, int DW, bool T8, bool SIG, bool TURN, bool EXT = false, bool SHARED = false>
 __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -497,9 +503,11 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
 
     int tile = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, slices = p.num_splits, dealt_pos = 0;
     pdl_trigger();
-    if (p.balanced > 0) {
-        kvh = blockIdx.x % p.nkv;
-        if (!deal<BN, EXT>(p, blockIdx.x / p.nkv, gridDim.x / p.nkv, lane, tile, split, slices, dealt_pos)) {
+    const bool dealt = DW == 8 && p.balanced > 0;   // (only blocks of eight warps are dealt out)
+    if (dealt) {
+        const int items = gridDim.x / p.nkv;
+        kvh = blockIdx.x / items;
+        if (!deal<BN, DW, EXT>(p, blockIdx.x % items, items, lane, tile, split, slices, dealt_pos)) {
             pdl_wait();
             return;
         }
@@ -515,7 +523,7 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
     const int ntok = p.tile_info ? p.tile_info[2 * tile + 1] : 1;
     const int G = p.nq / p.nkv;
     const int nrows = ntok * G;  // <= 16
-    const int pos0 = p.balanced > 0 ? dealt_pos : p.positions[n0];
+    const int pos0 = dealt ? dealt_pos : p.positions[n0];
     const int* table = p.block_table + (size_t)p.token_seq[n0] * p.max_blocks;
     const int hi = pos0 + ntok;  // one past the last visible key
     int lo = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
@@ -1110,7 +1118,7 @@ LLMIE_API int llmie_attn_plan(const int* seq_starts, int num_seqs, int tokens_pe
     return launch_kernel(attn_plan_kernel, dim3(1), dim3(32), 0, s, seq_starts, num_seqs, tokens_per_tile, tile_info, max_tiles);
 }
 
-// balanced (0, or the number of tokens: decode modes without tile_info, not as clusters): one block per multiprocessor, dealt out by the
+// balanced (0, or the number of tokens: decode mode 1 without tile_info, not as clusters): one block per multiprocessor, dealt out by the
 // tokens' lengths; num_splits is then the most slices that a token may have.
 // decode_mode 1 or 2: every tile has at most 16 rows (tokens * group); 2 asks for blocks of four warps instead of eight when
 // nothing is cut into slices. 0: at most 64 rows.
@@ -1122,7 +1130,7 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
                    bf16* out, float* scratch_o, float* scratch_ml, int* counters, int nq, int nkv, int d,
                    int page_size, float scale, int window, int num_splits, int decode_mode, int cluster, const float* qkv_acc,
                    int acc_stride, const float* bias, const float* cos_t, const float* sin_t, const int* slots, const float* turn_cos, const float* turn_sin,
-                   const float* sig_bias, const float* log_r1, const float* log_r2, int balanced, int num_sms, cudaStream_t s, const Params* extras = nullptr,
+                   const float* sig_bias, const float* log_r1, const float* log_r2, int balanced, int deal_rounds, int num_sms, cudaStream_t s, const Params* extras = nullptr,
                    int bias_at_rest = 0) {
     if (num_tiles <= 0) return 0;
     if ((turn_cos == nullptr) != (turn_sin == nullptr) || (log_r1 == nullptr) != (log_r2 == nullptr) || (log_r1 && !sig_bias) ||
@@ -1132,7 +1140,7 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
                     (acc_stride & 1) || ((uintptr_t)qkv_acc & 7) || ((uintptr_t)bias & 7) || ((uintptr_t)cos_t & 7) || ((uintptr_t)sin_t & 7)))
         return LLMIE_ERR_BAD_ARGUMENT;
     if (cluster && (!decode_mode || num_splits > 8)) return LLMIE_ERR_BAD_ARGUMENT;
-    if (balanced && (balanced != num_tiles || balanced > DEAL_TOKENS || !decode_mode || cluster || tile_info || nkv < 1 || num_tiles > num_sms / nkv))
+    if (balanced && (balanced != num_tiles || balanced > DEAL_TOKENS || decode_mode != 1 || cluster || tile_info || nkv < 1 || num_tiles > num_sms / nkv))
         return LLMIE_ERR_BAD_ARGUMENT;
     if ((d != 64 && d != 128) || nkv <= 0 || nq % nkv || page_size <= 0 || num_splits < 1 || q_stride % 8 || nkv > 65535 ||
         num_splits > 64 || (num_splits > 1 && !cluster && (!scratch_o || !scratch_ml || !counters)))
@@ -1144,7 +1152,7 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
     p.tile_info = tile_info; p.out = out; p.part_o = scratch_o; p.part_ml = scratch_ml; p.counters = counters;
     p.q_stride = q_stride; p.max_blocks = max_blocks; p.nq = nq; p.nkv = nkv; p.page_size = page_size; p.window = window;
     p.page_shift = (page_size & (page_size - 1)) == 0 ? __builtin_ctz((unsigned)page_size) : -1;
-    p.num_splits = num_splits; p.balanced = balanced; p.scale_log2 = scale * LOG2E; p.cluster = cluster;
+    p.num_splits = num_splits; p.balanced = balanced; p.deal_rounds = deal_rounds; p.scale_log2 = scale * LOG2E; p.cluster = cluster;
     p.qkv_acc = qkv_acc; p.acc_stride = acc_stride; p.bias = bias; p.bias_at_rest = bias_at_rest; p.cos_t = cos_t; p.sin_t = sin_t; p.slots = slots;
     p.turn_cos = turn_cos; p.turn_sin = turn_sin; p.sig_bias = sig_bias; p.log_r1 = log_r1; p.log_r2 = log_r2;
     if (extras) {
@@ -1160,11 +1168,11 @@ LLMIE_API int llmie_paged_attention_mma(const bf16* q, int q_stride, const bf16*
                                         int max_blocks, const int* token_seq, const int* positions, const int* tile_info, int num_tiles,
                                         bf16* out, float* scratch_o, float* scratch_ml, int* counters, int nq, int nkv, int d,
                                         int page_size, float scale, int window, int num_splits, int decode_mode, int cluster, const float* turn_cos,
-                                        const float* turn_sin, const float* sig_bias, const float* log_r1, const float* log_r2, int balanced,
+                                        const float* turn_sin, const float* sig_bias, const float* log_r1, const float* log_r2, int balanced, int deal_rounds,
                                         int num_sms, cudaStream_t s) {
     return run_mma(q, q_stride, k_pool, v_pool, block_table, max_blocks, token_seq, positions, tile_info, num_tiles, out, scratch_o, scratch_ml,
                    counters, nq, nkv, d, page_size, scale, window, num_splits, decode_mode, cluster, nullptr, 0, nullptr, nullptr, nullptr,
-                   nullptr, turn_cos, turn_sin, sig_bias, log_r1, log_r2, balanced, num_sms, s);
+                   nullptr, turn_cos, turn_sin, sig_bias, log_r1, log_r2, balanced, deal_rounds, num_sms, s);
 }
 
 // Decode steps (tile i is token i, at most 8 query heads per key/value head) with chunks, a soft cap, a bias by distance (rel [rel_rows][nq],
@@ -1174,7 +1182,7 @@ LLMIE_API int llmie_paged_attention_mma_ext(const bf16* q, int q_stride, const b
                                             const int* token_seq, const int* positions, int num_tokens, bf16* out, float* scratch_o, float* scratch_ml,
                                             int* counters, int nq, int nkv, int d, int page_size, float scale, int window, int num_splits, int cluster,
                                             int four_warps, int chunk, float softcap, const float* rel, const int* rows_of, int n_rows_of, int rel_rows,
-                                            const bf16* gate, int gate_stride, const float* key_scale, int balanced, int num_sms, cudaStream_t s) {
+                                            const bf16* gate, int gate_stride, const float* key_scale, int balanced, int deal_rounds, int num_sms, cudaStream_t s) {
     if (num_tokens <= 0) return 0;
     if (nkv <= 0 || nq / nkv > 8 || chunk < 0 || softcap < 0.f || scale == 0.f || (rel && (!rows_of || rel_rows < 1 || n_rows_of < 0)) ||
         (v_pool == nullptr) != (key_scale != nullptr))
@@ -1184,7 +1192,7 @@ LLMIE_API int llmie_paged_attention_mma_ext(const bf16* q, int q_stride, const b
     e.rel = rel; e.rows_of = rows_of; e.n_rows_of = n_rows_of; e.rel_rows = rel_rows; e.gate = gate; e.gate_stride = gate_stride; e.key_scale = key_scale;
     return run_mma(q, q_stride, k_pool, v_pool, block_table, max_blocks, token_seq, positions, nullptr, num_tokens, out, scratch_o, scratch_ml, counters,
                    nq, nkv, d, page_size, scale, window, num_splits, four_warps ? 2 : 1, cluster, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr,
-                   nullptr, nullptr, nullptr, nullptr, balanced, num_sms, s, &e);
+                   nullptr, nullptr, nullptr, nullptr, balanced, deal_rounds, num_sms, s, &e);
 }
 
 // Decode steps (every tile one token, at most 8 query heads per key/value head): the same attention, with the queries, keys and
@@ -1195,9 +1203,9 @@ LLMIE_API int llmie_paged_attention_mma_acc(const float* qkv_acc, int acc_stride
                                             const int* slots, bf16* k_pool, bf16* v_pool, const int* block_table, int max_blocks,
                                             const int* token_seq, const int* positions, int num_tokens, bf16* out, float* scratch_o,
                                             float* scratch_ml, int* counters, int nq, int nkv, int d, int page_size, float scale, int window,
-                                            int num_splits, int cluster, int four_warps, int balanced, int num_sms, int bias_at_rest, cudaStream_t s) {
+                                            int num_splits, int cluster, int four_warps, int balanced, int deal_rounds, int num_sms, int bias_at_rest, cudaStream_t s) {
     if (!qkv_acc) return LLMIE_ERR_BAD_ARGUMENT;
     return run_mma(nullptr, 8, k_pool, v_pool, block_table, max_blocks, token_seq, positions, nullptr, num_tokens, out, scratch_o, scratch_ml,
                    counters, nq, nkv, d, page_size, scale, window, num_splits, four_warps ? 2 : 1, cluster, qkv_acc, acc_stride, bias, cos_t, sin_t, slots,
-                   nullptr, nullptr, nullptr, nullptr, nullptr, balanced, num_sms, s, nullptr, bias_at_rest);
+                   nullptr, nullptr, nullptr, nullptr, nullptr, balanced, deal_rounds, num_sms, s, nullptr, bias_at_rest);
 }

@@ -136,6 +136,10 @@ class CudaKernels:
         self._decode_four_warps = False         # the last decode plan asked for blocks of four warps
         self._decode_balanced = 0               # ... and for blocks dealt out by the lengths of this many tokens
         self.balance_decode = True
+        # By head size: where the step's longest request is fewer rounds of a block's warps than this (2,049 and 897 keys), none is cut. Measured with
+        # blocks dealt out whatever the lengths, and with every token whole (us): heads of 64 over 4, 32 requests of 128 to 512 keys 7.7 / 4.5,
+        # to 2,048 10.9 / 9.8, to 4,096 15.8 / 18.0, 20 to 8,190 35 / 40; heads of 128 over 2, 64 requests to 512 8.4 / 7.4, to 1,024 11.0 / 11.3, to 2,048 18.2 / 20.5
+        self.deal_rounds = {64: 9, 128: 8}
         self.at_rest = AtRest()
         for fn in ("llmie_embed", "llmie_feed_tokens", "llmie_zero_fresh_state", "llmie_rope_tables", "llmie_add_rmsnorm", "llmie_rope_kv_write", "llmie_silu_mul",
                    "llmie_gemm_simt", "llmie_gemm_tc", "llmie_gateup_silu_tc", "llmie_qkv_rope_tc", "llmie_add_into", "llmie_attn_plan", "llmie_attn_tc_plan", "llmie_paged_attention_mma", "llmie_paged_attention_mma_acc", "llmie_paged_attention_tc", "llmie_paged_attention_f32", "llmie_paged_attention_bf16", "llmie_argmax", "llmie_sample",
@@ -780,9 +784,9 @@ class CudaKernels:
                 and chunks > 96):
             # Nearly a block per multiprocessor, whose requests may differ in length: without slices the launch lasts as long as its longest
             # request takes one multiprocessor. The blocks (one per multiprocessor) are dealt out on the device by the lengths that
-            # the step has (at most 16 slices of a token). Measured: heads of 128, 64 requests of 128 to 2,048 keys 18.6 -> 14.6 us, 48 requests of
-            # 20 to 8,190 60 -> 17; where all are alike the look at the lengths costs 0.4 us (of 24 at 2,048 keys), which the few rounds of
-            # shorter contexts do not win back (heads of 64, 128 to 2,048 keys, 65 chunks: 10.1 -> 11.2)
+            # the step has (at most 16 slices of a token), if they are long enough for it (deal_rounds; the host knows only the longest
+            # that a captured step may ever bring). 64 requests of 20 to 8,190 keys, heads of 64 over 2: 42 -> 31 us; where no token is cut
+            # the look at the lengths costs 0.1 to 0.4 us
             num_splits, self._decode_balanced = 16, tiles
         elif decode and num_splits == 1:
             blocks = max(1, tiles * num_kv_heads)
@@ -830,7 +834,8 @@ class CudaKernels:
             _ptr(positions), _ptr(tile_info), tiles, _ptr(out), _ptr(scratch_o), _ptr(scratch_ml), _ptr(counters), num_heads,
             num_kv_heads, head_dim, page_size, ctypes.c_float(scale), int(window), num_splits,
             2 if (decode and self._decode_four_warps) else int(decode), cluster,
-            *self._turn_and_sigmoid(turn, sigmoid_bias, log_distance), self._decode_balanced if decode else 0, self.num_sms, self._stream()),
+            *self._turn_and_sigmoid(turn, sigmoid_bias, log_distance), self._decode_balanced if decode else 0, self.deal_rounds.get(head_dim, 0),
+            self.num_sms, self._stream()),
             "paged_attention (tensor cores)")
         return out
 
@@ -897,7 +902,7 @@ class CudaKernels:
                 _ptr(sums), width, _ptr(bias), _ptr(cos), _ptr(sin), _ptr(slot_mapping if write_kv else None), _ptr(k_pool), _ptr(v_pool),
                 _ptr(block_table), block_table.shape[1], _ptr(token_seq), _ptr(positions), M, _ptr(out), _ptr(scratch_o), _ptr(scratch_ml),
                 _ptr(counters), num_heads, num_kv_heads, head_dim, page_size, ctypes.c_float(scale), int(window), num_splits, cluster,
-                int(self._decode_four_warps), self._decode_balanced, self.num_sms, self._weights_at_rest(), self._stream()), "qkv_attention (tensor cores)")
+                int(self._decode_four_warps), self._decode_balanced, self.deal_rounds.get(head_dim, 0), self.num_sms, self._weights_at_rest(), self._stream()), "qkv_attention (tensor cores)")
             self._dirty_qkv = sums
             return out
         qkv = self.qkv_rope(x, w, bias, cos, sin, slot_mapping, k_pool, v_pool, num_heads, num_kv_heads, head_dim, page_size, write_kv,
@@ -1211,7 +1216,7 @@ class CudaKernels:
                     n_splits, cluster, int(self._decode_four_warps), int(chunk), ctypes.c_float(softcap), _ptr(rel), _ptr(rel_rows),
                     0 if rel_rows is None else rel_rows.shape[0], 0 if rel is None else rel.shape[0],
                     ctypes.c_void_p(0 if gate is None else gate.data_ptr() + gate_col * esize), 0 if gate is None else gate.shape[1], _ptr(key_scale),
-                    self._decode_balanced, self.num_sms, self._stream()), "attention_ext (decode, tensor cores)")
+                    self._decode_balanced, self.deal_rounds.get(head_dim, 0), self.num_sms, self._stream()), "attention_ext (decode, tensor cores)")
                 return out
             done = self._attention_tc(q, k_pool, v_pool, block_table, token_seq, positions, out, num_heads, num_kv_heads, head_dim, page_size, scale,
                                       int(window), span, batch, num_splits, chunk=chunk, softcap=softcap, rel=rel, rel_rows=rel_rows, gate=gate, gate_col=gate_col,

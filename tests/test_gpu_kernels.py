@@ -714,3 +714,18 @@ def test_linear_float32_of_a_matrix_that_was_just_made(K, rows, outputs, inner):
         w = K.linear(left, made_of)             # [outputs, inner]
         got = K.linear(x, w)
         assert torch.equal(got, K.linear(x, w.clone())), f"time {i}"
+
+
+@pytest.mark.parametrize("nq,nkv,d,lens", [
+    (14, 2, 64, [128 + 29 * i for i in range(64)]), (12, 2, 128, [128 + 6 * i for i in range(64)]), (8, 4, 64, [128 + 12 * i for i in range(32)]), (16, 8, 64, [20] * 18)])
+def test_short_contexts_are_not_cut_whatever_the_step_could_hold(K, nq, nkv, d, lens):
+    """A captured step is planned for the longest context there may be. Where the step's own are so short that a merge costs more than the
+    slices save, every token stays whole: the bits of a launch that cannot cut."""
+    span = 32768
+    qkv, kp, vp, table, tseq, pos = _attention_case(torch.bfloat16, nq, nkv, d, 16, lens, [1] * len(lens), 0, 5)
+    table = torch.nn.functional.pad(table, (0, span // 16 - table.shape[1]))
+    dev = [t.cuda() for t in (qkv, kp, vp, table, tseq, pos)]
+    got = K.paged_attention(*dev, nq, nkv, d, 16, d ** -0.5, 0, span, batch=_Batch([1] * len(lens)))
+    assert K._decode_balanced == len(lens)
+    whole = K.paged_attention(*dev, nq, nkv, d, 16, d ** -0.5, 0, span, batch=_Batch([1] * len(lens)), num_splits=1)
+    assert torch.equal(got, whole)
