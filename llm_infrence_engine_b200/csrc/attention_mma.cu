@@ -488,12 +488,17 @@ __device__ __forceinline__ bool deal(const Params& p, int item, int items, int l
 
 // T8: every tile has at most 8 rows and one token (a decode step of a model with up to 8 heads per group): the transposed form.
 // SIG: sigmoid weights; TURN: results are turned back (each compiled in only where it is asked for)
-// EXT: the extras of ExtTerms (T8 only); SHARED: keys are values, a chunk is one tile of the ring
-template <int D, int BN, int STAGES, int DW, bool T8, bool SIG, bool TURN, bool EXT = false, bool SHARED = false>
-__global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p) {
+// EXT: the extras of ExtTerms (T8 only); SHARED: keys are values, a chunk is one tile of the ring; ACC: queries, keys and values come as the
+// projection's sums; BAL: p.balanced > 0, the blocks are dealt out by the tokens' lengths. (Compiled in only where they are: a choice at run
+// time cost launches that have neither up to 28 registers and, heads of 128, 6 to 12 % of their time: 256 blocks of 128 to 2,048 keys 35 -> 39 us)
+// One block of eight warps fills a multiprocessor's shared memory, so it may take the registers of two (heads of 128: 154 instead of the 128 that the
+// compiler chose by itself; a step of 64 requests of 20 to 8,190 keys, twelve layers of 1,536: 1,549 -> 1,403 us).
+template <int D, int BN, int STAGES, int DW, bool T8, bool SIG, bool TURN, bool EXT = false, bool SHARED = false, bool ACC = false, bool BAL = false>
+__global__ void __launch_bounds__(DW * 32, DW == 8 ? 1 : 2) attn_mma_decode_kernel(const Params p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     static_assert((!EXT || (T8 && !SIG && !TURN)) && (!SHARED || EXT), "the extras are built for the transposed form");
+    static_assert(!ACC || (T8 && !SIG && !TURN && !EXT), "the projection's sums are taken by the plain transposed form");
     constexpr int TILE = BN * D;                       // elements of one K or V chunk
     constexpr int SLOT = SHARED ? TILE : 2 * TILE;     // elements of a slot of the ring
     constexpr int V_AT = SHARED ? 0 : TILE;            // where the values of a slot lie
@@ -501,16 +506,23 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
     float* my_numbers = reinterpret_cast<float*>(smem_raw + (size_t)DW * STAGES * SLOT * sizeof(bf16)) + warp * STAGES * BN;   // SHARED: [STAGES][BN]
     __shared__ int flag;
 
-    int tile = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, slices = p.num_splits, dealt_pos = 0;
+    int tile = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, slices = p.num_splits, dealt_pos = 0, dealt_seq = 0;
     pdl_trigger();
-    const bool dealt = DW == 8 && p.balanced > 0;   // (only blocks of eight warps are dealt out)
-    if (dealt) {
-        const int items = gridDim.x / p.nkv;
+    if constexpr (BAL) {
+        const int items = gridDim.x / p.nkv, item = blockIdx.x % items;
         kvh = blockIdx.x / items;
-        if (!deal<BN, DW, EXT>(p, blockIdx.x % items, items, lane, tile, split, slices, dealt_pos)) {
+        dealt_seq = p.token_seq[min(item, p.balanced - 1)];   // (on its way beside the positions: right if no token is cut)
+        if (!deal<BN, DW, EXT>(p, item, items, lane, tile, split, slices, dealt_pos)) {
             pdl_wait();
             return;
         }
+        if (tile != item) dealt_seq = p.token_seq[tile];
+        // (the same in every lane, which a warp-wide reduction tells the compiler: addresses made of them stay in uniform registers)
+        tile = __reduce_max_sync(0xffffffffu, tile);
+        split = __reduce_max_sync(0xffffffffu, split);
+        slices = __reduce_max_sync(0xffffffffu, slices);
+        dealt_pos = __reduce_max_sync(0xffffffffu, dealt_pos);
+        dealt_seq = __reduce_max_sync(0xffffffffu, dealt_seq);
     }
     // What this block needs of the step's own integers (positions, table rows, block tables) was copied to the device
     // before the step's first kernel, and keys and values of earlier positions were written by earlier steps: none of it
@@ -523,8 +535,8 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
     const int ntok = p.tile_info ? p.tile_info[2 * tile + 1] : 1;
     const int G = p.nq / p.nkv;
     const int nrows = ntok * G;  // <= 16
-    const int pos0 = dealt ? dealt_pos : p.positions[n0];
-    const int* table = p.block_table + (size_t)p.token_seq[n0] * p.max_blocks;
+    const int pos0 = BAL ? dealt_pos : p.positions[n0];
+    const int* table = p.block_table + (size_t)(BAL ? dealt_seq : p.token_seq[n0]) * p.max_blocks;
     const int hi = pos0 + ntok;  // one past the last visible key
     int lo = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
     if (EXT && p.chunk > 0) lo = max(lo, pos0 / p.chunk * p.chunk);
@@ -537,7 +549,7 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
     const int mine = first < c_end ? (c_end - first + DW - 1) / DW : 0;
     // Where the first chunks lie is looked up before the wait for all of them. (From the projection's sums) a chunk that holds the
     // token's own position is fetched early too: the rows that the cache does not hold yet are replaced below by the warp that owns it.
-    const bool own_here = T8 && p.qkv_acc && p.slots;
+    const bool own_here = ACC && p.slots;
     int own_it = -1;
     if (own_here) {
         const int c_p = (pos0 - lo) / BN;   // the chunk that holds the token's own position
@@ -557,14 +569,14 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
         if (fetched[s]) copy_rows_warp<D, BN, SHARED>(p, rows_at[s], 0, my + s * SLOT, my + s * SLOT + V_AT, lane, my_numbers + s * BN);
     }
     // biases at rest are asked for before the wait as well
-    float q_bias[T8 ? D / 16 : 1][4];
-    if constexpr (T8) {
-        if (early && p.qkv_acc && p.bias) pdl_wait_unless(p.bias_at_rest);
+    float q_bias[ACC ? D / 16 : 1][4];
+    if constexpr (ACC) {
+        if (p.bias) pdl_wait_unless(p.bias_at_rest);
         const int head = kvh * G + ((lane >> 2) < nrows ? lane >> 2 : 0);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
             q_bias[kk][0] = q_bias[kk][1] = q_bias[kk][2] = q_bias[kk][3] = 0.f;
-            if (p.qkv_acc && p.bias) {
+            if (p.bias) {
                 const int col = kk * 16 + ((lane & 3) << 1);
                 const float2 ba = *reinterpret_cast<const float2*>(p.bias + (size_t)head * D + col);
                 const float2 bc = *reinterpret_cast<const float2*>(p.bias + (size_t)head * D + col + 8);
@@ -588,12 +600,12 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
     float o[T8 ? D / 16 : D / 8][4];
     // (from the projection's sums) the token's own key and value, finished by the warp that owns its position: pairs
     // (j, j + D / 2) for j = lane, lane + 32, ...
-    constexpr int NP = D / 64;
+    constexpr int NP = ACC ? D / 64 : 1;
     uint32_t own_k[NP], own_v[NP];   // (element j, element j + D / 2) as two bfloat16
     if constexpr (T8) {
         const int row = lane >> 2;
         const bool ok = row < nrows;
-        if (p.qkv_acc) {
+        if constexpr (ACC) {
             const int head = kvh * G + (ok ? row : 0);
             const float* src = p.qkv_acc + (size_t)n0 * p.acc_stride + (size_t)head * D;
             const float* ct = p.cos_t + (size_t)n0 * (D / 2);
@@ -742,7 +754,7 @@ __global__ void __launch_bounds__(DW * 32) attn_mma_decode_kernel(const Params p
         __syncwarp();
         bf16* cur = my + (it % STAGES) * SLOT;
         const int key0 = lo + (first + it * DW) * BN;
-        if (it == own_it) {
+        if (ACC && it == own_it) {
             // The token's own position lies in this chunk, and the cache did not hold its key and value when the chunk was
             // fetched: the row (and the rows behind it, which were fetched from the same place and which the mask hides, but
             // whose values would still be multiplied by zero) gets what this warp has just made.
@@ -1041,8 +1053,11 @@ __global__ void attn_plan_kernel(const int* __restrict__ starts, int num_seqs, i
     for (; t < max_tiles; ++t) { tile_info[2 * t] = 0; tile_info[2 * t + 1] = 0; }
 }
 
-template <int D, bool T8, int DW, bool SIG, bool TURN, bool EXT = false, bool SHARED = false>
+template <int D, bool T8, int DW, bool SIG, bool TURN, bool EXT = false, bool SHARED = false, bool ACC = false, bool BAL = false>
 int launch_decode_as(const Params& p, dim3 grid, cudaStream_t s) {
+    if constexpr (DW == 8 && !BAL) {
+        if (p.balanced > 0) return launch_decode_as<D, T8, DW, SIG, TURN, EXT, SHARED, ACC, true>(p, grid, s);
+    }
     // DW warps, each with its own ring of three slots of 8 KB: keys and values of BN of them, or twice as many keys that are values
     constexpr int BN = (D == 64 ? 32 : 16) * (SHARED ? 2 : 1), STAGES = 3;
     constexpr size_t ring = (size_t)DW * STAGES * ((SHARED ? 1 : 2) * BN * D * sizeof(bf16) + (SHARED ? BN * sizeof(float) : 0));
@@ -1050,7 +1065,7 @@ int launch_decode_as(const Params& p, dim3 grid, cudaStream_t s) {
     constexpr size_t smem = ring > merge ? ring : merge;
     static bool set = false;
     if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(attn_mma_decode_kernel<D, BN, STAGES, DW, T8, SIG, TURN, EXT, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_mma_decode_kernel<D, BN, STAGES, DW, T8, SIG, TURN, EXT, SHARED, ACC, BAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         set = true;
     }
@@ -1069,9 +1084,9 @@ int launch_decode_as(const Params& p, dim3 grid, cudaStream_t s) {
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = llmie_pdl_flag ? 2 : 1;
-        return (int)cudaLaunchKernelEx(&cfg, attn_mma_decode_kernel<D, BN, STAGES, DW, T8, SIG, TURN, EXT, SHARED>, p);
+        return (int)cudaLaunchKernelEx(&cfg, attn_mma_decode_kernel<D, BN, STAGES, DW, T8, SIG, TURN, EXT, SHARED, ACC, BAL>, p);
     }
-    return launch_kernel(attn_mma_decode_kernel<D, BN, STAGES, DW, T8, SIG, TURN, EXT, SHARED>, grid, dim3(DW * 32), smem, s, p);
+    return launch_kernel(attn_mma_decode_kernel<D, BN, STAGES, DW, T8, SIG, TURN, EXT, SHARED, ACC, BAL>, grid, dim3(DW * 32), smem, s, p);
 }
 
 template <int D, bool T8, int DW>
@@ -1079,6 +1094,9 @@ int launch_decode(const Params& p, dim3 grid, cudaStream_t s) {
     if (p.x_scale != 0.f) {   // (set for the extras only)
         if constexpr (T8) return p.key_scale ? launch_decode_as<D, T8, DW, false, false, true, true>(p, grid, s) : launch_decode_as<D, T8, DW, false, false, true, false>(p, grid, s);
         else return LLMIE_ERR_BAD_ARGUMENT;
+    }
+    if constexpr (T8) {
+        if (p.qkv_acc) return launch_decode_as<D, T8, DW, false, false, false, false, true>(p, grid, s);
     }
     if (p.sig_bias) return p.turn_cos ? launch_decode_as<D, T8, DW, true, true>(p, grid, s) : launch_decode_as<D, T8, DW, true, false>(p, grid, s);
     return p.turn_cos ? launch_decode_as<D, T8, DW, false, true>(p, grid, s) : launch_decode_as<D, T8, DW, false, false>(p, grid, s);

@@ -663,24 +663,101 @@ def test_transient_products_are_consumed_and_cleared(K):
     K.check_device_errors()
 
 
-@pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("N,W,E,top,gates", [(1, 512, 8, 2, 0), (3, 1024, 16, 4, 2), (64, 1024, 64, 6, 0), (5, 2048, 128, 8, 1), (148, 896, 300, 2, 0), (149, 512, 18, 2, 0), (2, 300, 17, 3, 0)])
-def test_router_forms_agree(K, monkeypatch, dtype, N, W, E, top, gates):
-    """All pieces asked for at once or output by output, sixteen warps or eight (more rows than multiprocessors): the same sums in the same order."""
-    h, w = torch.randn(N, W, generator=torch.Generator().manual_seed(1)).to(dtype), torch.randn(E + gates, W, generator=torch.Generator().manual_seed(2)).to(dtype)
-    monkeypatch.setattr(K, "tc_max_rows", 1 << 20)
-    hd, wd = h.cuda(), w.cuda()
-    apart = torch.empty(w.numel() + 1, dtype=dtype, device="cuda")[1:].view_as(wd)   # not on a 16-byte boundary
-    apart.copy_(wd)
-    many = K.moe_router(hd.repeat(150, 1), wd, None, top, gates=gates)
-    outs = [K.moe_router(hd, wd, None, top, gates=gates), [o[:N] for o in many]]
-    with K.at_rest:
-        outs.append(K.moe_router(hd, wd, None, top, gates=gates))
-    for o in outs[1:]:
-        assert all(torch.equal(a, b) for a, b in zip(outs[0], o))
-    want = REF.moe_router(h, w, None, top, gates=gates)
-    for o in (outs[0], K.moe_router(hd, apart, None, top, gates=gates)):
-        close(o[1].sort().values, want[1].sort().values, 2e-5)   # (logits of a scale of 45: 32-bit sums of 2,048 products in another order)
+# ------------------------------------------------------------------ blocks of decoded tokens dealt out by length, in every form
+DEALT = [3300, 1, 2, 15, 16, 17, 31, 32, 33, 3200, 3201, 1600, 2049, 4096, 4095, 64, 65, 5000] + [40 + 57 * i for i in range(30)]
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("form", ["sums", "sums, cached before", "window", "sigmoid", "sigmoid and distance", "turned back", "sigmoid, turned back",
+                                  "chunk", "cap, bias by distance and gate", "keys that are values", "keys that are values, chunk and gate"])
+def test_decode_attention_dealt_out_in_every_form(K, monkeypatch, d, form):
+    """Tokens cut into slices by the step's lengths against every token whole (which the other tests hold against plain torch): own
+    positions at the edges of chunks and of slices, requests of one token, padding rows of a captured step (token 0 of a null table row). Bound: the same
+    32-bit sums in another order, rounded to bfloat16 once (2^-8 of a result), as in the tests of the kernel's slices."""
+    monkeypatch.setattr(K, "fuse_decode_rope_head_dims", (64, 128))
+    monkeypatch.setattr(K, "deal_rounds", {64: 0, 128: 0})   # short requests are cut too where that saves a round
+    nq, nkv, ps = 12, 2, 16
+    lens = DEALT + [1, 1]
+    n, span = len(lens), max(DEALT)
+    g = torch.Generator().manual_seed(60)
+    qkv, kp, vp, table, tseq, pos = _attention_case(torch.bfloat16, nq, nkv, d, ps, lens, [1] * n, 0, 61)
+    table[-2:] = 0
+    width, scale = (nq + 2 * nkv) * d, d ** -0.5
+    batch = _Batch([1] * n)
+    cu = lambda *ts: [t.cuda() for t in ts]
+    table, tseq, pos_d = cu(table, tseq, pos)
+    slots = torch.tensor([int(table[r, (L - 1) // ps]) * ps + (L - 1) % ps for r, L in enumerate(lens)], dtype=torch.int32)
+    if form.startswith("sums"):
+        # small whole numbers: the product's split sums are exact, whatever order its blocks add them in
+        x, w = torch.randint(-4, 5, (n, 256), generator=g).to(torch.bfloat16).cuda(), (torch.randint(-8, 9, (width, 256), generator=g) / 128).to(torch.bfloat16).cuda()
+        cos, sin = (t.cuda() for t in REF.rope_tables(pos, 1.0 / (1e6 ** (torch.arange(0, d, 2).float() / d))))
+        bias = torch.randn(width, generator=g).cuda()
+        write = form == "sums"
+        if write:   # (the padding rows share the null page, which nobody reads with these lengths' masks but themselves)
+            for r, L in enumerate(lens[:-2]):
+                kp[int(table[r, (L - 1) // ps]), :, (L - 1) % ps:] = float("nan")
+                vp[int(table[r, (L - 1) // ps]), :, (L - 1) % ps:] = float("nan")
+        pools = {}
+
+        def run(how):
+            pools[how] = (kp.cuda(), vp.cuda())
+            K._clear_dirty()
+            return K.qkv_attention(x, w, bias, cos, sin, slots.cuda(), *pools[how], table, tseq, pos_d, nq, nkv, d, ps, scale, 0, span, batch=batch, write_kv=write)
+    elif form == "window":
+        dev = cu(qkv, kp, vp)
+
+        def run(how):
+            return K.paged_attention(*dev, table, tseq, pos_d, nq, nkv, d, ps, scale, 3300, span, batch=batch)
+    else:
+        q = qkv[:, :nq * d + 2 * nkv * d].contiguous().cuda()
+        pools_d = cu(kp, vp)
+        rel_rows = torch.tensor([min(8, i // 400) for i in range(4000)], dtype=torch.int32).cuda()
+        rel, gate = torch.randn(9, nq, generator=g).cuda(), torch.randn(n, nq + 4, generator=g).to(torch.bfloat16).cuda()
+        number = (torch.rand(kp.shape[0], ps, generator=g) + 0.2).cuda()
+        ang = torch.randn(n, d // 2, generator=g)
+        turn = (torch.cos(ang).cuda(), torch.sin(ang).cuda(), False)
+        per_head = lambda s=1.0: (torch.rand(nq, generator=g) * s).cuda()
+        kw = {"sigmoid": dict(sigmoid_bias=per_head() - 5), "sigmoid and distance": dict(sigmoid_bias=per_head() - 4, log_distance=(per_head(0.5), per_head(0.1))),
+              "turned back": dict(turn=turn), "sigmoid, turned back": dict(sigmoid_bias=per_head() - 5, turn=turn), "chunk": dict(chunk=4000),
+              "cap, bias by distance and gate": dict(softcap=3.0, rel=rel, rel_rows=rel_rows, gate=gate, gate_col=2, gate_per_head=True),
+              "keys that are values": dict(key_scale=number), "keys that are values, chunk and gate": dict(key_scale=number, chunk=4000, gate=gate, gate_col=2, gate_per_head=True)}[form]
+        values = None if "key_scale" in kw else pools_d[1]
+
+        def run(how):
+            return K.attention_ext(q, 0, nq, nkv, d, d, pools_d[0], values, table, tseq, pos_d, ps, scale, 0, span, batch=batch, **kw)
+    monkeypatch.setattr(K, "balance_decode", False)
+    whole = run("whole")
+    assert K._decode_balanced == 0
+    monkeypatch.setattr(K, "balance_decode", True)
+    for _ in range(2):
+        cut = run("cut")
+        K.check_device_errors()
+        assert K._decode_balanced == n and not torch.isnan(cut).any()
+        close(cut, whole, 1e-2)
+        # (a penalty by distance leaves far slices below the rounding: the same bits whatever the cut)
+        assert form == "sigmoid and distance" or not torch.equal(cut, whole), "nothing was cut"
+        assert K._attn_counters is None or K._attn_counters.abs().sum().item() == 0
+    if form == "sums":
+        real = slots[:-2].long()
+        for a, b in zip(pools["whole"], pools["cut"]):
+            own = [t.permute(0, 2, 1, 3).reshape(-1, nkv, d)[real.cuda()] for t in (a, b)]
+            assert torch.equal(*own)
+    K._clear_dirty()
+
+
+@pytest.mark.parametrize("nq,nkv,d,lens", [
+    (14, 2, 64, [128 + 29 * i for i in range(64)]), (12, 2, 128, [128 + 6 * i for i in range(64)]), (8, 4, 64, [128 + 12 * i for i in range(32)]), (16, 8, 64, [20] * 18)])
+def test_short_contexts_are_not_cut_whatever_the_step_could_hold(K, nq, nkv, d, lens):
+    """A captured step is planned for the longest context there may be. Where the step's own are so short that a merge costs more than the
+    slices save, every token stays whole: the bits of a launch that cannot cut."""
+    span = 32768
+    qkv, kp, vp, table, tseq, pos = _attention_case(torch.bfloat16, nq, nkv, d, 16, lens, [1] * len(lens), 0, 5)
+    table = torch.nn.functional.pad(table, (0, span // 16 - table.shape[1]))
+    dev = [t.cuda() for t in (qkv, kp, vp, table, tseq, pos)]
+    got = K.paged_attention(*dev, nq, nkv, d, 16, d ** -0.5, 0, span, batch=_Batch([1] * len(lens)))
+    assert K._decode_balanced == len(lens)
+    whole = K.paged_attention(*dev, nq, nkv, d, 16, d ** -0.5, 0, span, batch=_Batch([1] * len(lens)), num_splits=1)
+    assert torch.equal(got, whole)
 
 
 @pytest.mark.parametrize("inner", [5124, 8960, 18944])
@@ -716,16 +793,21 @@ def test_linear_float32_of_a_matrix_that_was_just_made(K, rows, outputs, inner):
         assert torch.equal(got, K.linear(x, w.clone())), f"time {i}"
 
 
-@pytest.mark.parametrize("nq,nkv,d,lens", [
-    (14, 2, 64, [128 + 29 * i for i in range(64)]), (12, 2, 128, [128 + 6 * i for i in range(64)]), (8, 4, 64, [128 + 12 * i for i in range(32)]), (16, 8, 64, [20] * 18)])
-def test_short_contexts_are_not_cut_whatever_the_step_could_hold(K, nq, nkv, d, lens):
-    """A captured step is planned for the longest context there may be. Where the step's own are so short that a merge costs more than the
-    slices save, every token stays whole: the bits of a launch that cannot cut."""
-    span = 32768
-    qkv, kp, vp, table, tseq, pos = _attention_case(torch.bfloat16, nq, nkv, d, 16, lens, [1] * len(lens), 0, 5)
-    table = torch.nn.functional.pad(table, (0, span // 16 - table.shape[1]))
-    dev = [t.cuda() for t in (qkv, kp, vp, table, tseq, pos)]
-    got = K.paged_attention(*dev, nq, nkv, d, 16, d ** -0.5, 0, span, batch=_Batch([1] * len(lens)))
-    assert K._decode_balanced == len(lens)
-    whole = K.paged_attention(*dev, nq, nkv, d, 16, d ** -0.5, 0, span, batch=_Batch([1] * len(lens)), num_splits=1)
-    assert torch.equal(got, whole)
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("N,W,E,top,gates", [(1, 512, 8, 2, 0), (3, 1024, 16, 4, 2), (64, 1024, 64, 6, 0), (5, 2048, 128, 8, 1), (148, 896, 300, 2, 0), (149, 512, 18, 2, 0), (2, 300, 17, 3, 0)])
+def test_router_forms_agree(K, monkeypatch, dtype, N, W, E, top, gates):
+    """All pieces asked for at once or output by output, sixteen warps or eight (more rows than multiprocessors): the same sums in the same order."""
+    h, w = torch.randn(N, W, generator=torch.Generator().manual_seed(1)).to(dtype), torch.randn(E + gates, W, generator=torch.Generator().manual_seed(2)).to(dtype)
+    monkeypatch.setattr(K, "tc_max_rows", 1 << 20)
+    hd, wd = h.cuda(), w.cuda()
+    apart = torch.empty(w.numel() + 1, dtype=dtype, device="cuda")[1:].view_as(wd)   # not on a 16-byte boundary
+    apart.copy_(wd)
+    many = K.moe_router(hd.repeat(150, 1), wd, None, top, gates=gates)
+    outs = [K.moe_router(hd, wd, None, top, gates=gates), [o[:N] for o in many]]
+    with K.at_rest:
+        outs.append(K.moe_router(hd, wd, None, top, gates=gates))
+    for o in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(outs[0], o))
+    want = REF.moe_router(h, w, None, top, gates=gates)
+    for o in (outs[0], K.moe_router(hd, apart, None, top, gates=gates)):
+        close(o[1].sort().values, want[1].sort().values, 2e-5)   # (logits of a scale of 45: 32-bit sums of 2,048 products in another order)
