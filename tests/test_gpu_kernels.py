@@ -676,6 +676,11 @@ def test_decode_attention_dealt_out_in_every_form(K, monkeypatch, d, form):
     32-bit sums in another order, rounded to bfloat16 once (2^-8 of a result), as in the tests of the kernel's slices."""
     monkeypatch.setattr(K, "fuse_decode_rope_head_dims", (64, 128))
     monkeypatch.setattr(K, "deal_rounds", {64: 0, 128: 0})   # short requests are cut too where that saves a round
+
+    def clear():   # (sums that an engine left may have been made in inference mode)
+        with torch.inference_mode():
+            K._clear_dirty()
+
     nq, nkv, ps = 12, 2, 16
     lens = DEALT + [1, 1]
     n, span = len(lens), max(DEALT)
@@ -701,7 +706,7 @@ def test_decode_attention_dealt_out_in_every_form(K, monkeypatch, d, form):
 
         def run(how):
             pools[how] = (kp.cuda(), vp.cuda())
-            K._clear_dirty()
+            clear()
             return K.qkv_attention(x, w, bias, cos, sin, slots.cuda(), *pools[how], table, tseq, pos_d, nq, nkv, d, ps, scale, 0, span, batch=batch, write_kv=write)
     elif form == "window":
         dev = cu(qkv, kp, vp)
@@ -742,7 +747,7 @@ def test_decode_attention_dealt_out_in_every_form(K, monkeypatch, d, form):
         for a, b in zip(pools["whole"], pools["cut"]):
             own = [t.permute(0, 2, 1, 3).reshape(-1, nkv, d)[real.cuda()] for t in (a, b)]
             assert torch.equal(*own)
-    K._clear_dirty()
+    clear()
 
 
 @pytest.mark.parametrize("nq,nkv,d,lens", [
