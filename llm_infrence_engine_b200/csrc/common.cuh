@@ -53,6 +53,20 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return scratch[32];
 }
 
+// The sum over a block in every thread, at one barrier: the warps' sums meet in shared memory and every thread adds them up itself, in one
+// order. `buffer` (32 floats, 16-byte aligned) is another one than that of the sum before.
+template <int WARPS>
+__device__ __forceinline__ float quick_sum(float v, float* buffer) {
+    v = warp_sum(v);
+    if constexpr (WARPS == 1) return v;
+    if ((threadIdx.x & 31) == 0) buffer[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float t = buffer[0];
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w) t += buffer[w];
+    return t;
+}
+
 // 16-byte vector of storage elements, read as floats.
 template <typename T> struct Vec16;
 template <> struct Vec16<float> {

@@ -249,6 +249,53 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ residual, const T* __rest
     }
 }
 
+// The same for rows that fit a block's registers, 4 PER elements to a thread and 16 bytes to an access: everything is asked for at once (in the
+// loop above a second piece waits behind the first one's store) and the sum takes one barrier (decode steps: one row of 896
+// 2.0 -> 1.8 us, 64 rows of 1,536 3.2 -> 2.9).
+template <typename T, int WARPS, int PER>
+__global__ void __launch_bounds__(WARPS * 32) add_rmsnorm_held_kernel(float* __restrict__ residual, const T* __restrict__ delta, const float* __restrict__ weight,
+                                                                      T* __restrict__ out, const int* __restrict__ rows, int H, float eps) {
+    __shared__ __align__(16) float sums[32];
+    constexpr int STEP = WARPS * 32 * 4;
+    pdl_trigger();
+    float w[PER][4], v[PER][4], dv[PER][4];
+#pragma unroll
+    for (int n = 0; n < PER; ++n)   // the norm's weights do not depend on the kernel before
+        if (n * STEP + threadIdx.x * 4 < H) load4(weight + n * STEP + threadIdx.x * 4, w[n]);
+    pdl_wait();
+    const int r = rows ? rows[blockIdx.x] : blockIdx.x;
+    float* x = residual + (size_t)r * H;
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+        const int i = n * STEP + threadIdx.x * 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[n][j] = dv[n][j] = 0.f;
+        if (i < H) {
+            load4(x + i, v[n]);
+            if (delta) load4(delta + (size_t)r * H + i, dv[n]);
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+        const int i = n * STEP + threadIdx.x * 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { v[n][j] += dv[n][j]; ss += v[n][j] * v[n][j]; }
+        if (delta && !rows && i < H) store4(x + i, v[n]);
+    }
+    const float rstd = 1.0f / sqrtf(quick_sum<WARPS>(ss, sums) / (float)H + eps);
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+        const int i = n * STEP + threadIdx.x * 4;
+        if (i < H) {
+            float y[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[j] = w[n][j] * round_through<T>(v[n][j] * rstd);
+            store4(out + (size_t)blockIdx.x * H + i, y);
+        }
+    }
+}
+
 template <typename T>
 static int launch_add_rmsnorm(float* residual, const T* delta, const float* weight, T* out, const int* rows, int n_out, int H, float eps,
                               cudaStream_t s) {
@@ -258,6 +305,15 @@ static int launch_add_rmsnorm(float* residual, const T* delta, const float* weig
     const int per = vec ? 4 : 1;
     int threads = 32;
     while (threads < 512 && threads * per * 2 <= H) threads *= 2;
+    if (vec && (uintptr_t)out % 16 == 0 && (uintptr_t)delta % 16 == 0) {   // (by H alone otherwise: a row's bits do not depend on the step)
+#define LLMIE_HELD(WARPS, PER) return launch_kernel(add_rmsnorm_held_kernel<T, WARPS, PER>, dim3(n_out), dim3(WARPS * 32), 0, s, residual, delta, weight, out, rows, H, eps)
+        if (H <= 128) LLMIE_HELD(1, 1);
+        if (H <= 512) LLMIE_HELD(4, 1);
+        if (H <= 1024) LLMIE_HELD(4, 2);
+        if (H <= 2048) LLMIE_HELD(8, 2);
+        if (H <= 4096) LLMIE_HELD(16, 2);
+#undef LLMIE_HELD
+    }
     if (vec) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(add_rmsnorm_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         return launch_kernel(add_rmsnorm_kernel<T, 4>, dim3(n_out), dim3(threads), smem, s, residual, delta, weight, out, rows, H, eps);

@@ -1635,7 +1635,7 @@ class CudaKernels:
     def _dual_mix_now(self, add_to, a, b, weight_a, weight_b, eps, coef) -> None:
         N, H = add_to.shape
         self._check(self.lib.llmie_dual_rmsnorm_mix(_ptr(a), self._dt(a, "a"), _ptr(b), self._dt(b, "b"), _ptr(weight_a), _ptr(weight_b), _ptr(add_to),
-                                                    N, H, ctypes.c_float(eps), ctypes.c_float(coef), 1, int(self._clears(a)), int(self._clears(b)), self._stream()),
+                                                    N, H, ctypes.c_float(eps), ctypes.c_float(coef), 1, int(self._clears(a)), int(self._clears(b)), self._weights_at_rest(), self._stream()),
                     "dual_rmsnorm_mix")
         self._unfresh(add_to)
 

@@ -76,6 +76,85 @@ __global__ void streams_norm_kernel(float* __restrict__ xs, TY* __restrict__ y, 
     for (int c = threadIdx.x; c < H; c += blockDim.x) o[c] = from_f32<TO>(u_buf[c] * rstd * weight[c]);
 }
 
+// The same for up to four streams of rows that fit a block's registers, 4 PER channels of each stream to a thread and 16 bytes to an access: everything
+// is asked for at once, the parameters before the wait, and the sum of squares takes one barrier. Decoded tokens are bound by that chain,
+// prompt portions by the bytes (four streams in and out).
+// (Four streams of 896: four decoded tokens 3.7 -> 2.9 us, prompts of 1,977 tokens 22.5 -> 12.7.)
+template <typename TY, typename TO, int WARPS, int PER>
+__global__ void __launch_bounds__(WARPS * 32) streams_norm_held_kernel(float* __restrict__ xs, TY* __restrict__ y, int clear_y, const float* __restrict__ mix,
+                                                                       const float* __restrict__ coef_out, const float* __restrict__ coef_in,
+                                                                       const float* __restrict__ weight, TO* __restrict__ out, const int* __restrict__ rows,
+                                                                       int S, int H, float eps) {
+    constexpr int MAXS = 4, STEP = WARPS * 32 * 4;
+    __shared__ float sums[32], mix_s[MAXS * MAXS], out_s[MAXS];
+    pdl_trigger();
+    if (mix) {
+        if (threadIdx.x < S * S) mix_s[threadIdx.x] = mix[threadIdx.x];
+        if (threadIdx.x < S) out_s[threadIdx.x] = coef_out[threadIdx.x];
+    }
+    float in[MAXS], wt[PER][4];
+#pragma unroll
+    for (int k = 0; k < MAXS; ++k) in[k] = k < S ? coef_in[k] : 0.f;
+#pragma unroll
+    for (int n = 0; n < PER; ++n)
+        if (n * STEP + threadIdx.x * 4 < H) load4(weight + n * STEP + threadIdx.x * 4, wt[n]);
+    pdl_wait();
+    const int r = rows ? rows[blockIdx.x] : blockIdx.x;
+    float* base = xs + (size_t)r * S * H;
+    float x[PER][MAXS][4], u[PER][4];
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+        const int c = n * STEP + threadIdx.x * 4;
+        if (c < H) {
+#pragma unroll
+            for (int k = 0; k < MAXS; ++k)
+                if (k < S) load4(base + (size_t)k * H + c, x[n][k]);
+            if (y) load4(y + (size_t)r * H + c, u[n]);
+        }
+    }
+    __syncthreads();
+    float ss = 0.f;
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+        const int c = n * STEP + threadIdx.x * 4;
+        if (c < H) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float one[MAXS];
+#pragma unroll
+                for (int k = 0; k < MAXS; ++k) one[k] = k < S ? x[n][k][j] : 0.f;
+                if (y) mix_one<MAXS, TY>(one, u[n][j], mix_s, out_s, S);
+                float t = 0.f;
+#pragma unroll
+                for (int k = 0; k < MAXS; ++k)
+                    if (k < S) { x[n][k][j] = one[k]; t = fmaf(in[k], one[k], t); }
+                u[n][j] = t;
+                ss = fmaf(t, t, ss);
+            }
+            if (y) {
+                const float zero[4] = {0.f, 0.f, 0.f, 0.f};
+                if (clear_y) store4(y + (size_t)r * H + c, zero);
+                if (!rows) {
+#pragma unroll
+                    for (int k = 0; k < MAXS; ++k)
+                        if (k < S) store4(base + (size_t)k * H + c, x[n][k]);
+                }
+            }
+        }
+    }
+    ss = quick_sum<WARPS>(ss, sums);
+    const float rstd = 1.0f / sqrtf(ss / (float)H + eps);
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+        const int c = n * STEP + threadIdx.x * 4;
+        if (c < H) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) u[n][j] = u[n][j] * rstd * wt[n][j];
+            store4(out + (size_t)blockIdx.x * H + c, u[n]);
+        }
+    }
+}
+
 template <int MAXS, typename TY>
 __global__ void streams_update_kernel(float* __restrict__ xs, TY* __restrict__ y, int clear_y, const float* __restrict__ mix,
                                       const float* __restrict__ coef_out, int S, int H, long long total) {
@@ -115,6 +194,17 @@ __global__ void streams_expand_kernel(const float* __restrict__ x, float* __rest
 template <int MAXS, typename TY, typename TO>
 int launch_norm(float* xs, TY* y, int clear_y, const float* mix, const float* coef_out, const float* coef_in, const float* weight, TO* out,
                 const int* rows, int n_out, int S, int H, float eps, cudaStream_t s) {
+    if constexpr (MAXS == 4) {
+        if (H % 4 == 0 && H <= 2048 && (((uintptr_t)xs | (uintptr_t)y | (uintptr_t)weight | (uintptr_t)out) & 15) == 0) {
+#define LLMIE_HELD(WARPS, PER) \
+    return launch_kernel(streams_norm_held_kernel<TY, TO, WARPS, PER>, dim3(n_out), dim3(WARPS * 32), 0, s, xs, y, clear_y, mix, coef_out, coef_in, weight, out, rows, S, H, eps)
+            if (H <= 128) LLMIE_HELD(1, 1);
+            if (H <= 512) LLMIE_HELD(4, 1);
+            if (H <= 1024) LLMIE_HELD(8, 1);
+            LLMIE_HELD(16, 1);
+#undef LLMIE_HELD
+        }
+    }
     const size_t smem = sizeof(float) * ((size_t)H + 36 + S * S + 2 * S);
     if (smem > 200 * 1024) return LLMIE_ERR_BAD_ARGUMENT;
     if (smem > 48 * 1024) cudaFuncSetAttribute(streams_norm_kernel<MAXS, TY, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
