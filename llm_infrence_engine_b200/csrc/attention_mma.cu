@@ -69,6 +69,8 @@ struct Params {
     int chunk = 0;                     // > 0: only keys of the token's own run of `chunk` positions are seen
     float cap_log2 = 0.f;              // > 0: the soft cap times log2(e)
     float x_scale = 0.f;               // what a raw score is multiplied by: scale log2(e), or with a cap 2 scale log2(e) / cap
+    float temp_coef = 0.f;             // temp_every > 0: raw scores are multiplied by 1 + temp_coef ln(floor((pos + 1) / temp_every) + 1) as well
+    int temp_every = 0;
     const float* rel = nullptr;        // [rel_rows][nq] or null
     const int* rows_of = nullptr;      // [n_rows_of]
     int n_rows_of = 0, rel_rows = 0;
@@ -724,7 +726,7 @@ __global__ void __launch_bounds__(DW * 32, DW == 8 ? 1 : 2) attn_mma_decode_kern
     ExtTerms<BN> ext;
     float rel_last[2] = {0.f, 0.f};
     if constexpr (EXT) {
-        ext.x_scale = p.x_scale;
+        ext.x_scale = p.temp_every > 0 ? p.x_scale * (1.0f + p.temp_coef * logf((float)((pos0 + 1) / p.temp_every + 1))) : p.x_scale;
         ext.cap_log2 = p.cap_log2;
         ext.numbers = nullptr;
         if (p.rel) {
@@ -1176,7 +1178,7 @@ static int run_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* 
     if (extras) {
         p.chunk = extras->chunk; p.cap_log2 = extras->cap_log2; p.x_scale = extras->x_scale; p.rel = extras->rel; p.rows_of = extras->rows_of;
         p.n_rows_of = extras->n_rows_of; p.rel_rows = extras->rel_rows; p.gate = extras->gate; p.gate_stride = extras->gate_stride;
-        p.key_scale = extras->key_scale;
+        p.key_scale = extras->key_scale; p.temp_coef = extras->temp_coef; p.temp_every = extras->temp_every;
     }
     p.k_pool_w = const_cast<bf16*>(k_pool); p.v_pool_w = const_cast<bf16*>(v_pool);
     return d == 64 ? launch<64>(p, num_tiles, num_sms / nkv, decode_mode, s) : launch<128>(p, num_tiles, num_sms / nkv, decode_mode, s);
@@ -1195,12 +1197,13 @@ LLMIE_API int llmie_paged_attention_mma(const bf16* q, int q_stride, const bf16*
 
 // Decode steps (tile i is token i, at most 8 query heads per key/value head) with chunks, a soft cap, a bias by distance (rel [rel_rows][nq],
 // rows_of [n_rows_of]: distance -> row), a gate per head (gate + n * gate_stride), and, with key_scale [pages][page_size] and no v_pool, values
-// that are the keys; each off when its pointer is null or its number 0. four_warps as decode_mode 2.
+// that are the keys, and a query temperature by position; each off when its pointer is null or its number 0. four_warps as decode_mode 2.
 LLMIE_API int llmie_paged_attention_mma_ext(const bf16* q, int q_stride, const bf16* k_pool, const bf16* v_pool, const int* block_table, int max_blocks,
                                             const int* token_seq, const int* positions, int num_tokens, bf16* out, float* scratch_o, float* scratch_ml,
                                             int* counters, int nq, int nkv, int d, int page_size, float scale, int window, int num_splits, int cluster,
                                             int four_warps, int chunk, float softcap, const float* rel, const int* rows_of, int n_rows_of, int rel_rows,
-                                            const bf16* gate, int gate_stride, const float* key_scale, int balanced, int deal_rounds, int num_sms, cudaStream_t s) {
+                                            const bf16* gate, int gate_stride, const float* key_scale, float temp_coef, int temp_every, int balanced,
+                                            int deal_rounds, int num_sms, cudaStream_t s) {
     if (num_tokens <= 0) return 0;
     if (nkv <= 0 || nq / nkv > 8 || chunk < 0 || softcap < 0.f || scale == 0.f || (rel && (!rows_of || rel_rows < 1 || n_rows_of < 0)) ||
         (v_pool == nullptr) != (key_scale != nullptr))
@@ -1208,6 +1211,7 @@ LLMIE_API int llmie_paged_attention_mma_ext(const bf16* q, int q_stride, const b
     Params e;
     e.chunk = chunk; e.cap_log2 = softcap * LOG2E; e.x_scale = softcap > 0.f ? 2.f * LOG2E * scale / softcap : LOG2E * scale;
     e.rel = rel; e.rows_of = rows_of; e.n_rows_of = n_rows_of; e.rel_rows = rel_rows; e.gate = gate; e.gate_stride = gate_stride; e.key_scale = key_scale;
+    e.temp_coef = temp_coef; e.temp_every = temp_every;
     return run_mma(q, q_stride, k_pool, v_pool, block_table, max_blocks, token_seq, positions, nullptr, num_tokens, out, scratch_o, scratch_ml, counters,
                    nq, nkv, d, page_size, scale, window, num_splits, four_warps ? 2 : 1, cluster, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr,
                    nullptr, nullptr, nullptr, nullptr, balanced, deal_rounds, num_sms, s, &e);

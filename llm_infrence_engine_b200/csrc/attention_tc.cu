@@ -36,6 +36,10 @@
 // lies in shared memory as a table [distance][head of the group], in which the 64 biases of a row stand at a fixed stride. With SHARED
 // a chunk of keys is fetched once and is the B operand of both products (as it lies, K-major for the scores, MN-major for P V); both
 // rings' space is one ring, and a stage is free when its P V product is over; the tokens' numbers come with the keys by a plain bulk copy.
+// Keys that a window keeps at the request's start are chunks of their own in front of the tile's (those of them that the tile's own chunks do
+// not hold), and a query temperature is a factor of the row's scores. (On the mma.sync kernel these
+// mixers had before: heads of 128 with kept tokens, 2,048 tokens, 16 heads, 234 us, 67 here; heads of 64 with a temperature and a bias, four
+// prompts of 200 to 901 tokens, 72 and 47.)
 //
 // A launch follows a plan made once per step on the device (attn_tc_plan_kernel): which pieces of work there are (a tile,
 // or one slice of a long tile's keys, whose partial result the last slice merges), long pieces first.
@@ -91,6 +95,9 @@ struct TcParams {
     const float* log_r2;
     // EXT:
     int chunk;              // > 0: only keys of the row's own run of `chunk` positions are seen
+    int keep;               // keys [0, keep) stay visible when the window has passed them
+    float temp_coef;        // temp_every > 0: a row's raw scores are multiplied by 1 + temp_coef ln(floor((pos + 1) / temp_every) + 1)
+    int temp_every;
     float cap;              // > 0: scores are bounded by cap tanh(s / cap)
     float x_scale;          // what a raw score is multiplied by: scale log2(e), or with a cap 2 scale log2(e) / cap
     const float* rel;       // [rel_rows][nq] or null
@@ -177,6 +184,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // stages of the one ring where values are keys, and the bytes behind the ring(s) that the barriers may take
 template <int D> constexpr int SHARED_STAGES = D == 64 ? 6 : 4;
 constexpr int BARRIER_BYTES = 512;
+
+// How many chunks of kept keys go before a tile's own, which start at lo_al.
+__device__ __forceinline__ int kept_chunks(int keep, int lo_al) { return (min(keep, lo_al) + BN - 1) / BN; }
 
 template <int D, int KIND, bool SHARED>
 __global__ void __launch_bounds__(THREADS, 2) attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap tmap_k,
@@ -272,11 +282,16 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc_prefill_kernel(const __gri
     if (EXT && p.chunk > 0) lo = max(lo, pos0 / p.chunk * p.chunk);
     const int lo_al = lo / p.box_rows * p.box_rows;  // chunks start where a TMA box starts
     // this block's slice of the tile's chunks: [chunk0, chunk0 + chunks), empty for the later slices of a short tile
-    const int all_chunks = ntok > 0 ? (hi - lo_al + BN - 1) / BN : 0;
+    const int kept = (EXT && ntok > 0) ? kept_chunks(p.keep, lo_al) : 0;
+    const int all_chunks = ntok > 0 ? kept + (hi - lo_al + BN - 1) / BN : 0;
     const int per_split = (all_chunks + num_splits - 1) / num_splits;
     const int chunk0 = split * per_split;
     const int chunks = max(0, min(all_chunks, chunk0 + per_split) - chunk0);
     const int* table = p.block_table + (size_t)(ntok > 0 ? where.w : 0) * p.max_blocks;
+    const auto first_key = [&](int c) {   // of this block's chunk c
+        const int all = chunk0 + c;
+        return EXT && all < kept ? all * BN : lo_al + (all - kept) * BN;
+    };
 
     if (warp == 4) {
         // ---------------------------------------------------------------- producer
@@ -289,7 +304,7 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc_prefill_kernel(const __gri
         const int group = 1 << group_shift, my_box = lane & (boxes - 1);
         auto group_rows = [&](int g) {
             const int cc = (g << group_shift) + (lane >> box_shift);
-            const int key = lo_al + (chunk0 + cc) * BN + my_box * p.box_rows;
+            const int key = first_key(cc) + my_box * p.box_rows;
             const int page = (cc < chunks && key < hi) ? table[key / p.page_size] : 0;  // behind the sequence: any page, its keys are masked
             return (page * p.nkv + kvh) * p.page_size + key % p.page_size;
         };
@@ -440,6 +455,7 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc_prefill_kernel(const __gri
         }
         const float to_log2 = EXT ? 1.f : p.scale_log2;   // from the scores to units of log2 (EXT: they are)
         const int my_head = kvh * G + (row_ok ? row % G : 0);
+        const float x_scale = !EXT || p.temp_every <= 0 ? p.x_scale : p.x_scale * (1.0f + p.temp_coef * logf((float)((pos + 1) / p.temp_every + 1)));
         const float rel_last = (EXT && p.rel) ? LOG2E * p.rel[(size_t)(p.rel_rows - 1) * p.nq + my_head] : 0.f;
         const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
         const uint32_t o_addr = lane_base + S_BUFS * BN;
@@ -456,10 +472,11 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc_prefill_kernel(const __gri
         }
         for (int c = 0; c < chunks && ok; ++c) {
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            const int key0 = lo_al + (chunk0 + c) * BN;
+            const int key0 = first_key(c);
             // A chunk that every row of the tile sees in full needs no mask arithmetic (rows beyond the tile have zero
             // queries and collect numbers nobody reads). The scale is positive: the maximum is taken over the raw scores.
-            bool interior = key0 >= lo && key0 + BN - 1 <= pos0 && (p.window <= 0 || key0 > hi - 1 - p.window);
+            const bool before = EXT && chunk0 + c < kept;   // a chunk of kept keys
+            bool interior = !before && key0 >= lo && key0 + BN - 1 <= pos0 && (p.window <= 0 || key0 > hi - 1 - p.window);
             if (EXT && p.chunk > 0) interior = interior && (hi - 1) / p.chunk * p.chunk <= key0;
             if constexpr (EXT) {
                 // the row's 64 finished scores in units of log2: times the token's number, scaled, capped, biased by distance. (Columns the
@@ -472,7 +489,7 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc_prefill_kernel(const __gri
                 const int nearest = pos0 - (key0 + BN - 1), farthest = hi - 1 - key0;   // distances of the tile's rows to the chunk's keys
                 const bool in_table = p.rel && farthest < p.table, all_far = p.rel && nearest >= p.n_rows_of;
                 const float add = (p.cap > 0.f ? p.cap * LOG2E : 0.f) + (all_far ? rel_last : 0.f);
-                const uint64_t zero2 = pair_of(0.f, 0.f), x2 = pair_of(p.x_scale, p.x_scale), add2_ = pair_of(add, add);
+                const uint64_t zero2 = pair_of(0.f, 0.f), x2 = pair_of(x_scale, x_scale), add2_ = pair_of(add, add);
                 if (p.cap > 0.f) {
                     // cap tanh(v) = cap - 2 cap / (e^(2 v) + 1); an e^(2 v) beyond the largest number has the reciprocal zero, as it should
                     const float m2cap = -2.f * LOG2E * p.cap;
@@ -548,7 +565,12 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc_prefill_kernel(const __gri
                 int first = p.window > 0 ? max(pos - p.window + 1 - key0, 0) : 0;
                 if (EXT && p.chunk > 0) first = max(first, pos / p.chunk * p.chunk - key0);
                 const uint64_t upto = last < 0 ? 0ull : (last >= 63 ? ~0ull : ((1ull << (last + 1)) - 1ull));
-                const uint64_t seen = first >= 64 ? 0ull : upto & ~((1ull << first) - 1ull);
+                uint64_t seen = first >= 64 ? 0ull : upto & ~((1ull << first) - 1ull);
+                if (EXT && p.keep > 0) {
+                    const int kept_here = (before ? min(p.keep, lo_al) : p.keep) - key0;
+                    const uint64_t early = kept_here <= 0 ? 0ull : (kept_here >= 64 ? ~0ull : ((1ull << kept_here) - 1ull));
+                    seen = before ? upto & early : seen | (upto & early);
+                }
                 const uint32_t seen_lo = (uint32_t)seen, seen_hi = (uint32_t)(seen >> 32);
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
@@ -800,7 +822,7 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc_prefill_kernel(const __gri
 constexpr int MIN_SLICE = 8, SLICE_COST = 8, MAX_SLICES = 16, PLAN_THREADS = 256;
 
 __global__ void __launch_bounds__(PLAN_THREADS) attn_tc_plan_kernel(const int* __restrict__ tile_info, int num_tiles, const int* __restrict__ positions,
-                                                                    const int* __restrict__ token_seq, int window, int chunk, int box_rows, int capacity, int fixed_splits, int max_items,
+                                                                    const int* __restrict__ token_seq, int window, int chunk, int keep, int box_rows, int capacity, int fixed_splits, int max_items,
                                                                     int* __restrict__ work, int* __restrict__ tmp) {
     pdl_trigger();
     pdl_wait();
@@ -818,7 +840,8 @@ __global__ void __launch_bounds__(PLAN_THREADS) attn_tc_plan_kernel(const int* _
             const int pos0 = positions[n0], hi = pos0 + ntok;
             int lo = window > 0 ? max(0, pos0 - window + 1) : 0;
             if (chunk > 0) lo = max(lo, pos0 / chunk * chunk);
-            c = (hi - lo / box_rows * box_rows + BN - 1) / BN;
+            const int lo_al = lo / box_rows * box_rows;
+            c = kept_chunks(keep, lo_al) + (hi - lo_al + BN - 1) / BN;
         }
         chunks[t] = c;
         longest = max(longest, c);
@@ -890,13 +913,13 @@ __global__ void __launch_bounds__(PLAN_THREADS) attn_tc_plan_kernel(const int* _
 
 // The plan for llmie_paged_attention_tc (see attn_tc_plan_kernel): work [8 * max_items + 1] receives the pieces and their number,
 // tmp [3 * num_tiles] is scratch. capacity: pieces that can run at once. max_items >= num_tiles * max(1, fixed_splits).
-LLMIE_API int llmie_attn_tc_plan(const int* tile_info, int num_tiles, const int* positions, const int* token_seq, int window, int chunk, int page_size,
+LLMIE_API int llmie_attn_tc_plan(const int* tile_info, int num_tiles, const int* positions, const int* token_seq, int window, int chunk, int keep, int page_size,
                                  int capacity, int fixed_splits, int max_items, int* work, int* tmp, cudaStream_t s) {
     if (num_tiles <= 0) return 0;
-    if (!tile_info || !positions || !token_seq || !work || !tmp || page_size <= 0 || capacity <= 0 || fixed_splits < 0 || fixed_splits > MAX_SLICES ||
+    if (!tile_info || !positions || !token_seq || !work || !tmp || page_size <= 0 || capacity <= 0 || fixed_splits < 0 || fixed_splits > MAX_SLICES || keep < 0 ||
         max_items < (long long)num_tiles * (fixed_splits > 0 ? fixed_splits : 1) || ((uintptr_t)work & 15))
         return LLMIE_ERR_BAD_ARGUMENT;
-    return launch_kernel(attn_tc_plan_kernel, dim3(1), dim3(PLAN_THREADS), 0, s, tile_info, num_tiles, positions, token_seq, window, chunk,
+    return launch_kernel(attn_tc_plan_kernel, dim3(1), dim3(PLAN_THREADS), 0, s, tile_info, num_tiles, positions, token_seq, window, chunk, keep,
                          page_size < BN ? page_size : BN, capacity, fixed_splits, max_items, work, tmp);
 }
 
@@ -911,9 +934,10 @@ LLMIE_API int llmie_paged_attention_tc(const bf16* q, int q_stride, const bf16* 
                                        float* scratch_ml, int* counters, int nq, int nkv, int d, int page_size, float scale, int window,
                                        int* error_flag, const float* turn_cos, const float* turn_sin, const float* sig_bias, const float* log_r1,
                                        const float* log_r2, int chunk, float softcap, const float* rel, const int* rows_of, int n_rows_of, int rel_rows,
-                                       const bf16* gate, int gate_stride, const float* key_scale, cudaStream_t s) {
+                                       const bf16* gate, int gate_stride, const float* key_scale, int keep, float temp_coef, int temp_every, cudaStream_t s) {
     if (num_tiles <= 0) return 0;
-    const bool ext = chunk > 0 || softcap > 0.f || rel || gate || key_scale;
+    const bool ext = chunk > 0 || softcap > 0.f || rel || gate || key_scale || keep > 0 || temp_every > 0;
+    if (keep < 0 || (keep > 0 && window <= 0)) return LLMIE_ERR_BAD_ARGUMENT;
     if ((ext && (sig_bias || turn_cos)) || (rel && (!rows_of || rel_rows < 1 || n_rows_of < 0)) || (v_pool == nullptr) != (key_scale != nullptr) ||
         ((uintptr_t)key_scale & 15) || (!ext && !(scale > 0.f)))
         return LLMIE_ERR_BAD_ARGUMENT;
@@ -931,6 +955,7 @@ LLMIE_API int llmie_paged_attention_tc(const bf16* q, int q_stride, const bf16* 
     p.q_stride = q_stride; p.max_blocks = max_blocks; p.nq = nq; p.nkv = nkv; p.page_size = page_size; p.num_tiles = num_tiles;
     p.window = window; p.box_rows = page_size < BN ? page_size : BN; p.scale_log2 = scale * LOG2E;
     p.turn_cos = turn_cos; p.turn_sin = turn_sin; p.sig_bias = sig_bias; p.log_r1 = log_r1; p.log_r2 = log_r2;
+    p.keep = keep; p.temp_coef = temp_coef; p.temp_every = temp_every;
     p.chunk = chunk; p.cap = softcap; p.x_scale = softcap > 0.f ? 2.f * LOG2E * scale / softcap : LOG2E * scale;
     p.rel = rel; p.rows_of = rows_of; p.n_rows_of = n_rows_of; p.rel_rows = rel_rows; p.table = 0; p.rows_s = 0;
     p.gate = gate; p.gate_stride = gate_stride; p.key_scale = key_scale;

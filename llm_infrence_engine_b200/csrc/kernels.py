@@ -705,7 +705,7 @@ class CudaKernels:
 
     def _attention_tc(self, qkv, k_pool, v_pool, block_table, token_seq, positions, out, num_heads, num_kv_heads, head_dim,
                       page_size, scale, window, span, batch, num_splits, turn=None, sigmoid_bias=None, log_distance=None, chunk=0, softcap=0.0,
-                      rel=None, rel_rows=None, gate=None, gate_col=0, key_scale=None):
+                      rel=None, rel_rows=None, gate=None, gate_col=0, key_scale=None, keep_first=0, temp=(0.0, 0)):
         """The tcgen05 kernel for prompt portions, if it takes this case: returns ``out`` or None. (The extras: see ``attention_ext``; the
         gate is one per head.)"""
         group = num_heads // num_kv_heads
@@ -720,17 +720,17 @@ class CudaKernels:
         # long tiles into slices, as many pieces as fit on the device at once, and starts long pieces first.
         fixed = int(num_splits or 0)
         capacity = max(1, 2 * self.num_sms // num_kv_heads)   # two blocks per SM
-        if chunk or softcap or rel is not None or key_scale is not None:
+        if chunk or softcap or rel is not None or key_scale is not None or temp[1]:
             # a chunk with these extras takes half as long again, so a slice weighs less against it: more, shorter pieces than fit at
             # once (the long ones start first, the short ones fill the gaps)
             capacity = capacity * self.tc_ext_pieces // 4
         # (tiles of up to 16 chunks are never cut: a slice costs about 8 chunks' time and is at least 8 chunks long)
         max_items = tiles * fixed if fixed else max(tiles, min(capacity, 16 * tiles)) if span > 16 * 64 else tiles
-        key = ("tcgen05 attention plan", group, num_kv_heads, page_size, int(window), int(chunk), fixed)
+        key = ("tcgen05 attention plan", group, num_kv_heads, page_size, int(window), int(chunk), int(keep_first), fixed)
         if key not in batch._tables:
             work = torch.empty((8 * max_items + 4,), dtype=torch.int32, device=qkv.device)
             tmp = torch.empty((3 * tiles,), dtype=torch.int32, device=qkv.device)
-            self._check(self.lib.llmie_attn_tc_plan(_ptr(tile_info), tiles, _ptr(positions), _ptr(token_seq), int(window), int(chunk), page_size, capacity, fixed,
+            self._check(self.lib.llmie_attn_tc_plan(_ptr(tile_info), tiles, _ptr(positions), _ptr(token_seq), int(window), int(chunk), int(keep_first), page_size, capacity, fixed,
                                                     max_items, _ptr(work), _ptr(tmp), self._stream()), "attention plan (tcgen05)")
             batch._tables[key] = (work, tmp)
         work = batch._tables[key][0]
@@ -746,7 +746,7 @@ class CudaKernels:
             ctypes.c_float(scale), int(window), _ptr(self._errors(qkv.device)), *self._turn_and_sigmoid(turn, sigmoid_bias, log_distance),
             int(chunk), ctypes.c_float(softcap), _ptr(rel), _ptr(rel_rows), 0 if rel_rows is None else rel_rows.shape[0], 0 if rel is None else rel.shape[0],
             ctypes.c_void_p(0 if gate is None else gate.data_ptr() + gate_col * gate.element_size()), 0 if gate is None else gate.shape[1], _ptr(key_scale),
-            self._stream()), "paged_attention (tcgen05)")
+            int(keep_first), ctypes.c_float(temp[0]), int(temp[1]), self._stream()), "paged_attention (tcgen05)")
         return out
 
     @staticmethod
@@ -1203,11 +1203,11 @@ class CudaKernels:
             if done is not None:
                 return done
         if (self.use_tc_attention_ext and dt == 1 and batch is not None and head_dim == v_head_dim and q_col == 0 and q.shape[1] % 8 == 0
-                and not (keep_first or temp[1]) and sink is None and gate_mode != 2 and log_distance is None and sigmoid_bias is None and turn is None
+                and sink is None and gate_mode != 2 and log_distance is None and sigmoid_bias is None and turn is None
                 and (v_pool is None) == (key_scale is not None)):
             span = min(max_context, window or max_context, chunk or max_context)
             group = num_heads // num_kv_heads
-            if batch.max_seq_len == 1 and group <= 8 and head_dim in (64, 128) and scale != 0 and self.use_mma_attention:
+            if (batch.max_seq_len == 1 and group <= 8 and head_dim in (64, 128) and scale != 0 and self.use_mma_attention and not keep_first):
                 # single tokens: the decode kernel of plain attention
                 n_splits, cluster, scratch_o, scratch_ml, counters = self._decode_plan(N, num_kv_heads, head_dim, span, num_splits, q.device)
                 self._check(self.lib.llmie_paged_attention_mma_ext(
@@ -1216,11 +1216,11 @@ class CudaKernels:
                     n_splits, cluster, int(self._decode_four_warps), int(chunk), ctypes.c_float(softcap), _ptr(rel), _ptr(rel_rows),
                     0 if rel_rows is None else rel_rows.shape[0], 0 if rel is None else rel.shape[0],
                     ctypes.c_void_p(0 if gate is None else gate.data_ptr() + gate_col * esize), 0 if gate is None else gate.shape[1], _ptr(key_scale),
-                    self._decode_balanced, self.deal_rounds.get(head_dim, 0), self.num_sms, self._stream()), "attention_ext (decode, tensor cores)")
+                    ctypes.c_float(temp[0]), int(temp[1]), self._decode_balanced, self.deal_rounds.get(head_dim, 0), self.num_sms, self._stream()), "attention_ext (decode, tensor cores)")
                 return out
             done = self._attention_tc(q, k_pool, v_pool, block_table, token_seq, positions, out, num_heads, num_kv_heads, head_dim, page_size, scale,
                                       int(window), span, batch, num_splits, chunk=chunk, softcap=softcap, rel=rel, rel_rows=rel_rows, gate=gate, gate_col=gate_col,
-                                      key_scale=key_scale)
+                                      key_scale=key_scale, keep_first=keep_first, temp=temp)
             if done is not None:
                 return done
         max_rows = 0
