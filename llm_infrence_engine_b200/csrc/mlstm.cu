@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(ML_THREADS + 32) mlstm_scan_kernel(const T* __
     const int C = DV + 1;                 // the last column is the normaliser
     const int s0 = seq_starts[r], s1 = seq_starts[r + 1];
     const int slot = seq_slots[r];
+    if (s1 - s0 < ML_TILE) pdl_trigger();   // (a short walk: the kernel behind may move in and set up)
     if (threadIdx.x >= ML_THREADS) {      // the warp of the gates
         const int lane = threadIdx.x - ML_THREADS;
         float m_carry = before[(size_t)r * H + h];

@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(const T* __res
     const int g = h / (H / G);
     const bool vec = (D & 3) == 0;
     const int s0 = seq_starts[r], s1 = seq_starts[r + 1];
+    if (s1 - s0 < SCAN_TILE) pdl_trigger();   // (a short walk: the kernel behind may move in and set up; see the end)
     float* st = state + ((size_t)seq_slots[r] * H + h) * DV * D;
     float2 S[CPL][P2];
 #pragma unroll
@@ -570,6 +571,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssm_scan_kernel(const T* __restr
     const float rate = FIXED ? A_log[h] : expf(A_log[h]), bias = FIXED ? 0.f : dt_bias[h], skip = FIXED ? 0.f : Dskip[h];
     pdl_wait();
     const int s0 = seq_starts[r], s1 = seq_starts[r + 1];
+    if (s1 - s0 < SCAN_TILE) pdl_trigger();   // (a short walk: see the delta rule's kernel)
     float* st = state + ((size_t)seq_slots[r] * H + h) * DV * NS;
     float2 S[CPL][P2];
 #pragma unroll
@@ -757,6 +759,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const T* _
     pdl_wait();
     const float bias = stage_c < C ? dt_bias[stage_c] : 0.f;
     const int s0 = seq_starts[r], s1 = seq_starts[r + 1];
+    if (s1 - s0 < SCAN_TILE) pdl_trigger();   // (a short walk: see the delta rule's kernel)
     float* st = state + ((size_t)seq_slots[r] * C + (live ? col : 0)) * NS;
     float S[DPL];
     load_column<DPL, PARTS>(S, st, part, NS, live, vec);
@@ -984,13 +987,13 @@ LLMIE_API int llmie_causal_conv(const void* z, int z_stride, int C, const float*
         return LLMIE_ERR_BAD_ARGUMENT;
     if (dtype == DT_F32)
         return launch_conv<float>((const float*)z, z_stride, C, w, bias, state, seq_starts, seq_slots, (float*)out, out_stride, taps, act, R, max_rows, s);
-    return launch_conv<bf16>((const bf16*)z, z_stride, C, w, bias, state, seq_starts, seq_slots, (bf16*)out, out_stride, taps, act, R, max_rows, s);
-}
-
     if (taps == 4 && max_rows > 1 && C % 4 == 0 && z_stride % 4 == 0 && out_stride % 4 == 0 && (((uintptr_t)z | (uintptr_t)out) & 7) == 0 &&
         (((uintptr_t)w | (uintptr_t)bias | (uintptr_t)state) & 15) == 0)
         return launch_kernel(causal_conv4_kernel, dim3((C / 4 + 127) / 128, (max_rows + CONV_CHUNK - 1) / CONV_CHUNK, R), dim3(128), 0, s, (const bf16*)z,
                              z_stride, C, w, bias, state, seq_starts, seq_slots, (bf16*)out, out_stride, act);
+    return launch_conv<bf16>((const bf16*)z, z_stride, C, w, bias, state, seq_starts, seq_slots, (bf16*)out, out_stride, taps, act, R, max_rows, s);
+}
+
 LLMIE_API int llmie_delta_prepare(const void* qkv, int qkv_stride, int q_col, int k_col, const void* a, int a_stride, const void* b,
                                   int b_stride, const float* A_log, const float* dt_bias, float* qn, float* kn, float* kq, float* decay,
                                   float* beta, int N, int H, int G, int D, float q_scale, float unit_eps, int per_head, int dtype, cudaStream_t s) {
