@@ -471,8 +471,7 @@ LLMIE_API int llmie_paged_attention_ext_fa(const bf16* q, int q_stride, const bf
     else rc = launch<8, 8>(P, grid, smem, s);
     if (rc) return rc;
     if (num_splits > 1) {
-        attn_ext::attn_ext_combine_kernel<bf16><<<N * nq, 128, 0, s>>>(P.part_acc, P.part_ml, out, nq, dv, num_splits, P.ex);
-        rc = launch_status();
+        rc = attn_ext::launch_combine<bf16>(P.part_acc, P.part_ml, out, (long long)N * nq, nq, dv, num_splits, P.ex, s);
     }
     return rc;
 }

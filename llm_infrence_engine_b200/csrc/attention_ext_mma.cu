@@ -79,8 +79,7 @@ LLMIE_API int llmie_paged_attention_ext_mma(const bf16* q, int q_stride, const b
            : kind == attn_ext::MASKS ? launch_masks(P, grid, smem, s, R, deep) : launch_plain(P, grid, smem, s, R, deep);
     if (rc) return rc;
     if (num_splits > 1) {
-        attn_ext::attn_ext_combine_kernel<bf16><<<N * nq, 128, 0, s>>>(P.part_acc, P.part_ml, out, nq, dv, num_splits, P.ex);
-        rc = launch_status();
+        rc = attn_ext::launch_combine<bf16>(P.part_acc, P.part_ml, out, (long long)N * nq, nq, dv, num_splits, P.ex, s);
     }
     return rc;
 }

@@ -47,6 +47,8 @@ __global__ void __launch_bounds__(TALK_THREADS) paged_attn_talk_kernel(
     const int n = blockIdx.x, split = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int G = nq / nkv;
+    pdl_trigger();
+    pdl_wait();
     const int p = positions[n];
     const int lo = attn_ext::first_visible(p, window, ex);
     const int kept = min(ex.keep_first, lo);
@@ -311,16 +313,11 @@ int paged_attention_talk(const T* q, int q_stride, const T* k_pool, const T* v_p
     if (smem > 48 * 1024) cudaFuncSetAttribute(paged_attn_talk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     float* part_acc = scratch;
     float* part_ml = scratch ? scratch + (size_t)N * nq * num_splits * dv : nullptr;
-    paged_attn_talk_kernel<T><<<dim3(N, num_splits), TALK_THREADS, smem, s>>>(q, q_stride, k_pool, v_pool, block_table, max_blocks, token_seq, positions,
-                                                                               talk, out, part_acc, part_ml, nq, nkv, dk, dv, page_size, scale, window,
-                                                                               num_splits, slice_keys, vec_ok, v_chunk, ex);
-    int rc = launch_status();
-    if (rc) return rc;
-    if (num_splits > 1) {
-        attn_ext::attn_ext_combine_kernel<T><<<N * nq, 128, 0, s>>>(part_acc, part_ml, out, nq, dv, num_splits, ex);
-        rc = launch_status();
-    }
-    return rc;
+    const int rc = launch_kernel(paged_attn_talk_kernel<T>, dim3(N, num_splits), dim3(TALK_THREADS), smem, s, q, q_stride, k_pool, v_pool, block_table,
+                                 max_blocks, token_seq, positions, talk, out, part_acc, part_ml, nq, nkv, dk, dv, page_size, scale, window, num_splits,
+                                 slice_keys, vec_ok, v_chunk, ex);
+    if (rc || num_splits <= 1) return rc;
+    return attn_ext::launch_combine<T>(part_acc, part_ml, out, (long long)N * nq, nq, dv, num_splits, ex, s);
 }
 
 }  // namespace
