@@ -12,8 +12,11 @@
 //      registers over all chunks.
 //
 // Cap and exponentials take the fast forms here (this kernel serves bfloat16 only, where the weights are rounded to 8 bits anyway; the
-// 32-bit path never comes this way). A tile walks all keys up to its last token's position itself (no slices, no merge); sink and gate per head close a row. Only the
-// causal mask; sizes the form does not take (see llmie_attention_talk_mma_fits) go to the CUDA-core kernel.
+// 32-bit path never comes this way). A warp's chunk is one chain (copies, scores, a barrier, the mix, exponentials, products), so the keys of long
+// requests are cut into slices of `slice_chunks` chunks, a block each, whose partial results the merge kernel of the attention with extras
+// adds up (one slice: sink and gate per head close a row here). NQ: the number of heads where it is 8 or 16 (the matrix's row of a thread's
+// head then stays in registers), else 0. (Prompts of 700 and
+// 1,301 tokens, 8 heads over 2: one block to a tile and the mix in a loop 402 us, 129 with slices and the merge.) Only the causal mask; sizes the form does not take (see llmie_attention_talk_mma_fits) go to the CUDA-core kernel.
 #include "attention_ext.cuh"
 
 namespace {
@@ -54,14 +57,17 @@ struct TalkParams {
     int nq, nkv, dk, page_size;
     float scale;
     attn_ext::Extras ex;
+    int slice_chunks, num_slices;   // num_slices > 1: block y takes the chunks from y * slice_chunks on and leaves its part
+    float* part_acc;                // [rows][nq][num_slices][dv]
+    float* part_ml;                 // [rows][nq][num_slices][2]
 };
 
 // NV: pairs of n8 tiles over the value entries (dv = 16 NV)
-template <int NV>
+template <int NV, int NQ>
 __global__ void __launch_bounds__(256) attn_talk_mma_kernel(const TalkParams P) {
     extern __shared__ __align__(16) unsigned char tm_smem[];
     constexpr int dv = 16 * NV, vs = dv + 8;
-    const int nq = P.nq, nkv = P.nkv, dk = P.dk, ks = dk + 8;
+    const int nq = NQ ? NQ : P.nq, nkv = P.nkv, dk = P.dk, ks = dk + 8;
     const int Gs = nq / nkv, TT = 16 / Gs;
     const int nqp = (nq + 3) & ~3;
     bf16* Qs = reinterpret_cast<bf16*>(tm_smem);                       // [nkv][16][ks]: row (token, head of the group) of key/value head kvh
@@ -79,7 +85,16 @@ __global__ void __launch_bounds__(256) attn_talk_mma_kernel(const TalkParams P) 
     const int threads = nkv * 32;
     const int n0 = P.tile_info[2 * blockIdx.x], nt = P.tile_info[2 * blockIdx.x + 1];   // nt <= TT tokens from row n0
     const int* table = P.block_table + (size_t)P.token_seq[n0] * P.max_blocks;
-    const int p_last = P.positions[n0 + nt - 1];
+    const int first_key = blockIdx.y * P.slice_chunks * TM_KEYS;
+    const int p_last = min(P.positions[n0 + nt - 1], P.num_slices > 1 ? first_key + P.slice_chunks * TM_KEYS - 1 : 0x7fffffff);
+    if (first_key > p_last) {   // nothing of this slice is seen: the merge skips a part whose maximum is -inf
+        for (int i = tid; i < nt * nq; i += threads) {
+            float* ml = P.part_ml + (((size_t)n0 * nq + i) * P.num_slices + blockIdx.y) * 2;
+            ml[0] = -INFINITY;
+            ml[1] = 0.f;
+        }
+        return;
+    }
 
     for (int i = tid; i < nkv * 16 * (dk / 8); i += threads) {
         const int row = i / (dk / 8), c = (i % (dk / 8)) * 8;
@@ -144,11 +159,16 @@ __global__ void __launch_bounds__(256) attn_talk_mma_kernel(const TalkParams P) 
             }
         cp_commit_();
     };
-    place_rows(0);
+    float mix0[NQ ? NQ : 1], mix1[NQ ? NQ : 1];   // the matrix's rows of the thread's two heads
+    place_rows(first_key);
     __syncthreads();
-    fetch_keys(0);
-    fetch_values(0);
-    for (int c0 = 0; c0 <= p_last; c0 += TM_KEYS) {
+    if constexpr (NQ > 0) {
+#pragma unroll
+        for (int g = 0; g < NQ; ++g) { mix0[g] = tmx[h0 * nqp + g]; mix1[g] = tmx[h1 * nqp + g]; }
+    }
+    fetch_keys(first_key);
+    fetch_values(first_key);
+    for (int c0 = first_key; c0 <= p_last; c0 += TM_KEYS) {
         cp_wait_one();     // this chunk's keys have landed (its values may still be on their way)
         __syncthreads();   // ... for everyone (and, the first time, the queries and the matrix are in place)
 
@@ -195,6 +215,14 @@ __global__ void __launch_bounds__(256) attn_talk_mma_kernel(const TalkParams P) 
                     const float* src = sS + (size_t)t * stok + key * srow;
                     const float* mr = tmx + (size_t)h * nqp;
                     float a = 0.f;
+                    if constexpr (NQ > 0) {
+#pragma unroll
+                        for (int g = 0; g < NQ; g += 4) {
+                            const float4 sv = *reinterpret_cast<const float4*>(src + g);
+                            const float* mv = i < 2 ? mix0 + g : mix1 + g;
+                            a = fmaf(mv[0], sv.x, a); a = fmaf(mv[1], sv.y, a); a = fmaf(mv[2], sv.z, a); a = fmaf(mv[3], sv.w, a);
+                        }
+                    } else
                     for (int g = 0; g < nqp; g += 4) {
                         const float4 sv = *reinterpret_cast<const float4*>(src + g), mv = *reinterpret_cast<const float4*>(mr + g);
                         a = fmaf(mv.x, sv.x, a); a = fmaf(mv.y, sv.y, a); a = fmaf(mv.z, sv.z, a); a = fmaf(mv.w, sv.w, a);
@@ -253,6 +281,14 @@ __global__ void __launch_bounds__(256) attn_talk_mma_kernel(const TalkParams P) 
         const int t = half ? t1 : t0, h = half ? h1 : h0;
         if (t >= nt) continue;
         const int n = n0 + t;
+        if (P.num_slices > 1) {
+            const size_t slot = ((size_t)n * nq + h) * P.num_slices + blockIdx.y;
+            float* part = P.part_acc + slot * dv + 2 * qd;
+#pragma unroll
+            for (int j = 0; j < 2 * NV; ++j) *reinterpret_cast<float2*>(part + j * 8) = make_float2(O[j][2 * half], O[j][2 * half + 1]);
+            if (qd == 0) { P.part_ml[slot * 2] = half ? m1 : m0; P.part_ml[slot * 2 + 1] = half ? l1 : l0; }
+            continue;
+        }
         const bf16* gate_row = P.ex.gate_mode ? reinterpret_cast<const bf16*>(P.ex.gate) + (size_t)n * P.ex.gate_stride : nullptr;
         const float f = attn_ext::finish_scale<bf16>(half ? m1 : m0, half ? l1 : l0, P.ex, h, gate_row);
         bf16* o = P.out + ((size_t)n * nq + h) * dv + 2 * qd;
@@ -268,11 +304,17 @@ size_t talk_mma_smem(int nq, int nkv, int dk, int dv) {
            sizeof(float) * ((size_t)TT * (TM_KEYS * (nqp + 4) + 4) + (size_t)nq * nqp) + sizeof(int) * TM_KEYS;
 }
 
+template <int NV, int NQ>
+int launch_talk_as(const TalkParams& P, int tiles, size_t smem, cudaStream_t s) {
+    if (smem > 48 * 1024) cudaFuncSetAttribute(attn_talk_mma_kernel<NV, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    attn_talk_mma_kernel<NV, NQ><<<dim3(tiles, P.num_slices), P.nkv * 32, smem, s>>>(P);
+    return launch_status();
+}
 template <int NV>
 int launch_talk_mma(const TalkParams& P, int tiles, size_t smem, cudaStream_t s) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(attn_talk_mma_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attn_talk_mma_kernel<NV><<<tiles, P.nkv * 32, smem, s>>>(P);
-    return launch_status();
+    if (P.nq == 8) return launch_talk_as<NV, 8>(P, tiles, smem, s);
+    if (P.nq == 16) return launch_talk_as<NV, 16>(P, tiles, smem, s);
+    return launch_talk_as<NV, 0>(P, tiles, smem, s);
 }
 
 }  // namespace
@@ -290,11 +332,13 @@ LLMIE_API int llmie_attention_talk_mma_fits(int nq, int nkv, int dk, int dv) {
 
 // tile_info [tiles, 2]: (first row, rows) of tiles of up to llmie_attention_talk_mma_fits(...) consecutive rows of one request. q: nq heads
 // of dk from the rows' start (16-byte aligned, row stride a multiple of 8); gate: one number per head in rows of gate_stride, or null.
+// num_slices > 1: keys in slices of slice_chunks * 32, merged by a second kernel; scratch: rows * nq * num_slices * (dv + 2) floats.
 LLMIE_API int llmie_paged_attention_talk_mma(const bf16* q, int q_stride, const bf16* k_pool, const bf16* v_pool, const int* block_table, int max_blocks,
                                              const int* token_seq, const int* positions, const int* tile_info, int tiles, const float* talk, bf16* out,
                                              int nq, int nkv, int dk, int dv, int page_size, float scale, const float* sink, const bf16* gate,
-                                             int gate_stride, float softcap, cudaStream_t s) {
+                                             int gate_stride, float softcap, int rows, int slice_chunks, int num_slices, float* scratch, cudaStream_t s) {
     if (tiles <= 0) return 0;
+    if (num_slices < 1 || num_slices > 65535 || slice_chunks < 1 || (num_slices > 1 && (!scratch || ((uintptr_t)scratch & 15)))) return LLMIE_ERR_BAD_ARGUMENT;
     if (!llmie_attention_talk_mma_fits(nq, nkv, dk, dv) || !v_pool || ((uintptr_t)q & 15) || q_stride % 8 || ((uintptr_t)k_pool & 15) ||
         ((uintptr_t)v_pool & 15) || page_size <= 0)
         return LLMIE_ERR_BAD_ARGUMENT;
@@ -305,8 +349,10 @@ LLMIE_API int llmie_paged_attention_talk_mma(const bf16* q, int q_stride, const 
     P.ex.temp_coef = 0.f; P.ex.temp_every = 0; P.ex.rel = nullptr; P.ex.rows_of = nullptr; P.ex.n_rows_of = 0; P.ex.rel_rows = 0;
     P.ex.sink = sink; P.ex.gate = gate; P.ex.gate_stride = gate_stride; P.ex.gate_mode = gate ? 1 : 0;
     P.ex.keep_first = 0; P.ex.chunk = 0; P.ex.softcap = softcap;
+    P.slice_chunks = slice_chunks; P.num_slices = num_slices;
+    P.part_acc = scratch; P.part_ml = scratch ? scratch + (size_t)rows * nq * num_slices * dv : nullptr;
     const size_t smem = talk_mma_smem(nq, nkv, dk, dv);
-    if (dv == 32) return launch_talk_mma<2>(P, tiles, smem, s);
-    if (dv == 64) return launch_talk_mma<4>(P, tiles, smem, s);
-    return launch_talk_mma<8>(P, tiles, smem, s);
+    const int rc = dv == 32 ? launch_talk_mma<2>(P, tiles, smem, s) : (dv == 64 ? launch_talk_mma<4>(P, tiles, smem, s) : launch_talk_mma<8>(P, tiles, smem, s));
+    if (rc || num_slices == 1) return rc;
+    return attn_ext::launch_combine<bf16>(P.part_acc, P.part_ml, out, (long long)rows * nq, nq, dv, num_slices, P.ex, s);
 }

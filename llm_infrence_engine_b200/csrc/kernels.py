@@ -76,6 +76,8 @@ class CudaKernels:
         self.use_cluster_gate_up = False  # ... by pairs of blocks that share their weight rows (TMA multicast within a cluster of two)
         self.use_pair_gate_up = True     # ... by pairs of multiprocessors on tiles of 256 rows (tcgen05 cta_group::2) ...
         self.pair_gate_up_min_rows = 1024  # ... from this many rows on (measured: 3 to 8 % faster at 2,048 rows, 5 % slower at 512)
+        self.short_talk_slices = True
+        self.talk_slice_chunks = 8     # heads that talk, prompt portions: chunks of 32 keys that a block walks at least
         self.use_fused_router = os.environ.get("LLMIE_FUSED_ROUTER", "1") != "0"   # a router's product and choice in one kernel (few rows, float32)
         self.use_tc_experts = True     # routed experts with many rows per expert: both grouped products on tcgen05 (bfloat16)
         self.use_tc_gate_up = True     # prompt portions: gate/up product with the activation as its epilogue, one tcgen05 kernel
@@ -1317,7 +1319,8 @@ class CudaKernels:
                 ctypes.c_void_p(q.data_ptr() + q_col * esize), q.shape[1], _ptr(k_pool), _ptr(v_pool), _ptr(block_table), block_table.shape[1],
                 _ptr(token_seq), _ptr(positions), _ptr(tile_info), tiles, _ptr(talk), _ptr(out), num_heads, num_kv_heads, head_dim, v_head_dim,
                 page_size, ctypes.c_float(scale), _ptr(sink), ctypes.c_void_p(0 if gate is None else gate.data_ptr() + gate_col * esize),
-                0 if gate is None else gate.shape[1], ctypes.c_float(softcap), self._stream()), "attention_ext (talking heads, tensor cores)")
+                0 if gate is None else gate.shape[1], ctypes.c_float(softcap), N, per_slice, slices, _ptr(scratch), self._stream()),
+                "attention_ext (talking heads, tensor cores)")
             return out
         slice_keys = self.lib.llmie_attention_talk_slice(num_heads, head_dim)
         if slice_keys < 32:
@@ -1358,6 +1361,12 @@ class CudaKernels:
             raise KernelError("mlstm: one bias per head and gate is needed")
         if D > 256:
             raise KernelError(f"mlstm: head_dim {D} is more than the 256 entries of a column that the kernel keeps in registers")
+            # slices of at least 256 keys, at most 16 of them, where a block would walk more than two of them alone
+            chunks = -(-max_context // 32)
+            per_slice = max(self.talk_slice_chunks, -(-chunks // 16))
+            slices = -(-chunks // per_slice) if chunks > 2 * per_slice else 1
+            scratch = self._scratch(N * num_heads * slices * (v_head_dim + 2), q.device) if slices > 1 else None
+            self.launches += int(slices > 1)
         dev = z.device
         work = torch.empty((2 * N * H * D + 2 * N * H,), dtype=torch.float32, device=dev)
         qf, kf = work[:N * H * D], work[N * H * D:2 * N * H * D]
@@ -1367,6 +1376,10 @@ class CudaKernels:
         self._check(self.lib.llmie_mlstm_prepare(_ptr(z), z.shape[1], q_col, k_col, _ptr(gates), gates.shape[1], _ptr(bias_i), _ptr(bias_f),
                                                  ctypes.c_float(cap or 0.0), ctypes.c_float(D ** -0.5), _ptr(qf), _ptr(kf), _ptr(ig), _ptr(fg), _ptr(mstate),
                                                  _ptr(batch.seq_slots), _ptr(before), batch.num_seqs, N, H, D, dt, self._stream()), "mlstm (prepare)")
+        # bfloat16: shorter slices while the blocks are fewer than the multiprocessors (a block walks its slice alone, 0.55 us a key). In float32 the
+        # places where a request is cut stay the same, and with them its bits
+        while q.dtype == torch.bfloat16 and self.short_talk_slices and slice_keys >= 64 and N * -(-max_context // slice_keys) < self.num_sms:
+            slice_keys = slice_keys // 64 * 32
         num = torch.empty((N, H, DV + 1), dtype=torch.float32, device=dev)
         m = torch.empty((N, H), dtype=torch.float32, device=dev)
         self._check(self.lib.llmie_mlstm_scan(_ptr(z), z.shape[1], v_col, _ptr(qf), _ptr(kf), _ptr(ig), _ptr(fg), _ptr(state), _ptr(mstate),
