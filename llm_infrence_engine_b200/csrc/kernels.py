@@ -84,6 +84,7 @@ class CudaKernels:
         self.up_act_min_rows = 512     # ... and a plain product with a GELU as its epilogue, from this many rows on (below, product and activation are faster)
         self.use_tc_qkv = True         # prompt portions, head size 64: q/k/v product with bias, rotation and cache write in one kernel ...
         self.tc_qkv_min_rows = 2048    # ... from this many rows on: below, the library product + the rotation kernel are 4 to 10 % of a step faster
+        self.tc_store_max_rows = 32   # ... and products of up to this many rows whose result is stored its cluster form (see _stored_by_tc)
         self.tc_max_rows = 128        # batches up to this many rows take the small-batch tensor-core product
         self.use_mma_attention_ext = True    # bfloat16 attention with extras on the tensor cores (else the generic kernel)
         # ... on tiles of at most this many rows. The kernel also has tiles of 64 and 128 rows (a chunk's keys fetched once for
@@ -144,7 +145,7 @@ class CudaKernels:
         self.deal_rounds = {64: 9, 128: 8}
         self.at_rest = AtRest()
         for fn in ("llmie_embed", "llmie_feed_tokens", "llmie_zero_fresh_state", "llmie_rope_tables", "llmie_add_rmsnorm", "llmie_rope_kv_write", "llmie_silu_mul",
-                   "llmie_gemm_simt", "llmie_gemm_tc", "llmie_gateup_silu_tc", "llmie_qkv_rope_tc", "llmie_add_into", "llmie_attn_plan", "llmie_attn_tc_plan", "llmie_paged_attention_mma", "llmie_paged_attention_mma_acc", "llmie_paged_attention_tc", "llmie_paged_attention_f32", "llmie_paged_attention_bf16", "llmie_argmax", "llmie_sample",
+                   "llmie_gemm_simt", "llmie_gemm_tc", "llmie_gemm_tc_store", "llmie_gateup_silu_tc", "llmie_qkv_rope_tc", "llmie_add_into", "llmie_attn_plan", "llmie_attn_tc_plan", "llmie_paged_attention_mma", "llmie_paged_attention_mma_acc", "llmie_paged_attention_tc", "llmie_paged_attention_f32", "llmie_paged_attention_bf16", "llmie_argmax", "llmie_sample",
                    "llmie_streams_expand", "llmie_streams_update", "llmie_streams_norm", "llmie_latent_prepare", "llmie_head_matmul",
                    "llmie_kv_store", "llmie_act", "llmie_paged_attention_ext_f32", "llmie_paged_attention_ext_bf16", "llmie_paged_attention_ext_mma",
                    "llmie_attention_ext_mma_fits", "llmie_paged_attention_ext_fa", "llmie_attention_ext_fa_fits",
@@ -462,6 +463,8 @@ class CudaKernels:
         M, K = x.shape
         N = w.shape[0]
         self._need(w, "w", x.dtype, 2)
+                if self._stored_by_tc(x, w):
+                    return self.linear_tc_store(x, w, torch.bfloat16, bias)
         if K != w.shape[1]:
             raise KernelError(f"linear: x has {K} columns, w has {w.shape[1]}")
         self._check_bias(bias, x, w)
@@ -492,8 +495,12 @@ class CudaKernels:
         if self.use_cublas and bf16 and out_dtype == torch.bfloat16:
             self.launches += 1
             return torch.nn.functional.linear(x, w, bias)
+        if small and out_dtype == torch.float32 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and self.store_blocks(M, N, K) > 1:
+            return self.linear_tc_store(x, w, out_dtype, bias)   # (few outputs: a block alone would walk all of K)
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
         self._check(self.lib.llmie_gemm_simt(_ptr(x), _ptr(w), _ptr(out), M, N, K, self._dt(x, "x"), self._dt(out, "out"), 0,
+        if small and self._stored_by_tc(x, w):
+            return self.linear_tc_store(x, w, out_dtype, bias)
                                              _ptr(bias), self._weights_at_rest(), self._stream()), "linear")
         return out
 
@@ -549,6 +556,36 @@ class CudaKernels:
 
     def error_flag(self, device) -> torch.Tensor:
         """The device word that a kernel sets when it gives up on a bounded wait (0: nothing happened). Whoever reads a
+    def _stored_by_tc(self, x, w) -> bool:
+        """Whether a bfloat16 product with a bfloat16 result takes the cluster form of the small-batch product instead of the library's. Measured
+        behind a norm (us, library / here): 896 x 896, 1 / 4 / 16 / 32 rows 6.2 / 4.7, 5.8 / 4.8, 5.7 / 5.1, 5.4 / 5.7; 4,160 x 1,024 7.9 / 6.0, 7.4 / 6.0,
+        6.9 / 5.8, 6.9 / 6.5; 6,336 x 2,048 9.6 / 8.2, 9.4 / 8.3, 9.8 / 8.7, 10.0 / 9.3, 64 rows 9.3 / 10.5."""
+        M, K = x.shape
+        return (self.use_tc_gemm and (M <= 16 or (M <= self.tc_store_max_rows and K >= 1024)) and K % 8 == 0 and x.data_ptr() % 16 == 0
+                and w.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0)
+
+    def store_blocks(self, M: int, N: int, K: int) -> int:
+        """How many blocks of a cluster share the K range of a small-batch product that is stored: up to two blocks per multiprocessor (9,728 x 896
+        at 16 rows: 2, 4, 8 blocks 7.1, 6.0, 11.4 us behind a norm; 6,336 x 2,048 11.4, 8.7, 13.9), no more than K has pieces."""
+        tiles = -(-N // 128) * -(-M // 64)
+        blocks = 1
+        while blocks < 8 and 2 * blocks <= -(-K // 64) and 2 * blocks * tiles <= 2.1 * self.num_sms:
+            blocks *= 2
+        return blocks
+
+    def linear_tc_store(self, x, w, out_dtype, bias=None, blocks=None):
+        """``x w^T (+ bias)``, stored as ``out_dtype``, on the tcgen05 tensor cores for small batches: the blocks that share a tile's K range
+        form a cluster and add their sums in shared memory, first to last. ``x`` may be a run of columns of wider rows (16-byte aligned).
+        ``w`` is fetched ahead of the kernel before only where it lies at rest."""
+        self._need(w, "w", torch.bfloat16, 2)
+        M, K = x.shape
+        N = w.shape[0]
+        out = torch.empty((M, N), dtype=out_dtype, device=w.device)
+        rc = self.lib.llmie_gemm_tc_store(_ptr(x), x.stride(0), _ptr(w), _ptr(out), _DT[out_dtype], M, N, K, blocks or self.store_blocks(M, N, K),
+                                          _ptr(self._errors(w.device)), _ptr(bias), self._weights_at_rest(), self._stream())
+        self._check(rc, "linear_tc_store")
+        return out
+
         step's results back reads this word with them and hands it to ``raise_for_error_code``."""
         return self._errors(torch.device(device))
 

@@ -77,7 +77,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
 // ------------------------------------------------------------------------------------------------ host side
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 std::mutex g_lock;
-std::map<std::tuple<const void*, int, int, int>, CUtensorMap> g_maps;  // (base, rows, K, box rows) -> descriptor
+std::map<std::tuple<const void*, int, int, int, int>, CUtensorMap> g_maps;  // (base, rows, K, box rows, row stride) -> descriptor
 
 int get_encoder() {
     if (g_encode) return 0;
@@ -90,16 +90,18 @@ int get_encoder() {
     return 0;
 }
 
-// A [rows, K] row-major bfloat16 matrix, read in boxes of box_rows x 64 elements with 128-byte swizzle; outside: zeros.
-int tensor_map(const void* base, int rows, int K, int box_rows, CUtensorMap* out) {
+// A [rows, K] row-major bfloat16 matrix (rows `stride` elements apart, K if 0), read in boxes of box_rows x 64 elements with 128-byte
+// swizzle; outside: zeros.
+int tensor_map(const void* base, int rows, int K, int box_rows, CUtensorMap* out, int stride = 0) {
     std::lock_guard<std::mutex> hold(g_lock);
-    const auto key = std::make_tuple(base, rows, K, box_rows);
+    if (stride == 0) stride = K;
+    const auto key = std::make_tuple(base, rows, K, box_rows, stride);
     auto it = g_maps.find(key);
     if (it != g_maps.end()) { *out = it->second; return 0; }
     int rc = get_encoder();
     if (rc) return rc;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+    const cuuint64_t strides[1] = {(cuuint64_t)stride * 2};
     const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
     CUtensorMap m;
