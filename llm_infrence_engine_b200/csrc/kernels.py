@@ -100,6 +100,12 @@ class CudaKernels:
         # projections that are activated by the product that makes them; below, the scan activates them as it reads them
         self.linear_attention_mma_rows = 24
         self.use_linear_attention_step = True   # ... and decoded tokens alone in bfloat16 a kernel that streams the states (float32: always the scan)
+        # Recurrences in bfloat16 walk sixteen tokens at a time (recurrent_chunk.cu) from this many rows of the longest request on, by kind (delta rule
+        # with a decay per channel, per head; state space), as long as their blocks of 16 columns are no more than so many per multiprocessor.
+        # (us, token by token / so: delta rule, 16 heads of 128 x 128, 64 tokens 20.9 / 23.3, 128 34.2 / 30.4, 2,048 462 / 302; eight requests of 128,
+        # 8 heads, 512 blocks 50 / 69; state space, 256 blocks, 64 tokens 16 / 28, 2,048 354 / 299: about 0.6 us a chunk for 10 us of start)
+        self.chunk_scan_rows = (128, 128, 512)
+        self.chunk_scan_blocks = (1.0, 1.0, 2.0)
         self.use_mma_attention_talk = True   # heads that talk, steps with prompt portions in bfloat16: plain scores and P V on the tensor cores
         self.head_matmul_library_rows = 64   # per-head products of latent attention: from this many rows on, one batched library product
         self.slice_keys = 1024         # generic attention: keys per slice, at fixed places of a request (a multiple of 32)
@@ -156,8 +162,10 @@ class CudaKernels:
                    "llmie_embed_add", "llmie_mlstm_prepare", "llmie_mlstm_scan", "llmie_mlstm_finish", "llmie_paged_attention_talk",
                    "llmie_attention_talk_slice", "llmie_attention_talk_mma_fits", "llmie_paged_attention_talk_mma", "llmie_embed_bigram",
                    "llmie_dynamic_tanh", "llmie_embed_positions", "llmie_post_rms", "llmie_qk_rows_norm_store", "llmie_linear_attention_scan",
-                   "llmie_linear_attention_mma", "llmie_linear_attention_mma_fits", "llmie_linear_attention_step", "llmie_paged_attention_mma_ext"):
+                   "llmie_linear_attention_mma", "llmie_linear_attention_mma_fits", "llmie_linear_attention_step", "llmie_paged_attention_mma_ext",
+                   "llmie_chunk_delta", "llmie_chunk_ssm"):
             getattr(self.lib, fn).restype = ctypes.c_int
+        self.lib.llmie_chunk_scratch.restype = ctypes.c_longlong
         # two forms of the gate/up kernel live in source files of their own, and the library also builds without them
         self._gate_up_cluster = self._gate_up_pair = self._gate_up_glu_pair = self._up_gelu_pair = None
         self.lib.llmie_gateup_glu_tc.restype = ctypes.c_int
@@ -455,6 +463,8 @@ class CudaKernels:
                 if x.shape[1] != w.shape[1]:
                     raise KernelError(f"linear: x has {x.shape[1]} columns, w has {w.shape[1]}")
                 self._check_bias(bias, x, w)
+                if self._stored_by_tc(x, w):
+                    return self.linear_tc_store(x, w, torch.bfloat16, bias)
                 self.launches += 1
                 return torch.nn.functional.linear(x, w, bias)
             x = x.contiguous()
@@ -463,8 +473,6 @@ class CudaKernels:
         M, K = x.shape
         N = w.shape[0]
         self._need(w, "w", x.dtype, 2)
-                if self._stored_by_tc(x, w):
-                    return self.linear_tc_store(x, w, torch.bfloat16, bias)
         if K != w.shape[1]:
             raise KernelError(f"linear: x has {K} columns, w has {w.shape[1]}")
         self._check_bias(bias, x, w)
@@ -487,20 +495,20 @@ class CudaKernels:
         out_dtype = out_dtype or x.dtype
         if small and transient:
             return self.linear_tc(x, w, out=self._transient(M, N, w.device), accumulate=True, bias=bias)
+        if small and out_dtype == torch.float32 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and self.store_blocks(M, N, K) > 1:
+            return self.linear_tc_store(x, w, out_dtype, bias)   # (few outputs: a block alone would walk all of K)
         if small and out_dtype == torch.float32:
             return self.linear_tc(x, w, bias=bias)
+        if small and self._stored_by_tc(x, w):
+            return self.linear_tc_store(x, w, out_dtype, bias)
         if bf16 and out_dtype == torch.float32 and self.use_tc_gemm and K % 8 == 0 and N <= 520:
             # few outputs in 32-bit for many rows (a router's logits over a prompt portion): a few tiles of weight rows, a block per 64 rows
             return self.linear_tc(x, w, bias=bias)
         if self.use_cublas and bf16 and out_dtype == torch.bfloat16:
             self.launches += 1
             return torch.nn.functional.linear(x, w, bias)
-        if small and out_dtype == torch.float32 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and self.store_blocks(M, N, K) > 1:
-            return self.linear_tc_store(x, w, out_dtype, bias)   # (few outputs: a block alone would walk all of K)
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
         self._check(self.lib.llmie_gemm_simt(_ptr(x), _ptr(w), _ptr(out), M, N, K, self._dt(x, "x"), self._dt(out, "out"), 0,
-        if small and self._stored_by_tc(x, w):
-            return self.linear_tc_store(x, w, out_dtype, bias)
                                              _ptr(bias), self._weights_at_rest(), self._stream()), "linear")
         return out
 
@@ -548,14 +556,6 @@ class CudaKernels:
         self._check(rc, "linear_tc")
         return out
 
-    def _errors(self, device) -> torch.Tensor:
-        if self._error_flag is None:
-            with torch.inference_mode(False):  # an ordinary tensor: it is cleared later from code that runs outside inference mode
-                self._error_flag = torch.zeros(1, dtype=torch.int32, device=device)
-        return self._error_flag
-
-    def error_flag(self, device) -> torch.Tensor:
-        """The device word that a kernel sets when it gives up on a bounded wait (0: nothing happened). Whoever reads a
     def _stored_by_tc(self, x, w) -> bool:
         """Whether a bfloat16 product with a bfloat16 result takes the cluster form of the small-batch product instead of the library's. Measured
         behind a norm (us, library / here): 896 x 896, 1 / 4 / 16 / 32 rows 6.2 / 4.7, 5.8 / 4.8, 5.7 / 5.1, 5.4 / 5.7; 4,160 x 1,024 7.9 / 6.0, 7.4 / 6.0,
@@ -586,6 +586,14 @@ class CudaKernels:
         self._check(rc, "linear_tc_store")
         return out
 
+    def _errors(self, device) -> torch.Tensor:
+        if self._error_flag is None:
+            with torch.inference_mode(False):  # an ordinary tensor: it is cleared later from code that runs outside inference mode
+                self._error_flag = torch.zeros(1, dtype=torch.int32, device=device)
+        return self._error_flag
+
+    def error_flag(self, device) -> torch.Tensor:
+        """The device word that a kernel sets when it gives up on a bounded wait (0: nothing happened). Whoever reads a
         step's results back reads this word with them and hands it to ``raise_for_error_code``."""
         return self._errors(torch.device(device))
 
@@ -1352,6 +1360,12 @@ class CudaKernels:
         if per_tile:
             # steps with prompt portions, bfloat16: a tile of 16 / (heads per key/value head) tokens and all heads on the tensor cores
             tiles, tile_info = self._tiles(batch, per_tile, q.device)
+            # slices of at least 256 keys, at most 16 of them, where a block would walk more than two of them alone
+            chunks = -(-max_context // 32)
+            per_slice = max(self.talk_slice_chunks, -(-chunks // 16))
+            slices = -(-chunks // per_slice) if chunks > 2 * per_slice else 1
+            scratch = self._scratch(N * num_heads * slices * (v_head_dim + 2), q.device) if slices > 1 else None
+            self.launches += int(slices > 1)
             self._check(self.lib.llmie_paged_attention_talk_mma(
                 ctypes.c_void_p(q.data_ptr() + q_col * esize), q.shape[1], _ptr(k_pool), _ptr(v_pool), _ptr(block_table), block_table.shape[1],
                 _ptr(token_seq), _ptr(positions), _ptr(tile_info), tiles, _ptr(talk), _ptr(out), num_heads, num_kv_heads, head_dim, v_head_dim,
@@ -1362,6 +1376,10 @@ class CudaKernels:
         slice_keys = self.lib.llmie_attention_talk_slice(num_heads, head_dim)
         if slice_keys < 32:
             raise KernelError(f"attention_ext: {num_heads} talking heads of {head_dim} entries do not fit the kernel's shared memory")
+        # bfloat16: shorter slices while the blocks are fewer than the multiprocessors (a block walks its slice alone, 0.55 us a key). In float32 the
+        # places where a request is cut stay the same, and with them its bits
+        while q.dtype == torch.bfloat16 and self.short_talk_slices and slice_keys >= 64 and N * -(-max_context // slice_keys) < self.num_sms:
+            slice_keys = slice_keys // 64 * 32
         splits = max(1, -(-max_context // slice_keys))
         scratch = self._scratch(N * num_heads * splits * (v_head_dim + 2), q.device) if splits > 1 else None
         self._check(self.lib.llmie_paged_attention_talk(
@@ -1398,12 +1416,6 @@ class CudaKernels:
             raise KernelError("mlstm: one bias per head and gate is needed")
         if D > 256:
             raise KernelError(f"mlstm: head_dim {D} is more than the 256 entries of a column that the kernel keeps in registers")
-            # slices of at least 256 keys, at most 16 of them, where a block would walk more than two of them alone
-            chunks = -(-max_context // 32)
-            per_slice = max(self.talk_slice_chunks, -(-chunks // 16))
-            slices = -(-chunks // per_slice) if chunks > 2 * per_slice else 1
-            scratch = self._scratch(N * num_heads * slices * (v_head_dim + 2), q.device) if slices > 1 else None
-            self.launches += int(slices > 1)
         dev = z.device
         work = torch.empty((2 * N * H * D + 2 * N * H,), dtype=torch.float32, device=dev)
         qf, kf = work[:N * H * D], work[N * H * D:2 * N * H * D]
@@ -1413,10 +1425,6 @@ class CudaKernels:
         self._check(self.lib.llmie_mlstm_prepare(_ptr(z), z.shape[1], q_col, k_col, _ptr(gates), gates.shape[1], _ptr(bias_i), _ptr(bias_f),
                                                  ctypes.c_float(cap or 0.0), ctypes.c_float(D ** -0.5), _ptr(qf), _ptr(kf), _ptr(ig), _ptr(fg), _ptr(mstate),
                                                  _ptr(batch.seq_slots), _ptr(before), batch.num_seqs, N, H, D, dt, self._stream()), "mlstm (prepare)")
-        # bfloat16: shorter slices while the blocks are fewer than the multiprocessors (a block walks its slice alone, 0.55 us a key). In float32 the
-        # places where a request is cut stay the same, and with them its bits
-        while q.dtype == torch.bfloat16 and self.short_talk_slices and slice_keys >= 64 and N * -(-max_context // slice_keys) < self.num_sms:
-            slice_keys = slice_keys // 64 * 32
         num = torch.empty((N, H, DV + 1), dtype=torch.float32, device=dev)
         m = torch.empty((N, H), dtype=torch.float32, device=dev)
         self._check(self.lib.llmie_mlstm_scan(_ptr(z), z.shape[1], v_col, _ptr(qf), _ptr(kf), _ptr(ig), _ptr(fg), _ptr(state), _ptr(mstate),
@@ -1821,6 +1829,15 @@ class CudaKernels:
                     "causal_conv")
         return out
 
+    def _chunk_scratch(self, kind: int, H: int, G: int, D: int, DV: int, N: int, batch, dtype, device):
+        """Scratch of the form that walks sixteen tokens at a time (kinds: 0 and 1 the delta rule with a decay per channel and per head, 2 the
+        state space), or None where a step stays with the token-by-token kernels: float32, short portions, many requests, sizes that are not built."""
+        if (dtype != torch.bfloat16 or batch.max_seq_len < self.chunk_scan_rows[kind]
+                or batch.num_seqs * H * -(-DV // 16) > self.chunk_scan_blocks[kind] * self.num_sms):
+            return None
+        floats = self.lib.llmie_chunk_scratch(kind, H, G, D, N, batch.num_seqs)
+        return torch.empty((floats,), dtype=torch.float32, device=device) if floats else None
+
     def delta_rule(self, qkv, num_heads, num_kv_heads, head_dim, v_head_dim, a, b, b_col, A_log, dt_bias, state, batch, unit_eps=1e-6,
                    decay_per_head=False):
         """The gated delta rule with a decay per key channel over the rows of each request, from ``state [slots, heads, v_head_dim, head_dim]``
@@ -1846,6 +1863,16 @@ class CudaKernels:
         self._need(A_log, "A_log", torch.float32, 1)
         self._need(dt_bias, "dt_bias", torch.float32, 1)
         dev = qkv.device
+        out = torch.empty((N, H * DV), dtype=torch.float32, device=dev)
+        scratch = self._chunk_scratch(int(bool(decay_per_head)), H, G, D, DV, N, batch, qkv.dtype, dev)
+        if scratch is not None:
+            self._check(self.lib.llmie_chunk_delta(
+                _ptr(qkv), qkv.shape[1], 0, G * D, 2 * G * D, _ptr(a), a.stride(0), ctypes.c_void_p(b.data_ptr() + b_col * b.element_size()), b.stride(0),
+                _ptr(A_log), _ptr(dt_bias), _ptr(scratch), _ptr(state), _ptr(batch.seq_starts_dev), _ptr(batch.seq_slots), _ptr(out), H, G, D, DV,
+                batch.num_seqs, batch.max_seq_len, ctypes.c_float(D ** -0.5), ctypes.c_float(unit_eps), int(bool(decay_per_head)), self._stream()),
+                "delta_rule (sixteen tokens at a time)")
+            self.launches += 1
+            return out
         work = torch.empty((N, 2 * G * D + G + H * DA + H), dtype=torch.float32, device=dev)
         flat = work.view(-1)
         o = 0
@@ -1858,7 +1885,6 @@ class CudaKernels:
         self._check(self.lib.llmie_delta_prepare(_ptr(qkv), qkv.shape[1], 0, G * D, _ptr(a), a.stride(0), ctypes.c_void_p(b.data_ptr() + b_col * b.element_size()),
                                                  b.stride(0), _ptr(A_log), _ptr(dt_bias), _ptr(qn), _ptr(kn), _ptr(kq), _ptr(decay), _ptr(beta), N, H, G, D,
                                                  ctypes.c_float(D ** -0.5), ctypes.c_float(unit_eps), int(bool(decay_per_head)), dt, self._stream()), "delta_rule (prepare)")
-        out = torch.empty((N, H * DV), dtype=torch.float32, device=dev)
         self._check(self.lib.llmie_delta_scan(_ptr(qkv), qkv.shape[1], 2 * G * D, _ptr(qn), _ptr(kn), _ptr(kq), _ptr(decay), _ptr(beta), _ptr(state),
                                               _ptr(batch.seq_starts_dev), _ptr(batch.seq_slots), _ptr(out), H, G, D, DV, batch.num_seqs, batch.max_seq_len,
                                               int(bool(decay_per_head)), dt, self._stream()), "delta_rule (scan)")
@@ -1882,6 +1908,14 @@ class CudaKernels:
             if t.shape[0] != H:
                 raise KernelError(f"ssm_scan: {name} needs one entry per head")
         out = torch.empty((xbc.shape[0], H * DV), dtype=torch.float32, device=xbc.device)
+        scratch = self._chunk_scratch(2, H, G, NS, DV, xbc.shape[0], batch, xbc.dtype, xbc.device)
+        if scratch is not None:
+            self._check(self.lib.llmie_chunk_ssm(
+                _ptr(xbc), xbc.shape[1], 0, H * DV, H * DV + G * NS, ctypes.c_void_p(dt.data_ptr() + dt_col * dt.element_size()), dt.stride(0), _ptr(A_log),
+                _ptr(dt_bias), _ptr(skip), _ptr(scratch), _ptr(state), _ptr(batch.seq_starts_dev), _ptr(batch.seq_slots), _ptr(out), H, G, NS, DV,
+                batch.num_seqs, batch.max_seq_len, self._stream()), "ssm_scan (sixteen tokens at a time)")
+            self.launches += 1
+            return out
         self._check(self.lib.llmie_ssm_scan(_ptr(xbc), xbc.shape[1], 0, H * DV, H * DV + G * NS, ctypes.c_void_p(dt.data_ptr() + dt_col * dt.element_size()),
                                             dt.stride(0), _ptr(A_log), _ptr(dt_bias), _ptr(skip), _ptr(state), _ptr(batch.seq_starts_dev), _ptr(batch.seq_slots),
                                             _ptr(out), H, G, NS, DV, batch.num_seqs, batch.max_seq_len, self._dt(xbc, "xbc"), self._stream()), "ssm_scan")
