@@ -84,7 +84,7 @@ class CudaKernels:
         self.up_act_min_rows = 512     # ... and a plain product with a GELU as its epilogue, from this many rows on (below, product and activation are faster)
         self.use_tc_qkv = True         # prompt portions, head size 64: q/k/v product with bias, rotation and cache write in one kernel ...
         self.tc_qkv_min_rows = 2048    # ... from this many rows on: below, the library product + the rotation kernel are 4 to 10 % of a step faster
-        self.tc_store_max_rows = 32   # ... and products of up to this many rows whose result is stored its cluster form (see _stored_by_tc)
+        self.tc_store_max_rows = 8    # ... and products of up to this many rows whose result is stored its cluster form (see _stored_by_tc)
         self.tc_max_rows = 128        # batches up to this many rows take the small-batch tensor-core product
         self.use_mma_attention_ext = True    # bfloat16 attention with extras on the tensor cores (else the generic kernel)
         # ... on tiles of at most this many rows. The kernel also has tiles of 64 and 128 rows (a chunk's keys fetched once for
@@ -559,10 +559,11 @@ class CudaKernels:
     def _stored_by_tc(self, x, w) -> bool:
         """Whether a bfloat16 product with a bfloat16 result takes the cluster form of the small-batch product instead of the library's. Measured
         behind a norm (us, library / here): 896 x 896, 1 / 4 / 16 / 32 rows 6.2 / 4.7, 5.8 / 4.8, 5.7 / 5.1, 5.4 / 5.7; 4,160 x 1,024 7.9 / 6.0, 7.4 / 6.0,
-        6.9 / 5.8, 6.9 / 6.5; 6,336 x 2,048 9.6 / 8.2, 9.4 / 8.3, 9.8 / 8.7, 10.0 / 9.3, 64 rows 9.3 / 10.5."""
+        6.9 / 5.8, 6.9 / 6.5; 6,336 x 2,048 9.6 / 8.2, 9.4 / 8.3, 9.8 / 8.7, 10.0 / 9.3. In whole steps it gains up to 8 rows; at 16 (a projection of
+        1,024, sixteen requests, routed experts) its early start costs the kernels around it more: 16 steps 10.0 -> 10.1 ms."""
         M, K = x.shape
-        return (self.use_tc_gemm and (M <= 16 or (M <= self.tc_store_max_rows and K >= 1024)) and K % 8 == 0 and x.data_ptr() % 16 == 0
-                and w.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0)
+        return (self.use_tc_gemm and M <= self.tc_store_max_rows and K % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+                and x.stride(0) % 8 == 0)
 
     def store_blocks(self, M: int, N: int, K: int) -> int:
         """How many blocks of a cluster share the K range of a small-batch product that is stored: up to two blocks per multiprocessor (9,728 x 896
